@@ -103,6 +103,12 @@ inline bool ranges_overlap(const void* a, size_t abytes, const void* b, size_t b
 
 int check_grid(int nx, int nz);
 
+// HV = -12 hv of the IEEE-FP64 form (hv = -hv_beta d / (16 dt_full),
+// interpolate.py:101,149), whose kernels carry fluxes divided by it: held above
+// 2^-400 (dt_full / d above 2^395), where the hyperviscosity term is far below
+// rounding either way.
+inline double ieee_hv(double d, double dt_full) { return std::fmax(12.0 * kHvBeta * d / (16 * dt_full), 0x1p-400); }
+
 inline bool valid_f64_mode(int m) { return m == MW_F64_NATIVE || m == MW_F64_SPLIT || m == MW_F64_IEEE; }
 
 // Rows per z CTA for a single-grid launch: the largest tile up to max_rows

@@ -44,28 +44,37 @@ constexpr Series make_series(double e) {
   return t;
 }
 
-// 1/y for the lanes in `mask`, which call it together: an FP32 estimate
-// (operand and result converted by integer operations) refined by one cubic
-// Newton step in FP64, r = r0 (1 + e + e^2), e = 1 - y r0, whose relative
-// error e^3 <= 2^-66 lies below FP64 rounding: 3 FP64 operations.  |y|
-// outside [2^-125, 2^126) (and Inf, NaN, 0) takes the FP64 division, behind
-// a warp-uniform branch so that it is never evaluated speculatively on the
-// other lanes.
+// 1/y for the lanes in `mask`, which call it together, in 2 FP64 operations.
+// With y = m 2^E, m in [1, 2), an estimate R of 1/m to about 2^-45 is formed
+// on the FP32 and integer pipes (which run beside the FP64 pipe): the hardware
+// estimate r0 of 1/mh, mh the leading 24 bits of m, corrected to first and
+// second order, r1 = r0 (e + e^2), e = 1 - m r0, and r0 + r1 put together as a
+// 53-bit integer significand.  One Newton step in FP64, r = R + R (1 - y R),
+// squares the error (2^-90), so r carries little more than its last rounding.
+// (A 24-bit estimate with a cubic step took 3 operations; the kernels are bound
+// by the FP64 pipe, which needs 16 SM clocks per warp operation.)  Zero,
+// subnormal, Inf, NaN and |y| >= 2^1022 take the FP64 division, behind a
+// warp-uniform branch so that it is never evaluated speculatively on the other
+// lanes.
 __device__ __forceinline__ double rcp(double y, unsigned mask) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(y);
   const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
   const unsigned ex = (hi >> 20) & 0x7ffu;
-  // float with y's sign, rebiased exponent and leading 23 significand bits
-  const unsigned fb = ((__funnelshift_l(lo, hi, 3) + 0x40000000u) & 0x7fffffffu) | (hi & 0x80000000u);
-  float rf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(__uint_as_float(fb)));
-  const unsigned rb = __float_as_uint(rf);
-  const unsigned rhi = (((rb >> 3) & 0x0fffffffu) + (896u << 20)) | (rb & 0x80000000u);
-  const double r0 = __longlong_as_double((long long)(((unsigned long long)rhi << 32) | (rb << 29)));
-  const double e = fma(-y, r0, 1.0);
-  const double t = fma(e, e, e);
-  double r = fma(r0, t, r0);
-  const bool out = ex - (1023u - 125u) > 250u;
+  const float mh = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffffu) | 0x3f800000u);
+  const float ml = __uint2float_rn(lo & 0x1fffffffu) * 0x1p-52f;
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(mh));
+  const float e0 = fmaf(-ml, r0, fmaf(-mh, r0, 1.0f));
+  const int i1 = __float2int_rn(fmaf(e0, e0, e0) * r0 * 0x1p53f);  // |i1| <= 2^31 2^-1
+  // R = (M0 2^29 + i1) 2^-53 with r0 = M0 2^-24 in [1/2, 1]: added to the bits of the
+  // double r0 2^-E as an integer (a carry or borrow moves the exponent as it should
+  // to the accuracy of R)
+  const unsigned rb = __float_as_uint(r0);
+  const unsigned rhi = (rb >> 3) + ((1919u - ex) << 20);  // 1919 = 1023 + 896: exponent of r0 less that of y
+  const long long rbits = (long long)(((unsigned long long)(rhi | (hi & 0x80000000u)) << 32) | (rb << 29)) + i1;
+  const double r0d = __longlong_as_double(rbits);
+  double r = fma(r0d, fma(-y, r0d, 1.0), r0d);
+  const bool out = ex - 1u > 2043u;
   if (__any_sync(mask, out)) {
     if (out) r = 1.0 / y;
   }
@@ -90,8 +99,20 @@ __device__ __forceinline__ double series_g(double d, int n, const Series& S) {
   return g;
 }
 
-// 12 x the 4-point interpolation (the stencil of interpolate.py:33-43 and
-// 69-79 with its division by 12 folded into the scaling).
+// The stencils of interpolate.py:33-43 and 69-79 by second differences.  With
+// t = s(k-1) + s(k+1) every cell gives e = t - 2 s and q = 8 s - t, and the
+// interface between cells k - 1 and k has
+//   12 x the 4-point interpolation  7 (s(k-1) + s(k)) - (s(k-2) + s(k+1)) = q(k-1) + q(k),
+//   the third difference            s(k+1) - s(k-2) + 3 (s(k-1) - s(k))   = e(k) - e(k-1):
+// 5 operations per cell and variable where the neighbouring interfaces share
+// e and q, against 6 for the two stencils taken one by one.
+__device__ __forceinline__ void cell_eq(double sm, double s, double sp, double& e, double& q) {
+  const double t = sm + sp;
+  e = fma(-2.0, s, t);
+  q = fma(8.0, s, -t);
+}
+
+// 12 x the 4-point interpolation on its own.
 __device__ __forceinline__ double interp12(double s0, double s1, double s2, double s3) {
   return fma(7.0, s1 + s2, -(s0 + s3));
 }

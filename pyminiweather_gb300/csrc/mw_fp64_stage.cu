@@ -9,35 +9,39 @@
 // warp-instructions: the kernels are bound by their FP64 operation count, and
 // integer work (conversions, index arithmetic, table look-ups) is nearly free.
 // Against the reference's formulas (one pow, three divides and ~50 operations
-// per interface, interpolate.py:82-186) each interface costs ~37 + n FP64
-// operations and each cell update 8 (ncu: 47.6 per cell-stage in x, 49.3 in
-// z on the collision case):
-//   - quantities are carried scaled by 12, so the 4-point interpolation is
-//     A = 7 (s1 + s2) - (s0 + s3) and needs no division; the third
-//     difference is D = (s3 - s0) + 3 (s1 - s2): 6 operations per variable;
-//   - one reciprocal per interface, 3 FP64 operations (ieee::rcp);
+// per interface, interpolate.py:82-186) a cell-stage costs 37 + n FP64
+// operations, n the degree of the pressure series (z: one more, gravity):
+//   - quantities are carried scaled by 12 and the two stencils are formed from
+//     second differences e and q of the cells, shared by the neighbouring
+//     interfaces: 5 operations per variable (ieee::cell_eq);
+//   - fluxes are carried divided by HV = -12 hv, so that the hyperviscosity
+//     term is the third difference itself, added by the FMA that forms the
+//     advective term: rho is scaled by HV (one FMA with the background), so
+//     that u / HV comes out of the reciprocal at no cost;
+//   - one reciprocal per interface, 2 FP64 operations (ieee::rcp);
 //   - pressure enters as the perturbation P_row ((1 + delta)^gamma - 1),
 //     delta = (rho theta)' / (rho theta)_bg, P_row = C0 (rho theta)_bg^gamma:
 //     exactly the reference's p - hy_pressure_int in z (hy_pressure_int is
 //     C0 hy_dens_theta_int^gamma, ics/initial.py:105); in x the row constant
 //     cancels in the flux difference.  (1 + delta)^gamma - 1 is its binomial
-//     series summed by Horner's rule to the degree n that the warp's largest
-//     |delta| needs for a truncation below 2^-54 relative (one FMA in a
-//     region at rest, up to 15 terms for |delta| < 1/8), and
-//     expm1(gamma log1p(delta)) beyond; the single-grid kernels evaluate it
-//     as a polynomial in 12 (rho theta)' with per-row coefficients (RowP), n
-//     operations in all;
-//   - the stage update is out = init + c (F(i) - F(i+1)), c = dt / (12 d):
+//     series summed by Horner's rule to the degree n that |delta| needs for a
+//     truncation below 2^-54 relative (one FMA in a region at rest, up to 15
+//     terms for |delta| < 1/8), and expm1(gamma log1p(delta)) beyond; the
+//     single-grid kernels evaluate it as a polynomial in 12 (rho theta)' with
+//     per-row coefficients (RowP), n operations in all;
+//   - the stage update is out = init + c (F(i) - F(i+1)), c = HV dt / (12 d):
 //     2 operations per value.
 //
-// x pass: warps walk 63-cell segments of the rows with no CTA barrier, lane l
-// evaluating the fluxes at interfaces x0+l and x0+32+l (two independent FP64
-// chains) from values staged in the warp's shared-memory slice.  z pass: one
-// thread per column marching a tile of rows with a rolling 4-row window, so
-// each interface flux is evaluated once.  Halo cells are never read: the
-// periodic-x and wall-z rules of ics/bcs.py are applied to the indices and
-// values as they are loaded.  Every global access goes through MW_AT
-// (bounds-checked in the debug library).
+// x pass: warps walk runs of a row in blocks of 64 cells with no CTA barrier,
+// lane l holding cells j+l and j+32+l (two independent FP64 chains) staged in
+// the warp's shared-memory slice; e, q and the flux of the cell before come
+// from the neighbouring lane, or from the block before.  z pass: one thread
+// per column marching a tile of rows, e, q and the flux of the row before kept
+// in registers.  Halo cells are never read: the periodic-x and wall-z rules of
+// ics/bcs.py are applied to the indices and values as they are loaded.  The
+// result at a cell depends on its neighbourhood alone, not on how the grid is
+// split over warps (the series' degree is chosen per lane).  Every global
+// access goes through MW_AT (bounds-checked in the debug library).
 #include <algorithm>
 #include <atomic>
 
@@ -51,31 +55,29 @@ namespace ieee {
 constexpr int kXT = 256;            // threads per x CTA
 constexpr int kZT = 128;            // columns per z CTA
 constexpr int kZTileMax = 64;       // rows per z CTA
-#ifndef MW_IEEE_X_SEGS_PER_WARP
-#define MW_IEEE_X_SEGS_PER_WARP 16
-#endif
+constexpr int kXRunBlocksMax = 16;  // blocks of 64 cells per warp of the x pass
 
 // (1 + d)^gamma: the pressure perturbation.
 __constant__ Series c_pow_g = make_series(kGamma);
 
-// Row constants, scaled by 12 like the interpolated values.
+// Row constants; the interpolated values are scaled by 12, the fluxes by 12 / HV.
 struct RowD {
-  double R12;    // 12 background rho
+  double R;      // HV x 12 background rho
   double RT12;   // 12 background rho theta
   double IRT12;  // 1 / (12 background rho theta)
-  double P12;    // 12 background pressure C0 (rho theta)^gamma
-  double PC1;    // P12 C(gamma, 1) IRT12: the pressure perturbation per unit of 12 (rho theta)' to first order
+  double P;      // 12 / HV x background pressure C0 (rho theta)^gamma
+  double PC1;    // P C(gamma, 1) IRT12: the pressure perturbation per unit of 12 (rho theta)' to first order
 };
-__device__ __forceinline__ RowD row_consts(double r, double rt, double P) {
-  const double irt = 1.0 / (12.0 * rt);
-  return {12.0 * r, 12.0 * rt, irt, 12.0 * P, 12.0 * P * c_pow_g.c[1] * irt};
+__device__ __forceinline__ RowD row_consts(double r, double rt, double P, double HV, double IHV) {
+  const double irt = 1.0 / (12.0 * rt), p = 12.0 * P * IHV;
+  return {12.0 * r * HV, 12.0 * rt, irt, p, p * c_pow_g.c[1] * irt};
 }
 
-// P12 ((1 + d)^gamma - 1) + add, d = AT IRT12, for the lanes in `mask`, which
+// P ((1 + d)^gamma - 1) + add, d = AT IRT12, for the lanes in `mask`, which
 // call it together: the binomial series to the degree the largest |d| among
 // them needs (a warp-uniform loop), or expm1(gamma log1p(d)) for |d| >= 1/8,
 // Inf and NaN.  At degree 1 (|d| < 2^-52 on every lane, e.g. a region at
-// rest) the series is P12 C1 d = AT PC1: one FMA in all.
+// rest) the series is P C1 d = AT PC1: one FMA in all.
 __device__ __forceinline__ double pressure(double AT, const RowD& r, double add, unsigned mask) {
   const double d = AT * r.IRT12;
   bool big;
@@ -85,13 +87,13 @@ __device__ __forceinline__ double pressure(double AT, const RowD& r, double add,
   if (__any_sync(mask, big)) {
     if (big) f = expm1(kGamma * log1p(d));
   }
-  return fma(r.P12, f, add);
+  return fma(r.P, f, add);
 }
 
 // Row constants with the pressure series as a polynomial in the interpolated
-// 12 (rho theta)' itself: b[n] = P12 C(gamma, n) IRT12^n, so that
-// P12 ((1 + d)^gamma - 1) = sum_n b[n] AT^n (d = AT IRT12) is Horner's rule in
-// AT with no multiplication by IRT12 before it and none by P12 after it: two
+// 12 (rho theta)' itself: b[n] = P C(gamma, n) IRT12^n, so that
+// P ((1 + d)^gamma - 1) = sum_n b[n] AT^n (d = AT IRT12) is Horner's rule in
+// AT with no multiplication by IRT12 before it and none by P after it: two
 // FP64 operations fewer per interface wherever the degree exceeds one.
 struct RowP {
   RowD d;
@@ -99,14 +101,14 @@ struct RowP {
   int eI;                 // biased exponent of IRT12; 4096 where the b[n] would leave the normal range
   unsigned mI;            // an upper bound of 2^16 x IRT12's significand (in [1, 2)): top 16 fraction bits + 1
 };
-__device__ __forceinline__ RowP row_consts_p(double r, double rt, double P) {
+__device__ __forceinline__ RowP row_consts_p(double r, double rt, double P, double HV, double IHV) {
   RowP o;
-  o.d = row_consts(r, rt, P);
+  o.d = row_consts(r, rt, P, HV, IHV);
   double pw = o.d.IRT12;
   o.b[0] = 0.0;
 #pragma unroll
   for (int n = 1; n <= kMaxDeg; ++n) {
-    o.b[n] = o.d.P12 * c_pow_g.c[n] * pw;
+    o.b[n] = o.d.P * c_pow_g.c[n] * pw;
     pw *= o.d.IRT12;
   }
   const double lo = fabs(o.b[kMaxDeg]), hi = fabs(o.b[1]);
@@ -117,69 +119,68 @@ __device__ __forceinline__ RowP row_consts_p(double r, double rt, double P) {
   return o;
 }
 
-// The same as pressure(AT, r.d, add, mask), evaluated in AT: the degree comes
-// from an upper bound on the exponent of d = AT IRT12 (the sum of the exponents
-// of AT and IRT12, plus one where the product of upper bounds of their leading
-// 17 significand bits reaches 2), found by integer operations and never below
-// the degree d itself needs; warps where the bound reaches 1/8 (and Inf, NaN,
-// rows with eI = 4096) take the series in d.
+// The same as pressure(AT, r.d, add, mask), evaluated in AT and to a degree
+// chosen per lane, so that a cell's result does not depend on the cells its
+// warp happens to hold.  The degree comes from an upper bound on the exponent
+// of d = AT IRT12 (the sum of the exponents of AT and IRT12, plus one where the
+// product of upper bounds of their leading 17 significand bits reaches 2),
+// found by integer operations and never below the degree d itself needs; the
+// Horner loop runs from the warp's largest degree, a lane's sum starting (from
+// zero) at its own.  Lanes whose bound reaches 1/8 (and Inf, NaN, rows with
+// eI = 4096) take the series in d, or expm1 / log1p, at their full degree.
 __device__ __forceinline__ double pressure(double AT, const RowP& r, double add, unsigned mask) {
   const unsigned long long bA = (unsigned long long)__double_as_longlong(AT);
   const int exA = (int)(bA >> 52 & 0x7ffu);
   const unsigned mA = (unsigned)(bA >> 36 & 0xffffu) + 0x10001u;
   const int carry = (unsigned long long)mA * r.mI >= (1ull << 33) ? 1 : 0;
   const int eu = exA == 0 ? 0 : exA + r.eI - 1023 + carry;  // biased exponent of d is at most eu
-  if (__any_sync(mask, eu >= 1020)) return pressure(AT, r.d, add, mask);
-  const int exm = (int)__reduce_max_sync(mask, (unsigned)max(eu, 0));
-  const int n = c_pow_g.deg[min(1022 - exm, 64)];
-  double g = r.b[n];
-  for (int k = n - 1; k >= 1; --k) g = fma(g, AT, r.b[k]);
-  return fma(g, AT, add);
+  const bool far = eu >= 1020;
+  const int n = far ? 1 : c_pow_g.deg[min(1022 - max(eu, 0), 64)];
+  const int nmax = (int)__reduce_max_sync(mask, (unsigned)n);
+  double g = n == nmax ? r.b[nmax] : 0.0;
+  for (int k = nmax - 1; k >= 1; --k) {
+    g = fma(g, AT, r.b[k]);
+    if (k > n) g = 0.0;
+  }
+  double p = fma(g, AT, add);
+  if (__any_sync(mask, far)) {
+    if (far) {
+      const double d = AT * r.d.IRT12;
+      const bool big = !(fabs(d) < 0.125);
+      double f = d * series_g(d, kMaxDeg, c_pow_g);
+      if (big) f = expm1(kGamma * log1p(d));
+      p = fma(r.d.P, f, add);
+    }
+  }
+  return p;
 }
 
 __device__ __forceinline__ const RowD& rowd(const RowD& r) { return r; }
 __device__ __forceinline__ const RowD& rowd(const RowP& r) { return r.d; }
 
-// 12 x the 4-point interpolation and the third difference of one variable
-// (the stencils of interpolate.py:33-43 and 69-79).
-__device__ __forceinline__ void interp(double s0, double s1, double s2, double s3, double& A, double& D) {
-  A = interp12(s0, s1, s2, s3);
-  D = fma(3.0, s1 - s2, s3 - s0);
-}
-
-// x flux times 12 (interpolate.py:82-129): with u = (rho u)' / rho,
+// x flux times 12 / HV (interpolate.py:82-129) from 12 x the interpolated
+// values A and the third differences D: with u = (rho u)' / rho,
 // F = ((rho u)', u (rho u)' + p', u (rho w)', u (rho theta)) - hv d3, HV = -12 hv.
 template <typename Row>
-__device__ __forceinline__ void flux_x(const double s[4][4], const Row& r, double HV, unsigned mask, double F[4]) {
-  double A[4], D[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) interp(s[q][0], s[q][1], s[q][2], s[q][3], A[q], D[q]);
-  const double ri = rcp(A[DENS] + rowd(r).R12, mask);
-  const double u = A[UMOM] * ri;
-  F[0] = fma(HV, D[DENS], A[UMOM]);
-  F[1] = fma(A[UMOM], u, pressure(A[RHOT], r, HV * D[UMOM], mask));
-  F[2] = fma(u, A[WMOM], HV * D[WMOM]);
-  F[3] = fma(u, A[RHOT] + rowd(r).RT12, HV * D[RHOT]);
+__device__ __forceinline__ void flux_x(const double A[4], const double D[4], const Row& r, double HV, double IHV,
+                                       unsigned mask, double F[4]) {
+  const double u = A[UMOM] * rcp(fma(HV, A[DENS], rowd(r).R), mask);  // u / HV
+  F[0] = fma(IHV, A[UMOM], D[DENS]);
+  F[1] = fma(A[UMOM], u, pressure(A[RHOT], r, D[UMOM], mask));
+  F[2] = fma(u, A[WMOM], D[WMOM]);
+  F[3] = fma(u, A[RHOT] + rowd(r).RT12, D[RHOT]);
 }
 
-// z flux times 12 (interpolate.py:132-186); w and d3[DENS] vanish at the walls.
+// z flux times 12 / HV (interpolate.py:132-186); w and d3[DENS] vanish at the walls.
 template <typename Row>
-__device__ __forceinline__ void flux_z(const double s[4][4], const Row& r, double HV, bool wall, unsigned mask,
-                                       double F[4]) {
-  double A[4], D[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) interp(s[q][0], s[q][1], s[q][2], s[q][3], A[q], D[q]);
-  double AW = A[WMOM];
-  if (wall) {
-    AW = 0.0;
-    D[DENS] = 0.0;
-  }
-  const double ri = rcp(A[DENS] + rowd(r).R12, mask);
-  const double w = AW * ri;
-  F[0] = fma(HV, D[DENS], AW);
-  F[1] = fma(w, A[UMOM], HV * D[UMOM]);
-  F[2] = fma(AW, w, pressure(A[RHOT], r, HV * D[WMOM], mask));
-  F[3] = fma(w, A[RHOT] + rowd(r).RT12, HV * D[RHOT]);
+__device__ __forceinline__ void flux_z(const double A[4], const double D[4], const Row& r, double HV, double IHV,
+                                       bool wall, unsigned mask, double F[4]) {
+  const double AW = wall ? 0.0 : A[WMOM];
+  const double w = AW * rcp(fma(HV, A[DENS], rowd(r).R), mask);  // w / HV
+  F[0] = fma(IHV, AW, wall ? 0.0 : D[DENS]);
+  F[1] = fma(w, A[UMOM], D[UMOM]);
+  F[2] = fma(AW, w, pressure(A[RHOT], r, D[WMOM], mask));
+  F[3] = fma(w, A[RHOT] + rowd(r).RT12, D[RHOT]);
 }
 
 // ---- arguments -------------------------------------------------------------
@@ -197,7 +198,8 @@ struct Args {
   double* out;
   unsigned flags;
   double HV;    // -12 hv, hv = -hv_beta d / (16 dt_full) (interpolate.py:101,149)
-  double c;     // dt_stage / (12 d)
+  double IHV;   // 1 / HV
+  double c;     // HV dt_stage / (12 d)
   double dt;    // dt_stage (source terms)
   double gdt;   // -dt_stage grav (z)
   int z_tile;
@@ -236,143 +238,155 @@ __device__ __forceinline__ void write_z_halo_column(const Args& a, int col, bool
 }
 
 // ---- x ---------------------------------------------------------------------
-// x, warp segments: the CTA owns the contiguous range [g0, g1) of the
-// row-major list of 63-cell segments (nseg per row) and splits it evenly over
-// its eight warps, which walk their segments with no CTA barrier.  Lane l
-// evaluates the fluxes at interfaces x0+l and x0+32+l (two independent FP64
-// chains) from the segment's values staged in the warp's shared-memory slice,
-// and updates cells x0+l and x0+32+l (l < 31) from its own and the next
-// lane's fluxes.  The next segment's values are loaded one segment ahead; the
-// row constants (an FP64 pow per row) are tabled once per CTA.
-constexpr int kWI = 64;             // interfaces per warp segment
-constexpr int kWCells = kWI - 1;    // cells per warp segment
+// A row is cut into runs of equal length (the last one shorter), one warp per
+// run.  The warp walks the run in blocks of 64 slots with no CTA barrier: slot
+// j of block b holds cell i = c0 - 1 + 64 b + j (lane l has slots l and 32 + l,
+// two independent FP64 chains), forms the cell's e and q, the flux at the
+// interface i between cells i - 1 and i, and updates cell i - 1.  e, q and the
+// flux of slot j - 1 come from the lane before, or for slot 0 from slot 63 of
+// the block before, so a run of n cells takes n + 2 slots.  The values of the
+// next block are loaded one block ahead.
+constexpr int kWSlots = 64;         // slots per block
 constexpr int kXWarps = kXT / 32;
-constexpr int kXRowsMax = 64;       // rows of one CTA's range
+constexpr int kXRowsMax = kXWarps;  // rows of one CTA's runs
 struct SmemXW {
-  double sS[kXWarps][4][kWI + 4];   // [warp][variable][cell x0-2 .. x0+64]
+  double sS[kXWarps][4][kWSlots + 2];  // [warp][variable][cell i0-1 .. i0+64], i0 the cell of slot 0
 };
+__host__ __device__ inline int run_blocks(int cells) { return (cells + 2 + kWSlots - 1) / kWSlots; }
 
-// Walks the segments [g0, g1) of the row-major list of kWCells-cell segments
-// (nseg per row); row_at(k) gives the constants of row k.  Every lane of the
-// warp calls it; prologue() runs once, after the first segment's loads are
-// issued (so that their latency overlaps it), also when the range is empty
-// (it may contain a CTA barrier).  sS is the warp's shared-memory slice.
+// Walks runs [g0, g1) of the row-major list of runs of `len` cells (nrun per
+// row); row_at(k) gives the constants of row k.  Every lane of the warp calls
+// it; prologue() runs once, after the first block's loads are issued (so that
+// their latency overlaps it), also when the range is empty (it may contain a
+// CTA barrier).  sS is the warp's shared-memory slice.
 template <typename RowAt, typename Prologue>
-__device__ __forceinline__ void x_warp_walk(const Args& a, int nseg, long long g0, long long g1, RowAt row_at,
-                                            bool halo, double (*sS)[kWI + 4], Prologue prologue) {
+__device__ __forceinline__ void x_warp_walk(const Args& a, int nrun, int len, long long g0, long long g1, RowAt row_at,
+                                            bool halo, double (*sS)[kWSlots + 2], Prologue prologue) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  // values of the segment in row k at x0: cells x0-2+lane, x0+30+lane and (lanes 0..2) x0+62+lane
-  auto load = [&](int k, int x0, double v[3][4]) {
+  // values of the block of row k whose slot 0 is cell i0: cells i0-1+lane, i0+31+lane and (lanes 0, 1)
+  // i0+63+lane; slots beyond the run hold valid values that nothing uses
+  auto load = [&](int k, int i0, double v[3][4]) {
     const long long row = (long long)(k + kHs) * a.pitch;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const int c = x0 - 2 + 32 * j + lane;
-      if ((j < 2 || lane < 3) && c <= a.nx + 1) {
-        const long long col = wrap_x(c, a.nx) + kHs;
+      if (j < 2 || lane < 2) {
+        const long long col = wrap_x(min(i0 - 1 + 32 * j + lane, a.nx + 1), a.nx) + kHs;
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[j][q] = __ldg(&MW_F(a, q * a.plane + row + col));
       }
     }
   };
-  // (row, segment in row) of the current segment, advanced incrementally (one
-  // 64-bit division per walk, not per segment)
-  int k = (int)(g0 / nseg), sg = (int)(g0 - (long long)k * nseg);
+  int k = (int)(g0 / nrun), rn = (int)(g0 - (long long)k * nrun);  // the current run: its row and place in the row
+  int c0 = rn * len, c1 = min(c0 + len, a.nx), b = 0;
   double v[3][4] = {};
-  if (g0 < g1) load(k, sg * kWCells, v);
+  if (g0 < g1) load(k, c0 - 1, v);
   prologue();
-  for (long long g = g0; g < g1; ++g) {
-    const int x0 = sg * kWCells;
-    const int kn = sg + 1 == nseg ? k + 1 : k, sgn = sg + 1 == nseg ? 0 : sg + 1;  // the next segment
+  double ce[4], cq[4], cF[4];  // e, q and flux of slots 32 .. 63 of the block before
+#pragma unroll
+  for (int q = 0; q < 4; ++q) ce[q] = cq[q] = cF[q] = 0.0;
+  for (long long g = g0; g < g1;) {
+    const int i0 = c0 - 1 + kWSlots * b;
     const long long row = (long long)(k + kHs) * a.pitch;
-    __syncwarp();  // the previous segment's taps are read
+    __syncwarp();  // the previous block's values are read
 #pragma unroll
     for (int j = 0; j < 3; ++j)
-      if (j < 2 || lane < 3)
+      if (j < 2 || lane < 2)
 #pragma unroll
         for (int q = 0; q < 4; ++q) sS[q][32 * j + lane] = v[j][q];
-    if (halo && sg == 0 && lane < 4) {  // columns 0, 1 <- nx, nx+1; nx+2, nx+3 <- 2, 3 (ics/bcs.py:35-39)
+    if (halo && rn == 0 && b == 0 && lane < 4) {  // columns 0, 1 <- nx, nx+1; nx+2, nx+3 <- 2, 3 (ics/bcs.py:35-39)
       const int dst = lane < 2 ? lane : a.nx + lane, src = lane < 2 ? a.nx + lane : lane;
 #pragma unroll
       for (int q = 0; q < 4; ++q) MW_F(a, q * a.plane + row + dst) = MW_F(a, q * a.plane + row + src);
     }
-    if (g + 1 < g1) load(kn, sgn * kWCells, v);
-    const int ia = x0 + lane, ib = x0 + 32 + lane;  // interfaces (and cells) of this lane
-    const bool ua = ia < a.nx, ub = lane < 31 && ib < a.nx;
+    // cells updated by this lane
+    const int ca = i0 - 1 + lane, cb = ca + 32;
+    const bool ua = ca >= c0 && ca < c1, ub = cb < c1;
     double iva[4], ivb[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      if (ua) iva[q] = MW_AT(a.init, q * a.plane + row + ia + kHs, 4 * a.plane);
-      if (ub) ivb[q] = MW_AT(a.init, q * a.plane + row + ib + kHs, 4 * a.plane);
+      if (ua) iva[q] = MW_AT(a.init, q * a.plane + row + ca + kHs, 4 * a.plane);
+      if (ub) ivb[q] = MW_AT(a.init, q * a.plane + row + cb + kHs, 4 * a.plane);
     }
+    const bool first = b == 0;
+    const int kc = k;
+    // the next block: of this run, of the row's next run, or of the next row's first run
+    if (++b == run_blocks(c1 - c0)) {
+      b = 0;
+      ++g;
+      if (++rn == nrun) {
+        rn = 0;
+        ++k;
+      }
+      c0 = rn * len;
+      c1 = min(c0 + len, a.nx);
+    }
+    if (g < g1) load(k, c0 - 1 + kWSlots * b, v);
     __syncwarp();
-    const auto& rc = row_at(k);
-    double Fa[4] = {0, 0, 0, 0}, Fb[4] = {0, 0, 0, 0};
-    const unsigned ma = __ballot_sync(0xffffffffu, ia <= a.nx), mb = __ballot_sync(0xffffffffu, ib <= a.nx);
-    if (ia <= a.nx) {
-      double s[4][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[q][j] = sS[q][lane + j];
-      flux_x(s, rc, a.HV, ma, Fa);
-    }
-    if (ib <= a.nx) {
-      double s[4][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[q][j] = sS[q][32 + lane + j];
-      flux_x(s, rc, a.HV, mb, Fb);
-    }
-    // lane l needs the flux at interface x0+l+1: lane l+1's Fa, or for l = 31 lane 0's Fb
-    double Fa1[4], Fb1[4];
+    const auto& rc = row_at(kc);
+    const int prev = (lane + 31) & 31;
+    double Aa[4], Da[4], Ab[4], Db[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      Fa1[q] = __shfl_sync(0xffffffffu, lane == 0 ? Fb[q] : Fa[q], (lane + 1) & 31);
-      Fb1[q] = __shfl_down_sync(0xffffffffu, Fb[q], 1);
+      double ea, qa, eb, qb;
+      cell_eq(sS[q][lane], sS[q][lane + 1], sS[q][lane + 2], ea, qa);
+      cell_eq(sS[q][32 + lane], sS[q][33 + lane], sS[q][34 + lane], eb, qb);
+      double ep = __shfl_sync(kAll, lane == 31 ? ce[q] : ea, prev);
+      double qp = __shfl_sync(kAll, lane == 31 ? cq[q] : qa, prev);
+      if (first && lane == 0) {  // no cell before the run's first: its flux is not used
+        ep = ea;
+        qp = qa;
+      }
+      Aa[q] = qp + qa;
+      Da[q] = ea - ep;
+      Ab[q] = __shfl_sync(kAll, lane == 31 ? qa : qb, prev) + qb;
+      Db[q] = eb - __shfl_sync(kAll, lane == 31 ? ea : eb, prev);
+      ce[q] = eb;
+      cq[q] = qb;
     }
-    if (ua) {
+    double Fa[4], Fb[4];
+    flux_x(Aa, Da, rc, a.HV, a.IHV, kAll, Fa);
+    flux_x(Ab, Db, rc, a.HV, a.IHV, kAll, Fb);
+    // the flux at interface i - 1: the lane before's
+    double Fpa[4], Fpb[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      Fpa[q] = __shfl_sync(kAll, lane == 31 ? cF[q] : Fa[q], prev);
+      Fpb[q] = __shfl_sync(kAll, lane == 31 ? Fa[q] : Fb[q], prev);
+      cF[q] = Fb[q];
+    }
+    auto update = [&](int c, const double* Fp, const double* F, const double* iv) {
       double o[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = fma(a.c, Fa[q] - Fa1[q], iva[q]);
-      if (a.srcw) o[WMOM] = fma(a.dt, MW_AT(a.srcw, (long long)k * a.nx + ia, (long long)a.nx * a.nz), o[WMOM]);
+      for (int q = 0; q < 4; ++q) o[q] = fma(a.c, Fp[q] - F[q], iv[q]);
+      if (a.srcw) o[WMOM] = fma(a.dt, MW_AT(a.srcw, (long long)kc * a.nx + c, (long long)a.nx * a.nz), o[WMOM]);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) MW_AT(a.out, q * a.plane + row + ia + kHs, 4 * a.plane) = o[q];
-    }
-    if (ub) {
-      double o[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = fma(a.c, Fb[q] - Fb1[q], ivb[q]);
-      if (a.srcw) o[WMOM] = fma(a.dt, MW_AT(a.srcw, (long long)k * a.nx + ib, (long long)a.nx * a.nz), o[WMOM]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) MW_AT(a.out, q * a.plane + row + ib + kHs, 4 * a.plane) = o[q];
-    }
-    k = kn;
-    sg = sgn;
+      for (int q = 0; q < 4; ++q) MW_AT(a.out, q * a.plane + row + c + kHs, 4 * a.plane) = o[q];
+    };
+    if (ua) update(ca, Fpa, Fa, iva);
+    if (ub) update(cb, Fpb, Fb, ivb);
   }
 }
 
 #ifndef MW_IEEE_X_MIN_BLOCKS
 #define MW_IEEE_X_MIN_BLOCKS 2
 #endif
-// Single grid: the CTA owns the contiguous range [g0, g1) of segments of rows
-// [r0, r1) and splits it evenly over its warps; the row constants (an FP64 pow
-// per row) are tabled once per CTA while the warps' first loads are in flight.
-__global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Args a, int nseg, long long total,
-                                                                               long long gbase) {
+// Single grid: one run per warp, eight consecutive runs of rows [r0, r1) per
+// CTA; the row constants (an FP64 pow per row) are tabled once per CTA while
+// the warps' first loads are in flight.
+__global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Args a, int nrun, int len, long long g0,
+                                                                               long long g1) {
   __shared__ SmemXW sm;
   __shared__ RowP rows[kXRowsMax];
-  const long long g0 = gbase + total * blockIdx.x / gridDim.x, g1 = gbase + total * (blockIdx.x + 1) / gridDim.x;
-  if (g0 >= g1) return;
-  const int row0 = (int)(g0 / nseg), nrows = (int)((g1 - 1) / nseg) - row0 + 1;  // nrows <= kXRowsMax (host)
+  const long long b0 = g0 + (long long)blockIdx.x * kXWarps, b1 = min(b0 + kXWarps, g1);
+  const int row0 = (int)(b0 / nrun), nrows = (int)((b1 - 1) / nrun) - row0 + 1;  // nrows <= kXRowsMax
   const int w = threadIdx.x >> 5;
-  const long long n = g1 - g0;
-  x_warp_walk(a, nseg, g0 + n * w / kXWarps, g0 + n * (w + 1) / kXWarps,
-              [&](int k) -> const RowP& { return rows[k - row0]; },
+  x_warp_walk(a, nrun, len, min(b0 + w, b1), min(b0 + w + 1, b1), [&](int k) -> const RowP& { return rows[k - row0]; },
               a.flags & MW_FLAG_WRITE_HALO, sm.sS[w], [&]() {
                 for (int r = threadIdx.x; r < nrows; r += kXT) {
                   const double rt = MW_AT(a.hytc, row0 + r + kHs, a.nz + 2 * kHs);
-                  rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow(rt, kGamma));
+                  rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow(rt, kGamma),
+                                         a.HV, a.IHV);
                 }
                 __syncthreads();
               });
@@ -390,7 +404,8 @@ template <int NC>
 __device__ __forceinline__ void z_tile(const Args& a, int cb, int z0, int z1, bool hbot, bool htop, SmemZ& sm) {
   for (int rr = threadIdx.x; rr <= z1 - z0; rr += NC) {
     const int k = z0 + rr;
-    sm.row[rr] = row_consts_p(MW_AT(a.hyi, k, a.nz + 1), MW_AT(a.hyti, k, a.nz + 1), MW_AT(a.hypi, k, a.nz + 1));
+    sm.row[rr] = row_consts_p(MW_AT(a.hyi, k, a.nz + 1), MW_AT(a.hyti, k, a.nz + 1), MW_AT(a.hypi, k, a.nz + 1), a.HV,
+                              a.IHV);
   }
   __syncthreads();
   const int c = cb * NC + threadIdx.x;  // interior column
@@ -400,35 +415,44 @@ __device__ __forceinline__ void z_tile(const Args& a, int cb, int z0, int z1, bo
   if (c < a.nx) {
     const int col = c + kHs;
     if (hbot || htop) write_z_halo_column(a, col, hbot, htop);
-    double w[4][4];
+    // s(k), s(k+1) and the e, q of cell k, k the row of the flux Fp just formed
+    double s0[4], s1[4], e[4], qv[4], nxt[4], A[4], D[4], Fp[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w[q][j] = zval(a, q, z0 - 2 + j, col);
-    double nxt[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) nxt[q] = zval(a, q, z0 + 2, col);
-    double Fp[4];
-    flux_z(w, sm.row[0], a.HV, z0 == 0, mask, Fp);
+    for (int q = 0; q < 4; ++q) {
+      const double sm2 = zval(a, q, z0 - 2, col), sm1 = zval(a, q, z0 - 1, col);
+      s0[q] = zval(a, q, z0, col);
+      s1[q] = zval(a, q, z0 + 1, col);
+      nxt[q] = zval(a, q, z0 + 2, col);
+      double e0, q0;
+      cell_eq(sm2, sm1, s0[q], e0, q0);
+      cell_eq(sm1, s0[q], s1[q], e[q], qv[q]);
+      A[q] = q0 + qv[q];
+      D[q] = e[q] - e0;
+    }
+    flux_z(A, D, sm.row[0], a.HV, a.IHV, z0 == 0, mask, Fp);
     for (int k = z0; k < z1; ++k) {
       const long long o = (long long)(k + kHs) * a.pitch + col;
       double iv[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) iv[q] = MW_AT(a.init, q * a.plane + o, 4 * a.plane);
-      const double rho_k = w[DENS][2];  // forcing rho' at cell k (interpolate.py:248-250)
+      const double rho_k = s0[DENS];  // forcing rho' at cell k (interpolate.py:248-250)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        w[q][0] = w[q][1];
-        w[q][1] = w[q][2];
-        w[q][2] = w[q][3];
-        w[q][3] = nxt[q];
+        double en, qn;
+        cell_eq(s0[q], s1[q], nxt[q], en, qn);  // cell k + 1
+        A[q] = qv[q] + qn;
+        D[q] = en - e[q];
+        e[q] = en;
+        qv[q] = qn;
+        s0[q] = s1[q];
+        s1[q] = nxt[q];
       }
       if (k + 1 < z1) {  // the row the next iteration needs, loaded one step ahead
 #pragma unroll
         for (int q = 0; q < 4; ++q) nxt[q] = zval(a, q, k + 3, col);
       }
       double Fn[4];
-      flux_z(w, sm.row[k + 1 - z0], a.HV, k + 1 == a.nz, mask, Fn);
+      flux_z(A, D, sm.row[k + 1 - z0], a.HV, a.IHV, k + 1 == a.nz, mask, Fn);
       double v[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) v[q] = fma(a.c, Fp[q] - Fn[q], iv[q]);
@@ -478,9 +502,10 @@ __device__ __forceinline__ Args member_args(const EnsStage& es, int e) {
   const EnsMemberConsts& c = MW_AT(reinterpret_cast<const EnsMemberConsts*>(es.mconsts), mconsts_index(es, e),
                                    (long long)kEnsConstsPerMember * es.n_members);
   a.HV = c.HV;
+  a.IHV = c.IHV;
   a.c = c.c;
   a.dt = c.dt;
-  a.gdt = c.gdt;
+  a.gdt = -c.dt * kGrav;
   a.z_tile = es.z_tile;
   a.r0 = 0;
   a.r1 = m.nz;
@@ -489,26 +514,27 @@ __device__ __forceinline__ Args member_args(const EnsStage& es, int e) {
 
 static_assert(sizeof(RowD) <= kEnsRowBytes, "row-constant table entry size");
 
+// The members' HV differ, so the table holds the constants for HV = 1; a warp scales its row's.
 __global__ void k_ens_row_table_ieee(const double* hyc, const double* hytc, long long n, RowD* table) {
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
     const double rt = MW_AT(hytc, j, n);
-    MW_AT(table, j, n) = row_consts(MW_AT(hyc, j, n), rt, kC0 * pow(rt, kGamma));
+    MW_AT(table, j, n) = row_consts(MW_AT(hyc, j, n), rt, kC0 * pow(rt, kGamma), 1.0, 1.0);
   }
 }
 
-// x items are rows (member, row), one per warp: the warp walks the row's
-// segments as the single-grid kernel does.
+// x items are rows (member, row), one per warp: the warp walks the row as one run.
 __global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_ens_x_ieee(EnsStage es) {
   __shared__ SmemXW sm;
   const int w = threadIdx.x >> 5;
   for (unsigned it = ens_take_warp(es.cursor); it < (unsigned)es.n_items; it = ens_take_warp(es.cursor)) {
     const int2 item = MW_AT(es.items, it, es.n_items);  // (member, row)
     const Args a = member_args(es, item.x);
-    const int nseg = (a.nx + kWCells - 1) / kWCells;
-    const RowD r = MW_AT(reinterpret_cast<const RowD*>(es.xrows),
-                         MW_AT(es.members, item.x, es.n_members).cell_off + item.y + kHs, es.n_xrows);
-    x_warp_walk(a, nseg, (long long)item.y * nseg, (long long)(item.y + 1) * nseg,
-                [&](int) -> const RowD& { return r; },
+    RowD r = MW_AT(reinterpret_cast<const RowD*>(es.xrows),
+                   MW_AT(es.members, item.x, es.n_members).cell_off + item.y + kHs, es.n_xrows);
+    r.R *= a.HV;
+    r.P *= a.IHV;
+    r.PC1 *= a.IHV;
+    x_warp_walk(a, 1, a.nx, (long long)item.y, (long long)item.y + 1, [&](int) -> const RowD& { return r; },
                 a.flags & MW_FLAG_WRITE_HALO, sm.sS[w], []() {});
   }
   ens_finish(es.cursor);
@@ -604,8 +630,9 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
   a.out = out;
   a.flags = flags;
   const double d = direction == MW_DIR_X ? dx : dz;
-  a.HV = 12.0 * kHvBeta * d / (16 * dt_full);  // -12 hv
-  a.c = dt_stage / (12.0 * d);
+  a.HV = ieee_hv(d, dt_full);
+  a.IHV = 1.0 / a.HV;
+  a.c = dt_stage / (12.0 * d) * a.HV;
   a.dt = dt_stage;
   a.gdt = -dt_stage * kGrav;
   a.r0 = r0;
@@ -627,19 +654,31 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     a.z_tile = kZTileMax;
   }
   if (direction == MW_DIR_X) {
-    // About MW_IEEE_X_SEGS_PER_WARP segments per warp in a whole number of
-    // resident waves of equal ranges (one wave, at least one segment per warp,
-    // for small grids); at most kXRowsMax rows per CTA range.
-    const int nseg = (nx + kWCells - 1) / kWCells;
-    const long long total = (long long)nseg * rows;
+    // Runs per row: a warp's time is its blocks (and about a third of one to
+    // start a run), and an SM's partitions each take two warps of every CTA it
+    // gets, so the row is cut where ceil(CTAs / SMs) x (blocks + 1/3) is least
+    // -- at most kXRunBlocksMax blocks, which leaves a large grid several waves.
     int resident = 0, st = resident_ctas(0, &resident);
     if (st) return st;
-    long long grid = std::min<long long>(resident, (total + kXWarps - 1) / kXWarps);
-    grid = std::max<long long>(grid, total / (kXWarps * MW_IEEE_X_SEGS_PER_WARP));
-    if (grid > resident) grid = (grid + resident - 1) / resident * resident;
-    grid = std::max<long long>(grid, (rows + kXRowsMax - 3) / (kXRowsMax - 2));
+    const long long sms = std::max(1, resident / MW_IEEE_X_MIN_BLOCKS);
+    int nrun = 1;
+    double best = 0.0;
+    for (int n = (nx + kXRunBlocksMax * kWSlots - 1) / (kXRunBlocksMax * kWSlots);
+         n <= (nx + kWSlots - 3) / (kWSlots - 2); ++n) {
+      const int blocks = run_blocks((nx + n - 1) / n);
+      const long long ctas = ((long long)n * rows + kXWarps - 1) / kXWarps;
+      const double cost = (double)((ctas + sms - 1) / sms) * (blocks + 1.0 / 3);
+      if (best == 0.0 || cost < best) {
+        best = cost;
+        nrun = n;
+      }
+    }
+    const int len = (nx + nrun - 1) / nrun;
+    nrun = (nx + len - 1) / len;
+    const long long g0 = (long long)r0 * nrun, g1 = (long long)r1 * nrun;
+    const long long grid = (g1 - g0 + kXWarps - 1) / kXWarps;
     MW_REQUIRE(grid <= 0x7fffffffLL, MW_ERR_SHAPE, "grid too large for the x direction-stage launch");
-    k_stage_x_ieee_w<<<(unsigned)grid, kXT, 0, stream>>>(a, nseg, total, (long long)r0 * nseg);
+    k_stage_x_ieee_w<<<(unsigned)grid, kXT, 0, stream>>>(a, nrun, len, g0, g1);
   } else {
     const int ntiles = (rows + a.z_tile - 1) / a.z_tile;
     for (int t0 = 0; t0 < ntiles; t0 += 65535) {
