@@ -28,6 +28,7 @@
 
 #include "mw_common.cuh"
 #include "mw_ensemble.cuh"
+#include "mw_fp64_line.cuh"
 #include "mw_split.cuh"
 
 namespace mw {
@@ -1174,6 +1175,34 @@ static int run_steps(double dt, T* S, T* Tmp, T* A, int nsteps, int* reverse, St
   return MW_OK;
 }
 
+// nsteps FP64 steps of validated arguments: one launch per direction where the
+// IEEE-FP64 line kernels take the grid, else one per direction-stage.
+static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, double dt, const double* hyc,
+                     const double* hytc, const double* hyi, const double* hyti, const double* hypi,
+                     const double* src_w, double* state, double* state_tmp, double* scratch, int nsteps, int* reverse,
+                     int f64_mode, unsigned flags, cudaStream_t s) {
+  if (f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)) {
+    const bool halo = flags & MW_FLAG_WRITE_HALO;
+    LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, state, state, nullptr, nullptr, halo ? state : nullptr,
+               halo ? state_tmp : nullptr};
+    for (int n = 0; n < nsteps; ++n) {
+      for (int d = 0; d < 2; ++d) {
+        a.s2 = n + 1 == nsteps && d == 1 ? state_tmp : nullptr;  // what the call leaves in state_tmp
+        const int st = launch_line_ieee(nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
+                                        n + d > 0, s);
+        if (st) return st;
+      }
+      *reverse = *reverse ? 0 : 1;
+    }
+    return MW_OK;
+  }
+  return run_steps<double>(dt, state, state_tmp, scratch, nsteps, reverse,
+                           [&](const double* init, double* forcing, double* out, double dts, int dir, int k) {
+                             return stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init,
+                                              forcing, out, dts, dir, f64_mode, flags, s, split_step_fmt(k));
+                           });
+}
+
 template <typename T>
 static int validate_step(int nx, int nz, double dx, double dz, double dt, const double* hyc, const double* hytc,
                          const double* hyi, const double* hyti, const double* hypi, const T* S, const T* Tmp,
@@ -1245,11 +1274,8 @@ extern "C" int mw_step_f64(int nx, int nz, double dx, double dz, double dt_full,
   MW_REQUIRE(valid_f64_mode(f64_mode), MW_ERR_INVALID_ARG, "unknown f64_mode %d",
              f64_mode);
   cudaStream_t s = (cudaStream_t)stream;
-  st = run_steps<double>(dt, state, state_tmp, scratch, nsteps, reverse,
-                         [&](const double* init, double* forcing, double* out, double dts, int dir, int k) {
-                           return stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init, forcing,
-                                            out, dts, dir, f64_mode, flags, s, split_step_fmt(k));
-                         });
+  st = steps_f64(nx, nz, dx, dz, dt_full, dt, hyc, hytc, hyi, hyti, hypi, src_w, state, state_tmp, scratch, nsteps,
+                 reverse, f64_mode, flags, s);
   if (st == MW_OK && nsteps > 0 && (flags & MW_FLAG_CHECK_FINITE)) st = check_finite_blocking(nx, nz, (const double*)state, scratch, s);
   return st;
 }
@@ -1343,11 +1369,8 @@ extern "C" int mw_step_f64_noalloc(int nx, int nz, double dx, double dz, double 
   MW_REQUIRE(valid_f64_mode(f64_mode), MW_ERR_INVALID_ARG, "unknown f64_mode %d",
              f64_mode);
   cudaStream_t s = (cudaStream_t)stream;
-  st = run_steps<double>(dt, state, state_tmp, scratch, nsteps, reverse,
-                         [&](const double* init, double* forcing, double* out, double dts, int dir, int k) {
-                           return stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init,
-                                            forcing, out, dts, dir, f64_mode, flags, s, split_step_fmt(k));
-                         });
+  st = steps_f64(nx, nz, dx, dz, dt_full, dt, hyc, hytc, hyi, hyti, hypi, src_w, state, state_tmp, scratch, nsteps,
+                 reverse, f64_mode, flags, s);
   // the finite check counts into the first 8 bytes of the built-in array (no allocation)
   if (st == MW_OK && nsteps > 0 && (flags & MW_FLAG_CHECK_FINITE)) st = check_finite_blocking(nx, nz, (const double*)state, scratch, s);
   return st;
@@ -1374,6 +1397,15 @@ extern "C" int mw_step_record_f64(int nx, int nz, double dx, double dz, double d
   cudaError_t e = cudaMemcpyAsync(stages, state_in, n * sizeof(double), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "stage copy: %s", cudaGetErrorString(e));
   const int dirs[2] = {reverse ? MW_DIR_X : MW_DIR_Z, reverse ? MW_DIR_Z : MW_DIR_X};
+  if (f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)) {
+    for (int d = 0; d < 2; ++d) {
+      double* S = stages + 3 * d * n;
+      const LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, S, d == 0 ? stages + 3 * n : state_out, S + n, S + 2 * n,
+                       nullptr, nullptr};
+      if ((st = launch_line_ieee(nx, nz, dx, dz, dt_full, dt, a, dirs[d], d > 0, s))) return st;
+    }
+    return MW_OK;
+  }
   for (int d = 0; d < 2; ++d) {
     double* S = stages + (3 * d) * n;
     double* s1 = S + n;

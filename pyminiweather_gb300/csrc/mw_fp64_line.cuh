@@ -1,0 +1,41 @@
+// mw_fp64_line.cuh -- the line kernels' interface (mw_fp64_line.cu): one
+// direction of a time step, all three RK stages, in one launch.
+#pragma once
+
+#include "mw_common.cuh"
+
+namespace mw {
+
+// Most cells of a grid that takes the line kernels: above this the CTAs of a
+// launch come in several waves and the stage kernels, which need no whole lines
+// in a CTA, do as well (us per step, line kernels / six stage launches replayed
+// from a graph: 100x50 22 / 121, 300x150 38 / 122, 512x256 120 / 145, 512x512
+// 237 / 240, 700x700 382 / 380, 992x992 671 / 663).
+constexpr long long kLineCellsMax = 400000;
+
+struct LineArgs {
+  const double* hyc;
+  const double* hytc;
+  const double* hyi;
+  const double* hyti;
+  const double* hypi;
+  const double* srcw;  // optional forcing of w
+  const double* in;    // the direction's initial state
+  double* out;         // its result (may be `in`: every CTA reads its lines before it writes them)
+  double* s1;          // first and second stage, each optional
+  double* s2;
+  double* halo_in;     // optional: arrays that get the direction's halo of the initial state
+  double* halo_tmp;    // and of the second stage
+};
+
+// Whether grids of nx x nz cells take the line kernels.
+bool line_ieee_fits(int nx, int nz);
+
+// One direction of one step of size dt.  overlap: the kernel may start while
+// the one before it on the stream is finishing, and waits for it before it
+// touches the state; only for a launch behind another line kernel of the same
+// call (what it reads before the wait, the backgrounds, is then complete).
+int launch_line_ieee(int nx, int nz, double dx, double dz, double dt_full, double dt, const LineArgs& a, int direction,
+                     bool overlap, cudaStream_t stream);
+
+}  // namespace mw

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "mw_common.cuh"
+#include "mw_fp64_line.cuh"
 
 namespace mw {
 
@@ -124,15 +125,19 @@ extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_
   const Geom g = make_geom(nx, nz);
   const size_t bytes = sizeof(double) * 4 * (size_t)g.plane;
   cudaStream_t s = (cudaStream_t)stream;
-  const int nb = std::max(1, std::min({nbands, kMaxBands, nz / 16}));
+  // grids of the line kernels (a direction per launch) are stepped whole, as mw_step_f64 steps them
+  const int nb = f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)
+                     ? 1
+                     : std::max(1, std::min({nbands, kMaxBands, nz / 16}));
   if ((f64_mode != MW_F64_SPLIT && f64_mode != MW_F64_IEEE) || nb == 1) {  // no bands: copy in, step, copy out
     cudaError_t e = cudaMemcpyAsync(state, h_in, bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "copy in: %s", cudaGetErrorString(e));
     if ((st = mw_step_f64(nx, nz, dx, dz, dt_full, dt, hyc, hytc, hyi, hyti, hypi, src_w, state, state_tmp, scratch, 1,
-                          reverse, f64_mode, flags, stream)))
+                          reverse, f64_mode, flags & ~MW_FLAG_CHECK_FINITE, stream)))
       return st;
     e = cudaMemcpyAsync(h_out, state, bytes, cudaMemcpyDeviceToHost, s);
-    return e == cudaSuccess ? MW_OK : fail(MW_ERR_CUDA, "copy out: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(MW_ERR_CUDA, "copy out: %s", cudaGetErrorString(e));
+    return flags & MW_FLAG_CHECK_FINITE ? check_finite_blocking(nx, nz, (const double*)state, scratch, s) : MW_OK;
   }
   std::lock_guard<std::mutex> lock(g_mu);
   CopyRes* c = nullptr;
