@@ -27,7 +27,7 @@
 #include <mutex>
 
 #include "mw_common.cuh"
-#include "mw_ensemble.cuh"
+#include "mw_f32_dir.cuh"
 #include "mw_fp64_line.cuh"
 #include "mw_split.cuh"
 
@@ -247,7 +247,7 @@ struct SmemXT {
   RowF row;
 };
 struct SmemZT {
-  RowF row[kEnsZTileMax + 1];
+  RowF row[kZTile + 1];
 };
 
 __device__ __forceinline__ RowF rowf_x(double hy_r, double hy_rt) {
@@ -336,24 +336,17 @@ __device__ __forceinline__ void x_rowrun_t(const StageArgs<T>& a, int k, int cbe
   }
 }
 
-// The plain-load FP32 passes wait on memory (one row or segment of loads in
-// flight per thread, no registers to spare for more): prefetch instructions
-// bring later rows / segments into L2 without holding registers.  Measured on
-// the 256-member thermal ensemble (ms per step): none 1.474, z 2 rows ahead
-// 1.410 (1, 3, 4, 8: 1.40-1.44 with x), x 1 segment 1.453, both (x 2, z 2) 1.393;
-// x 3 segments ahead 1.406, x prefetched into L1 instead of L2 1.391; the next
-// row taken one row early and its first lines prefetched 1.430.
+// The plain-load FP32 z pass waits on memory (one row of loads in flight per
+// thread, no registers to spare for more): prefetch instructions bring the rows
+// two steps ahead into L2 without holding registers.
 #ifndef MW_F32_PF_Z
 #define MW_F32_PF_Z 2  // FP32 z march: L2 prefetch of the rows this many steps ahead (0: none)
-#endif
-#ifndef MW_F32_PF_X
-#define MW_F32_PF_X 2  // FP32 ensemble x rows: L2 prefetch of the segment this many ahead (0: none)
 #endif
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// z: columns [cb*NC, cb*NC+NC) (NC threads), rows [z0, z0+zt), zt <= kEnsZTileMax; one
+// z: columns [cb*NC, cb*NC+NC) (NC threads), rows [z0, z0+zt), zt <= kZTile; one
 // thread per column marching the rows with a rolling 4-row window, the next
 // row loaded one step ahead.  halo: write the wall halo rows of these columns
 // (cb == 0 also does the four x-halo columns).
@@ -494,7 +487,7 @@ static __device__ unsigned long long g_bulk_timeouts;
 struct SmemZBulk {
   float f[kBulkStages][4][kBulkRows][kBulkCols];  // forcing rows
   float i[kBulkStages][4][kBulkRows][kBulkCols];  // init rows
-  RowF row[kEnsZTileMax + 1];
+  RowF row[kZTile + 1];
   unsigned long long full[kBulkStages];
 };
 
@@ -814,131 +807,6 @@ __global__ void __launch_bounds__(kBXThreads) k_stage_x_f32_bulk(StageArgs<float
     atomicAdd(&g_bulk_timeouts, 1ULL);
     for (int b = waited; b < issued; ++b) mbar_wait_bounded(&sm.full[b % kBXStages], (b / kBXStages) & 1);
   }
-}
-
-__device__ StageArgs<float> member_args_f32(const EnsStageT<float>& es, int e) {
-  const mw_ens_member m = MW_AT(es.members, e, es.n_members);
-  StageArgs<float> a;
-  a.nx = m.nx;
-  a.nz = m.nz;
-  a.pitch = m.nx + 2 * kHs;
-  a.plane = (long long)(m.nz + 2 * kHs) * a.pitch;
-  a.dx = m.dx;
-  a.dz = m.dz;
-  a.hv = 0.0;        // the FP32 kernels read hv_f, c_f, dt_f (below)
-  a.dt_stage = 0.0;
-  a.hyc = es.hyc + m.cell_off;
-  a.hytc = es.hytc + m.cell_off;
-  a.hyi = es.hyi + m.int_off;
-  a.hyti = es.hyti + m.int_off;
-  a.hypi = es.hypi + m.int_off;
-  a.srcw = nullptr;
-  a.init = es.init + m.state_off;
-  a.forcing = es.forcing + m.state_off;
-  a.out = es.out + m.state_off;
-  a.flags = es.flags;
-  a.chunks_per_block = 0;
-  a.z_tile = es.z_tile;
-  // hv_f, c_f, dt_f from the plan (formed on the host as set_f32_constants forms them)
-  const EnsMemberConsts& c = MW_AT(reinterpret_cast<const EnsMemberConsts*>(es.mconsts), mconsts_index(es, e),
-                                   (long long)kEnsConstsPerMember * es.n_members);
-  a.hv_f = c.hv_f;
-  a.c_f = c.c_f;
-  a.dt_f = c.dt_f;
-  return a;
-}
-
-// x items are rows (member, row), one per warp: lane l evaluates the flux at
-// interface x0+l of a 31-cell segment from its four taps (L1-resident loads)
-// and takes the flux of interface x0+l+1 from lane l+1 by a shuffle, so rows
-// of 64..1024 cells keep most lanes busy.
-constexpr int kF32WCells = 31;
-
-__device__ __forceinline__ void x_row_warp_f32(const StageArgs<float>& a, int k, bool halo) {
-  const int lane = threadIdx.x & 31;
-  const RowF r = rowf_x(MW_BC(a, hyc, k + kHs), MW_BC(a, hytc, k + kHs));
-  const long long row = (long long)(k + kHs) * a.pitch;
-  if (halo && lane < 4) {  // columns 0, 1 <- nx, nx+1; nx+2, nx+3 <- 2, 3
-    const int dst = lane < 2 ? lane : a.nx + lane, src = lane < 2 ? a.nx + lane : lane;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) MW_SF(a, q * a.plane + row + dst) = MW_SF(a, q * a.plane + row + src);
-  }
-  for (int x0 = 0; x0 < a.nx; x0 += kF32WCells) {
-    if (MW_F32_PF_X && x0 + MW_F32_PF_X * kF32WCells < a.nx && lane < 16) {  // a later segment's lines into L2
-      const int q = lane & 3;
-      const float* base = (lane & 4) ? a.init : a.forcing;
-      const int col = min(x0 + MW_F32_PF_X * kF32WCells + (lane >> 3) * 32, a.nx + 2 * kHs - 1);
-      prefetch_l2(base + q * a.plane + row + col);
-    }
-    const int i = x0 + lane;
-    const bool upd = lane < kF32WCells && i < a.nx;
-    const long long o = row + i + kHs;
-    float iv[4];
-    if (upd) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) iv[q] = MW_SI(a, q * a.plane + o);
-    }
-    float F[4] = {0.f, 0.f, 0.f, 0.f};
-    if (i <= a.nx) {
-      float s4[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const long long col = wrap_x(i - 2 + j, a.nx) + kHs;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) s4[q][j] = __ldg(&MW_SF(a, q * a.plane + row + col));
-      }
-      flux_x_f32(s4, r, a.hv_f, F);
-    }
-    float Fn[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) Fn[q] = __shfl_down_sync(0xffffffffu, F[q], 1);
-    if (upd) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) MW_SO(a, q * a.plane + o) = iv[q] + (F[q] - Fn[q]) * a.c_f;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kXThreads) k_ens_x_f32(EnsStageT<float> es) {
-  for (unsigned it = ens_take_warp(es.cursor); it < (unsigned)es.n_items; it = ens_take_warp(es.cursor)) {
-    const int2 item = MW_AT(es.items, it, es.n_items);  // (member, row)
-    const StageArgs<float> a = member_args_f32(es, item.x);
-    x_row_warp_f32(a, item.y, a.flags & MW_FLAG_WRITE_HALO);
-  }
-  ens_finish(es.cursor);
-}
-
-__global__ void __launch_bounds__(kEnsZCols) k_ens_z_f32(EnsStageT<float> es) {
-  __shared__ SmemZT sm;
-  __shared__ unsigned slot[2];
-  int parity = 0;
-  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)es.n_items;
-       it = ens_take_cta(es.cursor, slot, parity)) {
-    const int2 item = MW_AT(es.items, it, es.n_items);
-    const StageArgs<float> a = member_args_f32(es, item.x);
-    const int ncb = (a.nx + kEnsZCols - 1) / kEnsZCols;
-    const int cb = item.y % ncb, tile = item.y / ncb;
-    z_tile_t<float, MODE_F32, kEnsZCols>(a, cb, tile * es.z_tile, es.z_tile,
-                                         (a.flags & MW_FLAG_WRITE_HALO) && tile == 0, sm);
-  }
-  ens_finish(es.cursor);
-}
-
-int launch_ens_f32(const EnsStageT<float>& es, int grid) {
-  if (es.n_items == 0) return MW_OK;
-  if (es.direction == MW_DIR_X)
-    k_ens_x_f32<<<grid, kXThreads, 0, es.stream>>>(es);
-  else
-    k_ens_z_f32<<<grid, kEnsZCols, 0, es.stream>>>(es);
-  return check_launch("ensemble FP32 stage launch");
-}
-
-int ens_f32_occupancy(int direction, int* blocks_per_sm) {
-  cudaError_t e = direction == MW_DIR_X
-                      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_ens_x_f32, kXThreads, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_ens_z_f32, kEnsZCols, 0);
-  if (e != cudaSuccess) return fail(MW_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
-  return MW_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1290,11 +1158,18 @@ extern "C" int mw_step_f32(int nx, int nz, double dx, double dz, double dt_full,
   MW_REQUIRE(finite_pos(dt), MW_ERR_INVALID_ARG, "dt must be finite and positive");
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  st = run_steps<float>(dt, state, state_tmp, scratch, nsteps, reverse,
-                        [&](const float* init, float* forcing, float* out, double dts, int dir, int) {
-                          return launch_stage<float, MODE_F32>(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi,
-                                                               src_w, init, forcing, out, dts, dir, flags, s);
-                        });
+  const bool halo = flags & MW_FLAG_WRITE_HALO;
+  for (int n = 0; n < nsteps; ++n) {
+    for (int d = 0; d < 2; ++d) {  // state -> scratch -> state
+      const F32DirArgs a{hyc, hytc, hyi, hyti, hypi, src_w, d ? scratch : state, d ? state : scratch,
+                         n + 1 == nsteps && d == 1 ? state_tmp : nullptr, halo ? state : nullptr,
+                         halo ? state_tmp : nullptr};
+      if ((st = launch_dir_f32(nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
+                               n + d > 0, s)))
+        return st;
+    }
+    *reverse = *reverse ? 0 : 1;
+  }
   if (st == MW_OK && nsteps > 0 && (flags & MW_FLAG_CHECK_FINITE)) st = check_finite_blocking(nx, nz, (const float*)state, scratch, s);
   return st;
 }

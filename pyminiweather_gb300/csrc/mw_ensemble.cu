@@ -1,6 +1,6 @@
 // mw_ensemble.cu -- host side of the ensemble path: work plans and the time
 // step that advances every member with one persistent launch per
-// direction-stage (6 per step).
+// direction-stage (6 per step; FP32 form: one per direction, 2 per step).
 //
 // The plan lives in caller-provided device memory:
 //   [members: n x mw_ens_member][x items: int2 (member, row)]
@@ -23,6 +23,7 @@
 
 #include "mw_common.cuh"
 #include "mw_ensemble.cuh"
+#include "mw_f32_dir.cuh"
 #include "mw_split.cuh"
 
 namespace mw {
@@ -117,7 +118,7 @@ int ens_step(void* plan, const mw_ens_plan_info* info, const double* hyc, const 
     if ((st = occupancy(MW_DIR_Z, &b))) return st;
     grid_z = std::max(1, b) * sms;
   }
-  EnsStageT<T> es;
+  EnsStageT<T> es{};
   es.members = (const mw_ens_member*)((const char*)plan + info->members_off);
   es.cursor = (EnsCursor*)((char*)plan + ens_cursor_off(*info));
   es.z_tile = info->z_tile;
@@ -142,6 +143,17 @@ int ens_step(void* plan, const mw_ens_plan_info* info, const double* hyc, const 
       es.items = dirs[d] == MW_DIR_X ? xi : zi;
       es.n_items = dirs[d] == MW_DIR_X ? info->n_x_items : info->n_z_items;
       const int grid = dirs[d] == MW_DIR_X ? grid_x : grid_z;
+      if constexpr (std::is_same<T, float>::value) {  // one launch per direction, state -> scratch -> state
+        const bool halo = flags & MW_FLAG_WRITE_HALO;
+        es.init = d ? A : S;
+        es.out = d ? S : A;
+        es.s2 = n + 1 == nsteps && d == 1 ? Tmp : nullptr;
+        es.halo_in = halo ? S : nullptr;
+        es.halo_tmp = halo ? Tmp : nullptr;
+        es.stage_div = 3;  // the first stage's constants; the others' follow
+        if ((st = launch(es, grid))) return st;
+        continue;
+      }
       T* ins[3] = {S, S, S};
       T* frc[3] = {S, A, Tmp};
       T* outs[3] = {A, Tmp, S};
@@ -200,10 +212,11 @@ extern "C" int mw_ensemble_plan(int n_members, const mw_ens_member* members, int
         c.gz12[0] = gz12.h, c.gz12[1] = gz12.l;
         c.c12[0] = c12.h, c.c12[1] = c12.l;
         c.c12s = dts / (12.0 * d) * split::kTwoPow896;  // exact: a power-of-two scale
-        c.hv_f = (float)hv;
-        c.c_f = (float)(dts / d);
+        const F32Consts f = f32_consts(d, m.dt);  // as launch_dir_f32 forms them
+        c.hv_f = f.HV;
+        c.ihv_f = f.IHV;
+        c.c_f = f32_c(d, m.dt, dts);
         c.dt_f = (float)dts;
-        c.pad = 0.0f;
         c.HV = ieee_hv(d, m.dt);  // as launch_stage_ieee forms them
         c.IHV = 1.0 / c.HV;
         c.c = dts / (12.0 * d) * c.HV;

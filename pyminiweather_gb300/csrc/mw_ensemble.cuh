@@ -11,14 +11,14 @@ namespace mw {
 // Stage constants of one member for one direction-stage, formed on the host
 // when the plan is built, exactly as the single-grid launches form them.
 // Split form: (h, l) float pairs of 12 hv, 12 d, 12 dz g and dt_stage / (12 d),
-// and dt_stage / (12 d) * 2^896 in FP64.  FP32 form: hv, dt_stage / d and
-// dt_stage rounded to float.  IEEE-FP64 form: HV = -12 hv, 1 / HV,
+// and dt_stage / (12 d) * 2^896 in FP64.  FP32 form: HV, HV dt_stage / (2 d),
+// dt_stage and 1 / HV rounded to float (mw_f32_dir.cuh).  IEEE-FP64 form: HV = -12 hv, 1 / HV,
 // HV dt_stage / (12 d) and dt_stage.  Entry (member * 2 + (direction == z)) * 3 + stage
 // (stage 0, 1, 2: dt/3, dt/2, dt).
 struct EnsMemberConsts {
   float hv12[2], d12[2], gz12[2], c12[2];
   double c12s;
-  float hv_f, c_f, dt_f, pad;
+  float hv_f, c_f, dt_f, ihv_f;
   double HV, IHV, c, dt;
 };
 static_assert(sizeof(EnsMemberConsts) == 88, "EnsMemberConsts layout");
@@ -33,7 +33,8 @@ struct EnsCursor {
   unsigned next, done, pad[2];
 };
 
-// Arguments of one ensemble direction-stage launch (T = state storage type).
+// Arguments of one ensemble launch (T = state storage type): a direction-stage,
+// or in the FP32 form a direction.
 template <typename T>
 struct EnsStageT {
   const mw_ens_member* members;  // device
@@ -53,6 +54,9 @@ struct EnsStageT {
   const T* init;
   T* forcing;
   T* out;
+  T* s2;        // FP32 form (a launch takes a direction's three stages): second stage, and
+  T* halo_in;   // arrays that get the halos of the initial state and
+  T* halo_tmp;  // of the second stage (each may be NULL)
   const void* xrows;  // split form: row constants indexed like the cell-centre backgrounds
   long long n_xrows;  // entries of xrows
   const void* mconsts;  // EnsMemberConsts per (member, direction, stage), written with the plan

@@ -1,0 +1,44 @@
+// mw_f32_dir.cuh -- the FP32 direction kernels' interface (mw_f32_dir.cu).
+#pragma once
+
+#include "mw_common.cuh"
+
+namespace mw {
+
+struct F32DirArgs {
+  const double* hyc;
+  const double* hytc;
+  const double* hyi;
+  const double* hyti;
+  const double* hypi;
+  const double* srcw;  // optional forcing of w
+  const float* in;     // the direction's initial state
+  float* out;          // its result; must not overlap `in`
+  float* s2;           // second stage (optional)
+  float* halo_in;      // optional: arrays that get the direction's halo of the initial state
+  float* halo_tmp;     // and of the second stage
+};
+
+// HV = -2 hv of the FP32 form (hv = -hv_beta d / (16 dt_full)) and its
+// reciprocal, held in [2^-60, 2^110], where the fluxes over HV keep their range.
+struct F32Consts {
+  float HV, IHV;
+};
+inline double f32_hv(double d, double dt_full) {
+  return std::fmin(std::fmax(2.0 * kHvBeta * d / (16 * dt_full), 0x1p-60), 0x1p110);
+}
+inline F32Consts f32_consts(double d, double dt_full) {
+  const double hv = f32_hv(d, dt_full);
+  return {(float)hv, (float)(1.0 / hv)};
+}
+// The update's factor HV dt_stage / (2 d).
+inline float f32_c(double d, double dt_full, double dt_stage) {
+  return (float)(f32_hv(d, dt_full) * (dt_stage / (2.0 * d)));
+}
+
+// One direction of one step of size dt; overlap as for the line kernels
+// (mw_fp64_line.cuh).
+int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double dt, const F32DirArgs& d, int direction,
+                   bool overlap, cudaStream_t stream);
+
+}  // namespace mw
