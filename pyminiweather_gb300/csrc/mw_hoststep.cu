@@ -34,6 +34,11 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
 namespace {
 
 constexpr int kMaxBands = 64;
+// Least cells of a band: launches over fewer do not fill the GPU, and the step
+// is a chain of three z launches per band (ms per step at 2048x1024 in at most
+// 32, 16, 8, 4, 2 bands: IEEE form 3.14, 2.24, 1.78, 1.75, 1.84, split 1.93,
+// 1.20, 0.93, 1.00, 1.06; 4096x2048 in 32, 16, 8: IEEE 6.02, 5.24, 5.25).
+constexpr long long kBandCells = 1 << 19;
 
 struct CopyRes {
   bool ready = false;
@@ -128,7 +133,7 @@ extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_
   // grids of the line kernels (a direction per launch) are stepped whole, as mw_step_f64 steps them
   const int nb = f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)
                      ? 1
-                     : std::max(1, std::min({nbands, kMaxBands, nz / 16}));
+                     : std::max(1, (int)std::min<long long>({nbands, kMaxBands, nz / 16, (long long)nx * nz / kBandCells}));
   if ((f64_mode != MW_F64_SPLIT && f64_mode != MW_F64_IEEE) || nb == 1) {  // no bands: copy in, step, copy out
     cudaError_t e = cudaMemcpyAsync(state, h_in, bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "copy in: %s", cudaGetErrorString(e));

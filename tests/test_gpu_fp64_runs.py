@@ -72,3 +72,22 @@ def test_rows_do_not_depend_on_the_cut(nx):
         part = f.state[:, r0:r0 + n + 4].contiguous()
         _, out = stage(q, g, part, 0, 0)
         assert torch.equal(out[:, 2:-2, 2:-2], whole[:, r0 + 2:r0 + n + 2, 2:-2]), (r0, n)
+
+
+@pytest.mark.parametrize("mode", ("fp64", "split"))
+@pytest.mark.parametrize("nx,nz,nbands", [(2050, 1031, 32), (4100, 1300, 3)])
+def test_host_step_bands_of_ragged_grids(nx, nz, nbands, mode):
+    """Grids large enough for several bands, whose rows do not divide by them: evolve_host gives the bits of
+    copy in, evolve, copy out, in both direction orders."""
+    import pyminiweather_gb300.solve.step as S
+    p = dict(make_params(nx, nz, "collision"), f64_mode=mode)
+    a, b = developed(p, 3), developed(p, 3)
+    h = b.state.cpu().pin_memory()
+    for step in range(2):
+        S.reverse_direction = bool(step)
+        S.evolve(p, a, None, dt=p["dt"])
+        S.reverse_direction = bool(step)
+        S.evolve_host(p, b, h, h, dt=p["dt"], nbands=nbands)
+        torch.cuda.synchronize()
+        assert torch.equal(h, a.state.cpu()) and torch.equal(a.state_tmp, b.state_tmp), step
+    S.reset_direction()
