@@ -143,6 +143,9 @@ int ens_step(void* plan, const mw_ens_plan_info* info, const double* hyc, const 
       es.items = dirs[d] == MW_DIR_X ? xi : zi;
       es.n_items = dirs[d] == MW_DIR_X ? info->n_x_items : info->n_z_items;
       const int grid = dirs[d] == MW_DIR_X ? grid_x : grid_z;
+      es.z_parts = dirs[d] == MW_DIR_X ? 1
+                                       : ens_z_parts(info->n_z_items, info->z_tile, grid,
+                                                     std::is_same<T, float>::value ? 1 : 4);
       if constexpr (std::is_same<T, float>::value) {  // one launch per direction, state -> scratch -> state
         const bool halo = flags & MW_FLAG_WRITE_HALO;
         es.init = d ? A : S;

@@ -42,6 +42,7 @@ struct EnsStageT {
   EnsCursor* cursor;             // device, in the plan
   int n_items;
   int z_tile;      // rows per z item
+  int z_parts;     // equal parts an item's rows are handed out in (list position it: part it % z_parts of item it / z_parts)
   int direction;   // MW_DIR_X / MW_DIR_Z
   int stage_div;   // the stage uses dt / stage_div (3, 2, 1)
   int fmt;         // split form: storage format of forcing / out (kF64, kToPair, kFromPair)
@@ -69,6 +70,17 @@ using EnsStage = EnsStageT<double>;
 template <typename T>
 __host__ __device__ inline int mconsts_index(const EnsStageT<T>& es, int e) {
   return (e * 2 + (es.direction == MW_DIR_X ? 0 : 1)) * 3 + (3 - es.stage_div);
+}
+
+// Parts per z item: a launch whose items do not fill `want` grids of CTAs ends
+// on a few CTAs still marching whole tiles (48 FP64 members of 64-512 columns:
+// 317 us a z stage, 1.9 times an x stage), so the tiles are halved until they
+// do, but not below 16 rows (each part evaluates one interface more than it has
+// rows; in the FP32 form it marches 12 rows more, and one grid's worth is enough).
+inline int ens_z_parts(int n_items, int z_tile, int grid, int want) {
+  int parts = 1;
+  while ((long long)n_items * parts < (long long)want * grid && z_tile >= 32 * parts) parts *= 2;
+  return parts;
 }
 
 // Launchers (defined next to the kernels they launch).
@@ -110,6 +122,14 @@ __device__ __forceinline__ unsigned ens_take_cta(EnsCursor* c, unsigned* slot, i
   const unsigned v = slot[parity];
   parity ^= 1;
   return v;
+}
+// Rows [z0, z1) of part `part` of tile `tile` of a member of nz rows (empty
+// where the tile is short).
+template <typename T>
+__device__ __forceinline__ void ens_part_rows(const EnsStageT<T>& es, int tile, int part, int nz, int& z0, int& z1) {
+  const int rows = (es.z_tile + es.z_parts - 1) / es.z_parts, end = min((tile + 1) * es.z_tile, nz);
+  z0 = tile * es.z_tile + part * rows;
+  z1 = min(z0 + rows, end);
 }
 // Every thread of the CTA, once it has stopped taking items.
 __device__ __forceinline__ void ens_finish(EnsCursor* c) {

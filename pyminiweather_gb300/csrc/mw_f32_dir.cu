@@ -610,13 +610,16 @@ __global__ void __launch_bounds__(kEnsZCols, 8) k_ens_z_f32(EnsStageT<float> es)
   SmemZ<kEnsZCols>& sm = *reinterpret_cast<SmemZ<kEnsZCols>*>(smem_f32);
   __shared__ unsigned slot[2];
   int parity = 0;
-  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)es.n_items;
+  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)(es.n_items * es.z_parts);
        it = ens_take_cta(es.cursor, slot, parity)) {
-    const int2 item = MW_AT(es.items, it, es.n_items);  // (member, column block + ncb * tile)
+    const int2 item = MW_AT(es.items, it / es.z_parts, es.n_items);  // (member, column block + ncb * tile)
     const Args a = member_args(es, item.x);
     const int ncb = (a.nx + kEnsZCols - 1) / kEnsZCols;
-    const int cb = item.y % ncb, z0 = item.y / ncb * es.z_tile;
-    z_march<kEnsZCols, false>(a, cb, z0, min(z0 + es.z_tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1), false);
+    const int cb = item.y % ncb;
+    int z0, z1;
+    ens_part_rows(es, item.y / ncb, it % es.z_parts, a.nz, z0, z1);
+    if (z0 >= z1) continue;
+    z_march<kEnsZCols, false>(a, cb, z0, z1, sm, reinterpret_cast<Row*>(&sm + 1), false);
   }
   ens_finish(es.cursor);
 }

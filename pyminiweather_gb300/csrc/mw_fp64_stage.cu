@@ -419,13 +419,15 @@ __global__ void __launch_bounds__(kEnsZCols) k_ens_z_ieee(EnsStage es) {
   __shared__ SmemZ sm;
   __shared__ unsigned slot[2];
   int parity = 0;
-  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)es.n_items;
+  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)(es.n_items * es.z_parts);
        it = ens_take_cta(es.cursor, slot, parity)) {
-    const int2 item = MW_AT(es.items, it, es.n_items);  // (member, column block + ncb * tile)
+    const int2 item = MW_AT(es.items, it / es.z_parts, es.n_items);  // (member, column block + ncb * tile)
     const Args a = member_args(es, item.x);
     const int ncb = (a.nx + kEnsZCols - 1) / kEnsZCols;
     const int cb = item.y % ncb, tile = item.y / ncb;
-    const int z0 = tile * es.z_tile, z1 = min(z0 + es.z_tile, a.nz);
+    int z0, z1;
+    ens_part_rows(es, tile, it % es.z_parts, a.nz, z0, z1);
+    if (z0 >= z1) continue;
     const bool halo = a.flags & MW_FLAG_WRITE_HALO;
     z_tile<kEnsZCols>(a, cb, z0, z1, halo && z0 == 0, halo && z1 == a.nz, sm);
   }

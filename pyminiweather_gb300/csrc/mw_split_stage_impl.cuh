@@ -438,13 +438,15 @@ __global__ void __launch_bounds__(kEnsZCols,
   __shared__ SmemZ sm;
   __shared__ unsigned slot[2];
   int parity = 0;
-  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)es.n_items;
+  for (unsigned it = ens_take_cta(es.cursor, slot, parity); it < (unsigned)(es.n_items * es.z_parts);
        it = ens_take_cta(es.cursor, slot, parity)) {
-    const int2 item = MW_AT(es.items, it, es.n_items);  // (member, column block + ncb * tile)
+    const int2 item = MW_AT(es.items, it / es.z_parts, es.n_items);  // (member, column block + ncb * tile)
     const SplitArgs a = member_args(es, item.x);
     const int ncb = (a.nx + kEnsZCols - 1) / kEnsZCols;
     const int cb = item.y % ncb, tile = item.y / ncb;
-    const int k0 = tile * es.z_tile, kend = min(k0 + es.z_tile, a.nz);
+    int k0, kend;
+    ens_part_rows(es, tile, it % es.z_parts, a.nz, k0, kend);
+    if (k0 >= kend) continue;
     const bool halo = a.flags & MW_FLAG_WRITE_HALO;
     z_march<FMT, kEnsZCols>(a, cb, k0, kend, halo && k0 == 0, halo && kend == a.nz, sm);
   }

@@ -236,3 +236,17 @@ def test_uneven_thermal_ensemble_256():
             assert max(normwise(ens.member_state(e).cpu().numpy(), ref)) <= MEMBER_TOL[torch.float64]
         # the two FP64 forms agree with each other to the benchmark's tolerance
         assert max(normwise(e64s.member_state(e).cpu().numpy(), e64.member_state(e).cpu().numpy())) <= TOL_STEP
+
+
+@pytest.mark.parametrize("dtype,mode", [(torch.float64, "fp64"), (torch.float64, "split"), (torch.float32, "fp64")])
+def test_z_items_in_parts_give_the_same_bits(dtype, mode):
+    """A launch with few z items for its grid hands each out in parts of at least 16 rows: the same bits as whole
+    items (a grid of one CTA takes them whole), with tiles that end mid-part."""
+    mem = [(member_params(nx, nz), None) for nx, nz in ((70, 35), (64, 64), (130, 81), (40, 17), (33, 5))]
+    runs = []
+    for grid_z in (1, 4000):
+        ens = Ensemble(mem, dtype=dtype, f64_mode=mode, z_tile=64)
+        ens.grid_x, ens.grid_z = 304, grid_z
+        ens.step(3)
+        runs.append((ens.state.clone(), ens.state_tmp.clone()))
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
