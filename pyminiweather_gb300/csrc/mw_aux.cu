@@ -10,7 +10,7 @@
 #include <cmath>
 
 #include "mw_common.cuh"
-#include "mw_fp64_math.cuh"
+#include "mw_fp64_flux.cuh"
 #include "mw_split.cuh"
 
 namespace mw {
@@ -195,51 +195,59 @@ __device__ __forceinline__ double load_state(const float* p) { return split::f2d
 // rho Cv t is Cv K (rho theta)^gamma with K = (C0 / p0)^(Rd/Cp), and with
 // rho theta = (rho theta)_bg (1 + d) it is Pr (1 + ((1 + d)^gamma - 1)),
 // Pr = Cv K (rho theta)_bg^gamma formed once per row (ck = Cv K from the
-// host), the bracket by the binomial series of the stage kernels (degree per
-// warp, expm1 / log1p for |d| >= 1/8).  ke = ((rho u)^2 + (rho w)^2) / rho
-// with one reciprocal.  The same quantities as the reference's up to a few
-// roundings per cell (the sums agree to ~1e-16 relative).
-__constant__ ieee::Series c_stats_pow_g = ieee::make_series(kGamma);
+// host), the bracket by the stage kernels' polynomial in (rho theta)' (its row
+// coefficients formed once per row, its sum accumulated by its last FMA).  A
+// row's background terms, nx rho_bg and nx Pr, are added once per row, and
+// ke = ((rho u)^2 + (rho w)^2) / rho takes one reciprocal: 7 + n FP64
+// operations per cell, n the series' degree, which bounds the kernel (FP64
+// pipe).  The same quantities as the reference's up to a few roundings per
+// cell (the sums agree to ~1e-16 relative).  At 4096x2048: 213 us; with a
+// power per warp and row, the background in every cell's sums and the series
+// in d, 357 us.
+constexpr int kStatRows = 16;  // rows whose constants a block holds at a time
 
 template <typename T>
 __global__ void __launch_bounds__(kStatThreads) k_stats_partial(int nx, int nz, int rpb, double ck, const double* hyc,
                                                                 const double* hytc, const T* state, double* part) {
   __shared__ double sm[kStatThreads / 32], se[kStatThreads / 32];
+  __shared__ ieee::RowP rows[kStatRows];
   const int NX = nx + 2 * kHs;
   const long long plane = (long long)NX * (nz + 2 * kHs);
-  const int lane = threadIdx.x & 31;
-  double m = 0.0, e = 0.0;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int chunks = (nx + 31) / 32;  // 32-cell pieces of a row, a warp's unit of work
+  double m = 0.0, ek = 0.0, ep = 0.0;
   const int k0 = blockIdx.x * rpb, k1 = min(k0 + rpb, nz);
-  for (int k = k0; k < k1; ++k) {
-    const int kk = k + kHs;
-    const double hr = MW_AT(hyc, kk, nz + 2 * kHs), hrt = MW_AT(hytc, kk, nz + 2 * kHs);
-    double pr = 0.0;
-    if (lane == 0) pr = ck * pow(hrt, kGamma);  // one power per warp and row
-    pr = __shfl_sync(0xffffffffu, pr, 0);
-    const double irt = 1.0 / hrt;
-    for (int base = 0; base < nx; base += kStatThreads) {
-      const int i = base + threadIdx.x;
+  for (int kb = k0; kb < k1; kb += kStatRows) {
+    const int nr = min(kStatRows, k1 - kb);
+    __syncthreads();
+    if (threadIdx.x < nr) {
+      const double hr = MW_AT(hyc, kb + threadIdx.x + kHs, nz + 2 * kHs);
+      const double hrt = MW_AT(hytc, kb + threadIdx.x + kHs, nz + 2 * kHs);
+      const double pr = ck * pow(hrt, kGamma);
+      ieee::RowP r = ieee::row_consts_p(hr, hrt, pr, 1.0, 1.0, 1.0);
+      rows[threadIdx.x] = r;
+      m = fma((double)nx, hr, m);
+      ep = fma((double)nx, pr, ep);
+    }
+    __syncthreads();
+    // piece u of the nr x chunks of these rows, in row-major order
+    for (long long u = w; u < (long long)nr * chunks; u += kStatThreads / 32) {
+      const int r = (int)(u / chunks), i = (int)(u - (long long)r * chunks) * 32 + lane;
       const bool act = i < nx;
-      const unsigned mask = __ballot_sync(0xffffffffu, act);  // the lanes of this row step
+      const unsigned mask = __ballot_sync(0xffffffffu, act);
       if (act) {
-        const long long o = (long long)kk * NX + i + kHs;
-        const double rho = load_state(&MW_AT(state, o, 4 * plane)) + hr;
-        const double ri = ieee::rcp(rho, mask);
+        const long long o = (long long)(kb + r + kHs) * NX + i + kHs;
+        const double d = load_state(&MW_AT(state, o, 4 * plane));
         const double ru = load_state(&MW_AT(state, plane + o, 4 * plane));
         const double rw = load_state(&MW_AT(state, 2 * plane + o, 4 * plane));
-        const double ke = fma(ru, ru, rw * rw) * ri;
-        const double d = load_state(&MW_AT(state, 3 * plane + o, 4 * plane)) * irt;
-        bool big;
-        const int n = ieee::series_degree(d, mask, c_stats_pow_g, big);
-        double f = d * ieee::series_g(d, n, c_stats_pow_g);  // (1 + d)^gamma - 1
-        if (__any_sync(mask, big)) {
-          if (big) f = expm1(kGamma * log1p(d));
-        }
-        m += rho;
-        e += ke + fma(pr, f, pr);
+        const double rt = load_state(&MW_AT(state, 3 * plane + o, 4 * plane));
+        m += d;
+        ek = fma(fma(ru, ru, rw * rw), ieee::rcp(d + rows[r].d.R, mask), ek);
+        ep = ieee::pressure(rt, rows[r], ep, mask);
       }
     }
   }
+  double e = ek + ep;
   block_sum2<kStatThreads>(m, e, sm, se);
   if (threadIdx.x == 0) {
     MW_AT(part, 2 * blockIdx.x, 2 * gridDim.x) = m;
@@ -288,22 +296,40 @@ int run_stats(int nx, int nz, double dx, double dz, const double* hyc, const dou
   return check_launch("stats final launch");
 }
 
-// compute_solution_variables, post/stats.py:38-69
-__global__ void k_solution_vars(int nx, int nz, const double* hyc, const double* hytc, const double* state,
-                                double* out) {
+// compute_solution_variables, post/stats.py:38-69.  Bound by the FP64 pipe: 12
+// operations per cell (ieee::divide) where the three divisions of a cell and one
+// of the row took ~60 (4096x2048: 511 us, now 257 us; HBM alone 79 us).  A
+// block takes up to kSvCells cells of a row.
+constexpr int kSvThreads = 256, kSvCells = 8 * kSvThreads;
+
+__global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, int per_row, long long nblk,
+                                                              const double* hyc, const double* hytc,
+                                                              const double* state, double* out) {
   const int NX = nx + 2 * kHs;
   const long long plane = (long long)NX * (nz + 2 * kHs);
   const long long n = (long long)nx * nz;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(idx / nx), i = (int)(idx % nx);
-    const long long o = (long long)(k + kHs) * NX + i + kHs;
-    const double hr = MW_AT(hyc, k + kHs, nz + 2 * kHs), hrt = MW_AT(hytc, k + kHs, nz + 2 * kHs);
-    const double d = MW_AT(state, o, 4 * plane);
-    MW_AT(out, idx, 4 * n) = d;
-    MW_AT(out, n + idx, 4 * n) = div_(MW_AT(state, plane + o, 4 * plane), add_(hr, d));
-    MW_AT(out, 2 * n + idx, 4 * n) = div_(MW_AT(state, 2 * plane + o, 4 * plane), add_(hr, d));
-    MW_AT(out, 3 * n + idx, 4 * n) = sub_(div_(add_(MW_AT(state, 3 * plane + o, 4 * plane), hrt), add_(hr, d)),
-                                          div_(hrt, hr));
+  for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+    const int k = (int)(blk / per_row), i0 = (int)(blk - (long long)k * per_row) * kSvCells;
+    const double hr = MW_AT(hyc, k + kHs, nz + 2 * kHs);
+    const double hrt[1] = {MW_AT(hytc, k + kHs, nz + 2 * kHs)};
+    double th[1];
+    ieee::divide(hrt, hr, 0xffffffffu, th);
+    for (int i = i0 + threadIdx.x; i - (int)(threadIdx.x & 31) < min(i0 + kSvCells, nx); i += kSvThreads) {
+      const bool act = i < nx;
+      const unsigned mask = __ballot_sync(0xffffffffu, act);
+      if (act) {
+        const long long o = (long long)(k + kHs) * NX + i + kHs, idx = (long long)k * nx + i;
+        const double d = MW_AT(state, o, 4 * plane);
+        const double a[3] = {MW_AT(state, plane + o, 4 * plane), MW_AT(state, 2 * plane + o, 4 * plane),
+                             MW_AT(state, 3 * plane + o, 4 * plane) + hrt[0]};
+        double q[3];
+        ieee::divide(a, hr + d, mask, q);
+        MW_AT(out, idx, 4 * n) = d;
+        MW_AT(out, n + idx, 4 * n) = q[0];
+        MW_AT(out, 2 * n + idx, 4 * n) = q[1];
+        MW_AT(out, 3 * n + idx, 4 * n) = q[2] - th[0];
+      }
+    }
   }
 }
 
@@ -571,7 +597,10 @@ extern "C" int mw_solution_variables_f64(int nx, int nz, const double* hyc, cons
   if (st) return st;
   MW_REQUIRE(hyc && hytc && state && out, MW_ERR_INVALID_ARG, "NULL pointer argument");
   MW_REQUIRE(aligned(hyc) && aligned(hytc) && aligned(state) && aligned(out), MW_ERR_ALIGN, "misaligned pointer");
-  k_solution_vars<<<grid_for((long long)nx * nz, 256), 256, 0, (cudaStream_t)stream>>>(nx, nz, hyc, hytc, state, out);
+  const int per_row = (nx + kSvCells - 1) / kSvCells;
+  const long long nblk = (long long)per_row * nz;
+  k_solution_vars<<<(unsigned)std::min(nblk, 1LL << 20), kSvThreads, 0, (cudaStream_t)stream>>>(nx, nz, per_row, nblk,
+                                                                                              hyc, hytc, state, out);
   return check_launch("solution variables launch");
 }
 

@@ -44,19 +44,13 @@ constexpr Series make_series(double e) {
   return t;
 }
 
-// 1/y for the lanes in `mask`, which call it together, in 2 FP64 operations.
-// With y = m 2^E, m in [1, 2), an estimate R of 1/m to about 2^-45 is formed
-// on the FP32 and integer pipes (which run beside the FP64 pipe): the hardware
-// estimate r0 of 1/mh, mh the leading 24 bits of m, corrected to first and
-// second order, r1 = r0 (e + e^2), e = 1 - m r0, and r0 + r1 put together as a
-// 53-bit integer significand.  One Newton step in FP64, r = R + R (1 - y R),
-// squares the error (2^-90), so r carries little more than its last rounding.
-// (A 24-bit estimate with a cubic step took 3 operations; the kernels are bound
-// by the FP64 pipe, which needs 16 SM clocks per warp operation.)  Zero,
-// subnormal, Inf, NaN and |y| >= 2^1022 take the FP64 division, behind a
-// warp-uniform branch so that it is never evaluated speculatively on the other
-// lanes.
-__device__ __forceinline__ double rcp(double y, unsigned mask) {
+// An estimate R of 1/y to about 2^-45 without FP64 operations.  With y = m 2^E,
+// m in [1, 2), it is formed on the FP32 and integer pipes (which run beside the
+// FP64 pipe): the hardware estimate r0 of 1/mh, mh the leading 24 bits of m,
+// corrected to first and second order, r1 = r0 (e + e^2), e = 1 - m r0, and
+// r0 + r1 put together as a 53-bit integer significand.  far: zero, subnormal,
+// Inf, NaN and |y| >= 2^1022, for which R is meaningless.
+__device__ __forceinline__ double rcp_estimate(double y, bool& far) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(y);
   const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
   const unsigned ex = (hi >> 20) & 0x7ffu;
@@ -71,14 +65,52 @@ __device__ __forceinline__ double rcp(double y, unsigned mask) {
   // to the accuracy of R)
   const unsigned rb = __float_as_uint(r0);
   const unsigned rhi = (rb >> 3) + ((1919u - ex) << 20);  // 1919 = 1023 + 896: exponent of r0 less that of y
-  const long long rbits = (long long)(((unsigned long long)(rhi | (hi & 0x80000000u)) << 32) | (rb << 29)) + i1;
-  const double r0d = __longlong_as_double(rbits);
-  double r = fma(r0d, fma(-y, r0d, 1.0), r0d);
-  const bool out = ex - 1u > 2043u;
-  if (__any_sync(mask, out)) {
-    if (out) r = 1.0 / y;
+  far = ex - 1u > 2043u;
+  return __longlong_as_double((long long)(((unsigned long long)(rhi | (hi & 0x80000000u)) << 32) | (rb << 29)) + i1);
+}
+
+// 1/y for the lanes in `mask`, which call it together, in 2 FP64 operations:
+// one Newton step from the estimate, r = R + R (1 - y R), squares its error
+// (2^-90), so r carries little more than its last rounding.  (A 24-bit
+// estimate with a cubic step took 3 operations; the kernels are bound by the
+// FP64 pipe, which needs 16 SM clocks per warp operation.)  Where R is
+// meaningless the FP64 division is taken, behind a warp-uniform branch so that
+// it is never evaluated speculatively on the other lanes.
+__device__ __forceinline__ double rcp(double y, unsigned mask) {
+  bool far;
+  const double R = rcp_estimate(y, far);
+  double r = fma(R, fma(-y, R, 1.0), R);
+  if (__any_sync(mask, far)) {
+    if (far) r = 1.0 / y;
   }
   return r;
+}
+
+// N quotients a[k] / y in 3 FP64 operations each, for the lanes in `mask`:
+// q = a R, then q + R (a - y q), whose error before the last rounding is 2^-90
+// (so it is the correctly rounded quotient but for a few in 2^37).  Quotients
+// that leave the normal range, and divisors with no estimate, take the FP64
+// division.
+template <int N>
+__device__ __forceinline__ void divide(const double (&a)[N], double y, unsigned mask, double (&q)[N]) {
+  bool far;
+  const double R = rcp_estimate(y, far);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double q0 = a[k] * R;
+    q[k] = fma(R, fma(-y, q0, a[k]), q0);
+    // exponents of q and of a within [2^-900, 2^900], or a = 0 and q = 0 (integer tests)
+    const unsigned eq = (unsigned)(__double_as_longlong(q[k]) >> 52) & 0x7ffu;
+    const unsigned ea = (unsigned)(__double_as_longlong(a[k]) >> 52) & 0x7ffu;
+    const bool zero = (__double_as_longlong(a[k]) << 1) == 0;
+    far = far || (!zero && (eq - 123u > 1800u || ea - 123u > 1800u));
+  }
+  if (__any_sync(mask, far)) {
+    if (far) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) q[k] = a[k] / y;
+    }
+  }
 }
 
 // The Horner degree of series S that the largest |d| among the lanes in
