@@ -1049,14 +1049,19 @@ static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, doubl
                      const double* hytc, const double* hyi, const double* hyti, const double* hypi,
                      const double* src_w, double* state, double* state_tmp, double* scratch, int nsteps, int* reverse,
                      int f64_mode, unsigned flags, cudaStream_t s) {
-  if (f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)) {
+  LinePlan plan;
+  if (f64_mode == MW_F64_IEEE)
+    if (const int st = line_ieee_plan(nx, nz, &plan)) return st;
+  if (plan.fits) {
     const bool halo = flags & MW_FLAG_WRITE_HALO;
     LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, state, state, nullptr, nullptr, halo ? state : nullptr,
                halo ? state_tmp : nullptr};
     for (int n = 0; n < nsteps; ++n) {
       for (int d = 0; d < 2; ++d) {
         a.s2 = n + 1 == nsteps && d == 1 ? state_tmp : nullptr;  // what the call leaves in state_tmp
-        const int st = launch_line_ieee(nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
+        a.in = plan.cut && d == 1 ? scratch : state;  // cut lines: state -> scratch -> state, else in place
+        a.out = plan.cut && d == 0 ? scratch : state;
+        const int st = launch_line_ieee(plan, nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
                                         n + d > 0, s);
         if (st) return st;
       }
@@ -1272,12 +1277,14 @@ extern "C" int mw_step_record_f64(int nx, int nz, double dx, double dz, double d
   cudaError_t e = cudaMemcpyAsync(stages, state_in, n * sizeof(double), cudaMemcpyDeviceToDevice, s);
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "stage copy: %s", cudaGetErrorString(e));
   const int dirs[2] = {reverse ? MW_DIR_X : MW_DIR_Z, reverse ? MW_DIR_Z : MW_DIR_X};
-  if (f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)) {
+  LinePlan plan;
+  if (f64_mode == MW_F64_IEEE && (st = line_ieee_plan(nx, nz, &plan))) return st;
+  if (plan.fits) {
     for (int d = 0; d < 2; ++d) {
       double* S = stages + 3 * d * n;
       const LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, S, d == 0 ? stages + 3 * n : state_out, S + n, S + 2 * n,
                        nullptr, nullptr};
-      if ((st = launch_line_ieee(nx, nz, dx, dz, dt_full, dt, a, dirs[d], d > 0, s))) return st;
+      if ((st = launch_line_ieee(plan, nx, nz, dx, dz, dt_full, dt, a, dirs[d], d > 0, s))) return st;
     }
     return MW_OK;
   }

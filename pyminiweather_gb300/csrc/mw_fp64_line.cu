@@ -8,7 +8,7 @@
 // evolve, pyminiweather/solve/step.py:85-143).
 //
 // What bounds it: a warp's FP64 instruction occupies its SM partition for 64
-// cycles, however many of its lanes are active, and a stage is a chain of ~42
+// cycles, however many of its lanes are active, and a stage is a chain of ~45
 // of them.  On a small grid the stage kernels (mw_fp64_stage.cu) therefore pay
 // for every row a thread marches and for the row tables a CTA forms: 30 us a z
 // stage and 18 us an x stage at 100 x 50.  Here a cell is one lane's work: the
@@ -16,12 +16,16 @@
 // as in the x pass of mw_fp64_stage.cu), spread so that the SM partitions get
 // equal numbers of warps, and the constants of an interface's row live in the
 // registers of the lane that needs them (z) or are formed once per line (x).
+// Lines may be cut into pieces, each CTA computing four cells more on either
+// side of its piece in the first stage and two in the second, where that evens
+// out the CTAs per SM; the direction's result then goes to another array.
 #include <algorithm>
 #include <atomic>
 
 #include "mw_common.cuh"
 #include "mw_fp64_flux.cuh"
 #include "mw_fp64_line.cuh"
+#include "mw_pow.cuh"
 
 namespace mw {
 namespace ieee {
@@ -36,6 +40,7 @@ struct LineParams {
   int n, nlines;         // cells per line, lines
   int log_lines, runs;   // lines per CTA (a power of two), runs per line
   int run;               // cells per run
+  int pieces, piece;     // pieces per line, cells per piece
   int lp;                // shared-memory pitch of a line
   int pitch;
   long long plane;
@@ -46,25 +51,27 @@ struct LineParams {
 
 #define MW_LG(p, off) MW_AT((p), (off), 4 * P.plane)
 
-// Line l of variable q in one of the two buffers, cell c at [c + 2].
+// Line l of variable q in one of the two buffers.
 __device__ __forceinline__ double* line_at(const LineParams& P, double* buf, int q, int l) {
   return buf + ((size_t)(q << P.log_lines) + l) * P.lp;
 }
 
-// Stores cell c of a line and, where it is a source of them, its halo images:
-// periodic in x (ics/bcs.py:35-39), walls in z (bcs.py:92-148; hr[h] is
-// hyc(halo row) / hyc(wall row) for rows -2, -1, nz, nz + 1).
+// Stores cell c of a line (line[c]) and, where it is a source of them, its halo
+// images: periodic in x where the CTA holds the whole line (ics/bcs.py:35-39;
+// the pieces of a cut row hold their neighbours' cells instead), walls in z
+// (bcs.py:92-148; hr[h] is hyc(halo row) / hyc(wall row) for rows -2, -1, nz,
+// nz + 1).
 template <int DIR>
-__device__ __forceinline__ void put(double* line, int q, int c, int n, double v, const double* hr) {
-  line[c + kHs] = v;
+__device__ __forceinline__ void put(double* line, int q, int c, int n, bool whole, double v, const double* hr) {
+  line[c] = v;
   if (DIR == MW_DIR_X) {
-    if (c < kHs) line[n + kHs + c] = v;
-    if (c >= n - kHs) line[c - n + kHs] = v;
+    if (whole && c < kHs) line[n + c] = v;
+    if (whole && c >= n - kHs) line[c - n] = v;
   } else {
     if (c == 0)
-      for (int h = 0; h < 2; ++h) line[h] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[h] : v);
+      for (int h = 0; h < 2; ++h) line[h - 2] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[h] : v);
     if (c == n - 1)
-      for (int h = 0; h < 2; ++h) line[n + kHs + h] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[2 + h] : v);
+      for (int h = 0; h < 2; ++h) line[n + h] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[2 + h] : v);
   }
 }
 
@@ -88,21 +95,22 @@ __device__ __forceinline__ void halo_out(const LineParams& P, double* g, int lin
   }
 }
 
-// The CTA's lines between a global array and shared memory.  x: a warp per
-// line and variable; z: consecutive threads take the CTA's columns of a row.
+// Cells [ca, cb) of the CTA's lines, between a global array and shared memory
+// (x: periodic).  x: a warp per line and variable; z: consecutive threads take
+// the CTA's columns of a row.
 template <int DIR, typename Fn>
-__device__ __forceinline__ void each_cell(const LineParams& P, int l0, int nl, Fn fn) {
+__device__ __forceinline__ void each_cell(const LineParams& P, int l0, int nl, int ca, int cb, Fn fn) {
   if (DIR == MW_DIR_X) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int ql = w; ql < 4 * nl; ql += nw) {
       const int q = ql / nl, l = ql - q * nl;
       const long long o = q * P.plane + (long long)(l0 + l + kHs) * P.pitch + kHs;
-      for (int c = lane; c < P.n; c += 32) fn(q, l, c, o + c);
+      for (int c = ca + lane; c < cb; c += 32) fn(q, l, c, o + (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c)));
     }
   } else {
     for (int q = 0; q < 4; ++q)
-      for (int i = threadIdx.x; i < (P.n << P.log_lines); i += blockDim.x) {
-        const int l = i & ((1 << P.log_lines) - 1), c = i >> P.log_lines;
+      for (int i = threadIdx.x; i < ((cb - ca) << P.log_lines); i += blockDim.x) {
+        const int l = i & ((1 << P.log_lines) - 1), c = ca + (i >> P.log_lines);
         if (l < nl) fn(q, l, c, q * P.plane + (long long)(c + kHs) * P.pitch + l0 + l + kHs);
       }
   }
@@ -114,23 +122,37 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
   extern __shared__ __align__(16) unsigned char smem_line[];
   __shared__ RowD rows[kLineMax];
   __shared__ double hr[4];
+  __shared__ PowTables pow_tables;  // x
   const LineArgs& a = P.a;
   const int n = P.n, nl_cta = 1 << P.log_lines;
-  double* buf[2] = {reinterpret_cast<double*>(smem_line),
-                    reinterpret_cast<double*>(smem_line) + (size_t)4 * nl_cta * P.lp};
-  const int l0 = blockIdx.x << P.log_lines, nl = min(nl_cta, P.nlines - l0);
+  const int group = blockIdx.x / P.pieces, pc = blockIdx.x - group * P.pieces;
+  const int l0 = group << P.log_lines, nl = min(nl_cta, P.nlines - l0);
+  const bool whole = P.pieces == 1;
+  const int p0 = pc * P.piece, p1 = min(p0 + P.piece, n);  // the CTA's cells
+  // first and last + 1 cell of a stage's result that the next stages need of this piece
+  auto first = [&](int s) { return whole ? 0 : (DIR == MW_DIR_X ? p0 - 4 + 2 * s : max(p0 - 4 + 2 * s, 0)); };
+  auto past = [&](int s) { return whole ? n : (DIR == MW_DIR_X ? p1 + 4 - 2 * s : min(p1 + 4 - 2 * s, n)); };
+  // the two buffers, so that cell c of a line is at [c] from line_at
+  double* buf[2] = {reinterpret_cast<double*>(smem_line) + (whole ? kHs : 6 - p0),
+                    reinterpret_cast<double*>(smem_line) + (size_t)4 * nl_cta * P.lp + (whole ? kHs : 6 - p0)};
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int l = w / P.runs, rn = w - l * P.runs;   // the warp's line and run
-  const bool live = l < nl;
-  const int c0 = rn * P.run, c1 = live ? min(c0 + P.run, n) : 0;
+  const int c0 = first(0) + rn * P.run, c1 = min(c0 + P.run, past(0));
+  const bool live = l < nl && c0 < c1;
 
   // row constants and wall ratios (backgrounds only: the kernel before it does not write them)
   RowD rz[SL];
   if (DIR == MW_DIR_X) {
+    load_pow_tables(pow_tables);
+    double r = 0.0, rt = 1.0;
     if (threadIdx.x < nl) {
-      const int k = l0 + threadIdx.x + kHs;
-      const double rt = MW_AT(a.hytc, k, P.nlines + 2 * kHs);
-      rows[threadIdx.x] = row_consts(MW_AT(a.hyc, k, P.nlines + 2 * kHs), rt, kC0 * pow(rt, kGamma), P.HV, P.IHV);
+      r = MW_AT(a.hyc, l0 + threadIdx.x + kHs, P.nlines + 2 * kHs);
+      rt = MW_AT(a.hytc, l0 + threadIdx.x + kHs, P.nlines + 2 * kHs);
+    }
+    __syncthreads();
+    if (w == 0) {
+      const double pr = kC0 * pow_gamma(rt, pow_tables), irt = rcp(12.0 * rt, kAll), p = 12.0 * pr * P.IHV;
+      if (lane < nl) rows[lane] = {12.0 * r * P.HV, 12.0 * rt, irt, p, p * c_pow_g.c[1] * irt};
     }
   } else {
     if (threadIdx.x < 4) {
@@ -149,31 +171,21 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     }
   }
   if (P.wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (DIR == MW_DIR_Z) __syncthreads();  // hr
-  each_cell<DIR>(P, l0, nl, [&](int q, int ll, int c, long long o) {
-    put<DIR>(line_at(P, buf[0], q, ll), q, c, n, MW_LG(a.in, o), hr);
-  });
-  // the four x-halo columns of the wall halo rows, from the halo columns' own first and last rows
-  if (DIR == MW_DIR_Z && blockIdx.x == 0 && threadIdx.x < 8) {
-    double* g = threadIdx.x < 4 ? a.halo_in : a.halo_tmp;
-    const int col = (threadIdx.x & 2) ? P.nlines + (threadIdx.x & 3) : (threadIdx.x & 1);
-    if (g)
-      for (int e = 0; e < 2; ++e) {
-        double v[4];
-        for (int q = 0; q < 4; ++q) v[q] = MW_LG(g, q * P.plane + (long long)(e ? n + kHs - 1 : kHs) * P.pitch + col);
-        for (int q = 0; q < 4; ++q)
-          for (int h = 2 * e; h < 2 * e + 2; ++h)
-            MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + col) =
-                q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
-      }
+  {
+    const int ca = whole ? 0 : (DIR == MW_DIR_X ? p0 - 6 : max(p0 - 6, 0));
+    const int cb = whole ? n : (DIR == MW_DIR_X ? p1 + 6 : min(p1 + 6, n));
+    each_cell<DIR>(P, l0, nl, ca, cb, [&](int q, int ll, int c, long long o) {
+      put<DIR>(line_at(P, buf[0], q, ll), q, c, n, whole, MW_LG(a.in, o), hr);
+    });
   }
   double sw[SL];
 #pragma unroll
   for (int j = 0; j < SL; ++j) {
-    const int c = c0 - 2 + 32 * j + lane;  // the cell this slot updates
+    int c = c0 - 2 + 32 * j + lane;  // the cell this slot updates
     sw[j] = 0.0;
-    if (a.srcw && c >= c0 && c < c1) {
+    if (a.srcw && live && c >= c0 && c < c1) {
+      if (DIR == MW_DIR_X) c = c < 0 ? c + n : (c >= n ? c - n : c);
       const long long o = DIR == MW_DIR_X ? (long long)(l0 + l) * n + c : (long long)c * P.nlines + l0 + l;
       sw[j] = MW_AT(a.srcw, o, (long long)n * P.nlines);
     }
@@ -190,11 +202,12 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       const int prev = (lane + 31) & 31;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const double* ln = line_at(P, src, q, l) + kHs;
+        const double* ln = line_at(P, src, q, l);
         double e[SL], qv[SL];
 #pragma unroll
         for (int j = 0; j < SL; ++j) {
-          const int i = min(c0 - 1 + 32 * j + lane, n);
+          // slots beyond the stage's cells repeat its last ones (not used)
+          const int i = min(max(c0 - 1 + 32 * j + lane, first(s) - 1), past(s));
           const double sm = ln[i - 1];
           cell_eq(sm, ln[i], ln[i + 1], e[j], qv[j]);
           if (s == 0) sv[j][q] = sm;
@@ -228,10 +241,10 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
         }
         if (DIR == MW_DIR_Z) v[WMOM] = fma(-P.dt[s] * kGrav, wgt[j], v[WMOM]);
         if (a.srcw) v[WMOM] = fma(P.dt[s], sw[j], v[WMOM]);
-        if (c >= c0 && c < c1) {
+        if (c >= max(c0, first(s)) && c < min(c1, past(s))) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) put<DIR>(line_at(P, dst, q, l), q, c, n, v[q], hr);
-          const bool edge = DIR == MW_DIR_X ? (c < kHs || c >= n - kHs) : (c == 0 || c == n - 1);
+          for (int q = 0; q < 4; ++q) put<DIR>(line_at(P, dst, q, l), q, c, n, whole, v[q], hr);
+          const bool edge = c < p0 || c >= p1 ? false : DIR == MW_DIR_X ? (c < kHs || c >= n - kHs) : (c == 0 || c == n - 1);
           if (edge) {
             const int line = DIR == MW_DIR_X ? l0 + l : l0 + l + kHs;
             if (s == 0 && a.halo_in) halo_out<DIR>(P, a.halo_in, line, c, sv[j], hr);
@@ -241,11 +254,29 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       }
     }
     __syncthreads();
+    // The next kernel may come in now: its CTAs take what is free beside this
+    // one's, and earlier that is unevenly much (256x128: 60 us a step with this at
+    // the head of the kernel, 41 here, 47 without overlap).
+    if (s == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     double* g = s == 0 ? a.s1 : (s == 1 ? a.s2 : a.out);
     if (g)
-      each_cell<DIR>(P, l0, nl, [&](int q, int ll, int c, long long o) {
-        MW_LG(g, o) = line_at(P, dst, q, ll)[c + kHs];
+      each_cell<DIR>(P, l0, nl, p0, p1, [&](int q, int ll, int c, long long o) {
+        MW_LG(g, o) = line_at(P, dst, q, ll)[c];
       });
+  }
+  // the four x-halo columns of the wall halo rows, from the halo columns' own first and last rows
+  if (DIR == MW_DIR_Z && blockIdx.x == 0 && threadIdx.x < 8) {
+    double* g = threadIdx.x < 4 ? a.halo_in : a.halo_tmp;
+    const int col = (threadIdx.x & 2) ? P.nlines + (threadIdx.x & 3) : (threadIdx.x & 1);
+    if (g)
+      for (int e = 0; e < 2; ++e) {
+        double v[4];
+        for (int q = 0; q < 4; ++q) v[q] = MW_LG(g, q * P.plane + (long long)(e ? n + kHs - 1 : kHs) * P.pitch + col);
+        for (int q = 0; q < 4; ++q)
+          for (int h = 2 * e; h < 2 * e + 2; ++h)
+            MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + col) =
+                q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
+      }
   }
 }
 
@@ -289,16 +320,69 @@ int line_sms(int* out) {
 
 constexpr int run_cells(int sl) { return 32 * sl - 2; }
 
-}  // namespace ieee
+constexpr int kMaxPieces = 16;
 
-bool line_ieee_fits(int nx, int nz) {
-  using namespace ieee;
-  const int most = line_warps(2) * run_cells(2);
-  return nx <= most && nz <= most && (long long)nx * nz <= kLineCellsMax;
+// The spread with the least time.  An SM that gets m CTAs of W warps with SL
+// slots per lane gives its four partitions m W SL / 4 slot groups each, every
+// one the same FP64 instructions, and that is what the time follows: measured
+// over every spread of thirteen grids from 100x50 to 900x300, both directions in
+// turn, 5.5 to 6.5 us a group (401x199, x: whole rows in 14 warps, two CTAs on
+// some SMs, 7 groups, 42 us; in three pieces of five warps, four CTAs, 5 groups,
+// 30 us).  Where all CTAs of an SM are resident at once its fullest partition
+// counts (nearly: m W / 4 rounded up); else m is rounded up to whole turns of
+// the resident CTAs, but for a last turn that fewer than half would fill.  Two
+// slots per lane with less than two warps per partition wait on their own
+// latency.  The factors near 1 break ties: more resident CTAs (their heads and
+// tails fill one another), fewer pieces, fewer CTAs, in z whole sectors.
+LineSpread spread_lines(int n, int nlines, bool isx, int sms) {
+  LineSpread best;
+  double least = 0.0;
+  for (int sl = 1; sl <= 2; ++sl)
+    for (int pieces = 1; pieces == 1 || (pieces <= kMaxPieces && (n + pieces - 1) / pieces >= 24); ++pieces) {
+      const int piece = (n + pieces - 1) / pieces;
+      if ((n + piece - 1) / piece != pieces) continue;  // an empty last piece
+      const int range = pieces == 1 ? n : piece + 8;
+      if (pieces > 1 && range >= n) break;
+      const int runs = (range + run_cells(sl) - 1) / run_cells(sl);
+      const int lp = (pieces == 1 ? n + 2 * kHs : piece + 12) | 1;
+      for (int lg = 0; (1 << lg) <= kLineMax; ++lg) {
+        const int warps = runs << lg;
+        const size_t smem = (size_t)lp * sizeof(double) * 8 << lg;
+        if (warps > line_warps(sl) || smem > kLineSmem) break;
+        const int resident = std::min((int)(65536 / ((sl == 1 ? 96 : 128) * 32 * warps)), (int)((220 << 10) / smem));
+        const double load = (double)((nlines + (1 << lg) - 1) >> lg) * pieces / sms;
+        const double turns = std::min(std::ceil(load / resident) * resident, load + 0.5 * resident) * warps / 4.0;
+        const double once = std::ceil(load) * warps / 4.0;
+        double cost = sl * (load <= resident ? 0.1 * once + 0.9 * std::ceil(once) : turns);
+        cost *= (1.0 + 0.1 / resident) * (1.0 + 0.001 * load) * (pieces > 1 ? 1.01 : 1.0) *
+                (!isx && lg == 0 ? 1.03 : 1.0) * (sl == 2 && once < 2.0 ? 1.3 : 1.0);
+        if (best.sl == 0 || cost < least) {
+          least = cost;
+          const int run = (range + runs - 1) / runs;
+          best = {sl, lg, pieces, piece, (range + run - 1) / run, run, lp};
+        }
+      }
+    }
+  return best;
 }
 
-int launch_line_ieee(int nx, int nz, double dx, double dz, double dt_full, double dt, const LineArgs& a, int direction,
-                     bool overlap, cudaStream_t stream) {
+}  // namespace ieee
+
+int line_ieee_plan(int nx, int nz, LinePlan* plan) {
+  using namespace ieee;
+  *plan = LinePlan();
+  if ((long long)nx * nz > kLineCellsMax) return MW_OK;
+  int sms = 0, st = line_sms(&sms);
+  if (st) return st;
+  plan->x = spread_lines(nx, nz, true, sms);
+  plan->z = spread_lines(nz, nx, false, sms);
+  plan->fits = plan->x.sl > 0 && plan->z.sl > 0;
+  plan->cut = plan->x.pieces > 1 || plan->z.pieces > 1;
+  return MW_OK;
+}
+
+int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz, double dt_full, double dt,
+                     const LineArgs& a, int direction, bool overlap, cudaStream_t stream) {
   using namespace ieee;
   LineParams P;
   P.a = a;
@@ -308,7 +392,6 @@ int launch_line_ieee(int nx, int nz, double dx, double dz, double dt_full, doubl
   P.nlines = isx ? nz : nx;
   P.pitch = g.pitch;
   P.plane = g.plane;
-  P.lp = (P.n + 2 * kHs) | 1;
   const double d = isx ? dx : dz;
   P.HV = ieee_hv(d, dt_full);
   P.IHV = 1.0 / P.HV;
@@ -317,39 +400,20 @@ int launch_line_ieee(int nx, int nz, double dx, double dz, double dt_full, doubl
     P.c[s] = P.dt[s] / (12.0 * d) * P.HV;
   }
   P.wait = overlap;
-  int sms = 0, st = line_sms(&sms);
-  if (st) return st;
-  // Slots per lane and lines per CTA: the SM partitions' share of warp slots
-  // decides the time (every slot group costs its partition the same FP64
-  // instructions); among equals, z takes more lines (whole sectors of a row).
-  int best_sl = 0, best_log = 0;
-  long long best = 0;
-  for (int sl = 1; sl <= 2; ++sl) {
-    const int runs = (P.n + run_cells(sl) - 1) / run_cells(sl);
-    for (int lg = 0; (1 << lg) <= kLineMax; ++lg) {
-      const int warps = runs << lg;
-      if (warps > line_warps(sl) || ((size_t)P.lp * sizeof(double) * 8 << lg) > kLineSmem) break;
-      const long long ctas = (P.nlines + (1 << lg) - 1) >> lg;
-      const long long per_sm = (ctas + sms - 1) / sms;
-      const long long cost = per_sm * ((warps + 3) / 4) * sl;
-      if (best_sl == 0 || cost < best || (cost == best && !isx && sl == best_sl)) {
-        best = cost;
-        best_sl = sl;
-        best_log = lg;
-      }
-    }
-  }
-  MW_REQUIRE(best_sl, MW_ERR_SHAPE, "lines of %d cells do not fit a CTA", P.n);
-  P.log_lines = best_log;
-  const int min_runs = (P.n + run_cells(best_sl) - 1) / run_cells(best_sl);
-  P.run = (P.n + min_runs - 1) / min_runs;
-  P.runs = (P.n + P.run - 1) / P.run;
-  const int threads = 32 * (P.runs << best_log);
-  const int ctas = (P.nlines + (1 << best_log) - 1) >> best_log;
-  const size_t smem = (size_t)P.lp * sizeof(double) * 8 << best_log;
-  if (isx) return best_sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, stream)
+  const LineSpread& sp = isx ? plan.x : plan.z;
+  MW_REQUIRE(sp.pieces == 1 || a.in != a.out, MW_ERR_ALIAS, "a direction of cut lines needs another array for its result");
+  P.log_lines = sp.log_lines;
+  P.pieces = sp.pieces;
+  P.piece = sp.piece;
+  P.run = sp.run;
+  P.runs = sp.runs;
+  P.lp = sp.lp;
+  const int threads = 32 * (P.runs << P.log_lines);
+  const int ctas = ((P.nlines + (1 << P.log_lines) - 1) >> P.log_lines) * P.pieces;
+  const size_t smem = (size_t)P.lp * sizeof(double) * 8 << P.log_lines;
+  if (isx) return sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, stream)
                                : launch_line_t<MW_DIR_X, 2>(P, ctas, threads, smem, stream);
-  return best_sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, stream)
+  return sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, stream)
                       : launch_line_t<MW_DIR_Z, 2>(P, ctas, threads, smem, stream);
 }
 

@@ -21,21 +21,34 @@ struct LineArgs {
   const double* hypi;
   const double* srcw;  // optional forcing of w
   const double* in;    // the direction's initial state
-  double* out;         // its result (may be `in`: every CTA reads its lines before it writes them)
+  double* out;         // its result; may be `in` where the lines are not cut (a CTA reads its lines before it writes them)
   double* s1;          // first and second stage, each optional
   double* s2;
   double* halo_in;     // optional: arrays that get the direction's halo of the initial state
   double* halo_tmp;    // and of the second stage
 };
 
-// Whether grids of nx x nz cells take the line kernels.
-bool line_ieee_fits(int nx, int nz);
+// How a direction's lines are spread over CTAs: slots per lane, lines per CTA
+// (log2), pieces per line and cells per piece, runs (warps) per line and cells
+// per run, and a line's pitch in shared memory.
+struct LineSpread {
+  int sl = 0, log_lines = 0, pieces = 1, piece = 0, runs = 0, run = 0, lp = 0;
+};
+
+// Whether a grid takes the line kernels, and how.  cut: the lines of either
+// direction are cut into pieces, so a direction's result must go to another
+// array than its input.
+struct LinePlan {
+  LineSpread x, z;
+  bool fits = false, cut = false;
+};
+int line_ieee_plan(int nx, int nz, LinePlan* plan);
 
 // One direction of one step of size dt.  overlap: the kernel may start while
 // the one before it on the stream is finishing, and waits for it before it
 // touches the state; only for a launch behind another line kernel of the same
 // call (what it reads before the wait, the backgrounds, is then complete).
-int launch_line_ieee(int nx, int nz, double dx, double dz, double dt_full, double dt, const LineArgs& a, int direction,
-                     bool overlap, cudaStream_t stream);
+int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz, double dt_full, double dt,
+                     const LineArgs& a, int direction, bool overlap, cudaStream_t stream);
 
 }  // namespace mw

@@ -131,9 +131,11 @@ extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_
   const size_t bytes = sizeof(double) * 4 * (size_t)g.plane;
   cudaStream_t s = (cudaStream_t)stream;
   // grids of the line kernels (a direction per launch) are stepped whole, as mw_step_f64 steps them
-  const int nb = f64_mode == MW_F64_IEEE && line_ieee_fits(nx, nz)
-                     ? 1
-                     : std::max(1, (int)std::min<long long>({nbands, kMaxBands, nz / 16, (long long)nx * nz / kBandCells}));
+  LinePlan plan;
+  if (f64_mode == MW_F64_IEEE && (st = line_ieee_plan(nx, nz, &plan))) return st;
+  const int nb = plan.fits ? 1
+                           : std::max(1, (int)std::min<long long>({nbands, kMaxBands, nz / 16,
+                                                                    (long long)nx * nz / kBandCells}));
   if ((f64_mode != MW_F64_SPLIT && f64_mode != MW_F64_IEEE) || nb == 1) {  // no bands: copy in, step, copy out
     cudaError_t e = cudaMemcpyAsync(state, h_in, bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "copy in: %s", cudaGetErrorString(e));

@@ -20,7 +20,8 @@ pytestmark = pytest.mark.gpu
 # 3 steps are 18 stages of at most 3e-14 of max|s| each (test_gpu_fp64_runs.py): 6e-13.
 TOL = 1e-12
 GRIDS = [(2, 1), (3, 2), (4, 3), (30, 29), (31, 30), (29, 31), (60, 61), (62, 60), (63, 62), (64, 64), (100, 50),
-         (124, 31), (125, 63), (481, 37), (37, 481), (480, 240), (511, 257), (991, 20), (20, 992), (992, 5), (993, 4)]
+         (124, 31), (125, 63), (481, 37), (37, 481), (480, 240), (511, 257), (991, 20), (20, 992), (992, 5), (993, 4),
+         (200, 100), (256, 128), (401, 199), (512, 256), (24, 2000), (2000, 24), (3001, 40), (5, 9000), (640, 600)]
 
 
 def developed(p, seed):
