@@ -217,7 +217,11 @@ struct SmemZ {
 // Rows [z0, z1) of the columns [cb NC, cb NC + NC); every thread of the CTA
 // calls it (one barrier after the row table is formed).  tab: z1 - z0 + 17 rows
 // of shared memory.
-template <int NC, bool SRC>
+// TMP: the second stage is stored too.  Without it the march is unrolled by four
+// (8192x2048: 145 against 169 us, the streams' rows keep their registers); with
+// it the extra stores bound the pass and the compact loop does better (190
+// against 198 us).
+template <int NC, bool SRC, bool TMP>
 __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, SmemZ<NC>& sm, Row* tab, bool wait) {
   const int a0 = max(z0 - 6, 0), last = z1 - 1 + kLag;  // first row in; last iteration
   const int t = threadIdx.x, nz = a.nz;
@@ -315,7 +319,7 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
     const Vars v2 = stage(1, v1, r - 2, ring(r - 4));
     const Vars o = stage(2, v2, r - 4, ring(r - 6));
     const unsigned off = off_in - 16u * pitch4;  // row r - 6 (off_in is at row r + 10)
-    if (act && a.s2 && r - 4 >= z0 && r - 4 < z1) store(a.s2, off + 2u * pitch4, v2);
+    if (TMP && act && r - 4 >= z0 && r - 4 < z1) store(a.s2, off + 2u * pitch4, v2);
     if (W && act && a.halo_tmp) {
       if (r - 4 == 0 && z0 == 0) put_halo(a.halo_tmp, c + kHs, false, v2);
       if (r - 4 == nz - 1 && z1 == nz) put_halo(a.halo_tmp, c + kHs, true, v2);
@@ -326,18 +330,23 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
   const int fast0 = min(6, last + 1);
   for (; r < fast0; ++r) iterate(r, std::true_type{});
   const int fast1 = min(nz, last + 1);
+  if (TMP) {
 #pragma unroll 1
-  for (; r < fast1; ++r) iterate(r, std::false_type{});
+    for (; r < fast1; ++r) iterate(r, std::false_type{});
+  } else {
+#pragma unroll 4
+    for (; r < fast1; ++r) iterate(r, std::false_type{});
+  }
   for (; r <= last; ++r) iterate(r, std::true_type{});
   copies_wait<0>();
 }
 
-template <bool SRC>
+template <bool SRC, bool TMP>
 __global__ void __launch_bounds__(kZCols, 4) k_dir_z_f32(const __grid_constant__ Args a, int tile, int tile0, bool wait) {
   extern __shared__ __align__(16) unsigned char smem_f32[];
   SmemZ<kZCols>& sm = *reinterpret_cast<SmemZ<kZCols>*>(smem_f32);
   const int z0 = (tile0 + blockIdx.y) * tile;
-  z_march<kZCols, SRC>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1), wait);
+  z_march<kZCols, SRC, TMP>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1), wait);
 }
 
 // ---- x ---------------------------------------------------------------------
@@ -605,6 +614,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_ens_x_f32(EnsStageT<float> 
   ens_finish(es.cursor);
 }
 
+template <bool TMP>
 __global__ void __launch_bounds__(kEnsZCols, 8) k_ens_z_f32(EnsStageT<float> es) {
   extern __shared__ __align__(16) unsigned char smem_f32[];
   SmemZ<kEnsZCols>& sm = *reinterpret_cast<SmemZ<kEnsZCols>*>(smem_f32);
@@ -619,7 +629,7 @@ __global__ void __launch_bounds__(kEnsZCols, 8) k_ens_z_f32(EnsStageT<float> es)
     int z0, z1;
     ens_part_rows(es, item.y / ncb, it % es.z_parts, a.nz, z0, z1);
     if (z0 >= z1) continue;
-    z_march<kEnsZCols, false>(a, cb, z0, z1, sm, reinterpret_cast<Row*>(&sm + 1), false);
+    z_march<kEnsZCols, false, TMP>(a, cb, z0, z1, sm, reinterpret_cast<Row*>(&sm + 1), false);
   }
   ens_finish(es.cursor);
 }
@@ -648,19 +658,22 @@ int device(Device** out) {
   const size_t zs = z_smem(kZCols, kZTileMax), xs8 = sizeof(XBuf<8>) * 2 * kXWarps, xs4 = sizeof(XBuf<4>) * 2 * kXWarps;
   int sms = 0, x4 = 0, x8 = 0, z = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<false>, zs);
-  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true>, zs);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<false, false>, zs);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<false, true>, zs);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, false>, zs);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, true>, zs);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<4, false>, xs4);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<4, true>, xs4);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<8, false>, xs8);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<8, true>, xs8);
   if (e == cudaSuccess) e = raise_smem(k_ens_x_f32, xs8);
-  if (e == cudaSuccess) e = raise_smem(k_ens_z_f32, z_smem(kEnsZCols, kEnsZTileMax));
+  if (e == cudaSuccess) e = raise_smem(k_ens_z_f32<false>, z_smem(kEnsZCols, kEnsZTileMax));
+  if (e == cudaSuccess) e = raise_smem(k_ens_z_f32<true>, z_smem(kEnsZCols, kEnsZTileMax));
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x4, k_dir_x_f32<4, false>, 32 * kXWarps, xs4);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x8, k_dir_x_f32<8, false>, 32 * kXWarps, xs8);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&z, k_dir_z_f32<false>, kZCols, zs);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&z, k_dir_z_f32<false, false>, kZCols, zs);
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "FP32 kernel setup: %s", cudaGetErrorString(e));
   d.x_ctas[0] = std::max(1, x4);
   d.x_ctas[1] = std::max(1, x8);
@@ -744,7 +757,9 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
   const int ntiles = (nz + tile - 1) / tile;
   for (int t0 = 0; t0 < ntiles; t0 += 65535) {
     const dim3 grid((unsigned)ncb, (unsigned)std::min(ntiles - t0, 65535));
-    st = launch(a.srcw ? k_dir_z_f32<true> : k_dir_z_f32<false>, grid, kZCols, z_smem(kZCols, tile), stream,
+    auto kern = a.srcw ? (a.s2 ? k_dir_z_f32<true, true> : k_dir_z_f32<true, false>)
+                       : (a.s2 ? k_dir_z_f32<false, true> : k_dir_z_f32<false, false>);
+    st = launch(kern, grid, kZCols, z_smem(kZCols, tile), stream,
                 overlap && t0 == 0, "FP32 z direction", a, tile, t0, overlap && t0 == 0);
     if (st) return st;
   }
@@ -760,7 +775,7 @@ int launch_ens_f32(const EnsStageT<float>& es, int grid) {
   if (es.direction == MW_DIR_X)
     k_ens_x_f32<<<grid, 32 * kXWarps, sizeof(XBuf<kEnsV>) * 2 * kXWarps, es.stream>>>(es);
   else
-    k_ens_z_f32<<<grid, kEnsZCols, z_smem(kEnsZCols, es.z_tile), es.stream>>>(es);
+    (es.s2 ? k_ens_z_f32<true> : k_ens_z_f32<false>)<<<grid, kEnsZCols, z_smem(kEnsZCols, es.z_tile), es.stream>>>(es);
   return check_launch("ensemble FP32 direction launch");
 }
 
@@ -773,7 +788,7 @@ int ens_f32_occupancy(int direction, int* blocks_per_sm) {
       direction == MW_DIR_X
           ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_ens_x_f32, 32 * kXWarps,
                                                           sizeof(XBuf<kEnsV>) * 2 * kXWarps)
-          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_ens_z_f32, kEnsZCols,
+          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_ens_z_f32<false>, kEnsZCols,
                                                           z_smem(kEnsZCols, kEnsZTileMax));
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
   return MW_OK;
