@@ -9,9 +9,9 @@ namespace mw {
 // Most cells of a grid that takes the line kernels: above this the CTAs of a
 // launch come in several waves and the stage kernels, which need no whole lines
 // in a CTA, do as well (us per step, line kernels / six stage launches replayed
-// from a graph: 100x50 22 / 121, 300x150 38 / 122, 512x256 120 / 145, 512x512
-// 237 / 240, 700x700 382 / 380, 992x992 671 / 663).
-constexpr long long kLineCellsMax = 400000;
+// from a graph: 100x50 24 / 121, 300x150 41 / 122, 512x256 113 / 145, 800x400
+// 237 / 279, 990x495 354 / 387, 992x992 659 / 661, 1200x600 482 / 469).
+constexpr long long kLineCellsMax = 600000;
 
 struct LineArgs {
   const double* hyc;
