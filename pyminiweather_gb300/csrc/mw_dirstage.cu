@@ -1164,7 +1164,14 @@ extern "C" int mw_step_f32(int nx, int nz, double dx, double dz, double dt_full,
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
   const bool halo = flags & MW_FLAG_WRITE_HALO;
-  for (int n = 0; n < nsteps; ++n) {
+  const bool fits = f32_dir_fits(nx);
+  if (!fits)
+    st = run_steps<float>(dt, state, state_tmp, scratch, nsteps, reverse,
+                          [&](const float* init, float* forcing, float* out, double dts, int dir, int) {
+                            return launch_stage<float, MODE_F32>(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi,
+                                                                 src_w, init, forcing, out, dts, dir, flags, s);
+                          });
+  for (int n = 0; fits && n < nsteps; ++n) {
     for (int d = 0; d < 2; ++d) {  // state -> scratch -> state
       const F32DirArgs a{hyc, hytc, hyi, hyti, hypi, src_w, d ? scratch : state, d ? state : scratch,
                          n + 1 == nsteps && d == 1 ? state_tmp : nullptr, halo ? state : nullptr,

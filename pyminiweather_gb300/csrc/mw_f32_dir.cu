@@ -27,6 +27,7 @@
 // (WMOM, RHOT) through packed FP32 instructions.
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 
 #include "mw_common.cuh"
 #include "mw_ensemble.cuh"
@@ -639,6 +640,7 @@ size_t z_smem(int nc, int tile) { return (nc == kZCols ? sizeof(SmemZ<kZCols>) :
 // The kernels' shared-memory limits, raised once per device; the device's SMs
 // and resident CTAs per SM of the two passes.
 struct Device {
+  std::mutex mu;
   std::atomic<int> sms{0};
   int x_ctas[2] = {0, 0}, z_ctas = 0;  // x: V = 4, 8
 };
@@ -655,6 +657,8 @@ int device(Device** out) {
   Device& d = g_dev[dev];
   *out = &d;
   if (d.sms.load(std::memory_order_acquire) > 0) return MW_OK;
+  std::lock_guard<std::mutex> lock(d.mu);
+  if (d.sms.load(std::memory_order_relaxed) > 0) return MW_OK;
   const size_t zs = z_smem(kZCols, kZTileMax), xs8 = sizeof(XBuf<8>) * 2 * kXWarps, xs4 = sizeof(XBuf<4>) * 2 * kXWarps;
   int sms = 0, x4 = 0, x8 = 0, z = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -742,7 +746,7 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
   const long long ncb = (nx + kZCols - 1) / kZCols;
   int tile = 1;
   double best = 0.0;
-  for (int n = (nz + kZTileMax - 1) / kZTileMax; n <= std::max(1, nz / 8); ++n) {
+  for (int n = (nz + kZTileMax - 1) / kZTileMax; n <= std::max(1, nz / 8); n += std::max(1, n / 32)) {
     const int t = (nz + n - 1) / n;
     const long long ctas = ncb * ((nz + t - 1) / t);
     const long long per_sm = (ctas + sms - 1) / sms, waves = (per_sm + dev->z_ctas - 1) / dev->z_ctas;
@@ -753,7 +757,7 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
     }
     if (t <= 8) break;
   }
-  tile = (int)std::max<long long>(1, std::min<long long>(tile, (1LL << 32) / (4LL * g.pitch) - 24));
+  tile = (int)std::max<long long>(1, std::min<long long>(tile, (1LL << 32) / (4LL * g.pitch) - 24));  // >= 1: f32_dir_fits
   const int ntiles = (nz + tile - 1) / tile;
   for (int t0 = 0; t0 < ntiles; t0 += 65535) {
     const dim3 grid((unsigned)ncb, (unsigned)std::min(ntiles - t0, 65535));

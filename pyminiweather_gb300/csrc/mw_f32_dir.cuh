@@ -36,6 +36,10 @@ inline float f32_c(double d, double dt_full, double dt_stage) {
   return (float)(f32_hv(d, dt_full) * (dt_stage / (2.0 * d)));
 }
 
+// Whether a row is short enough for the z pass's 32-bit offsets within a tile
+// (25 rows below 2^32 bytes); longer ones are stepped stage by stage.
+inline bool f32_dir_fits(int nx) { return 25LL * 4 * (nx + 4LL) < (1LL << 32); }
+
 // One direction of one step of size dt; overlap as for the line kernels
 // (mw_fp64_line.cuh).
 int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double dt, const F32DirArgs& d, int direction,

@@ -540,8 +540,9 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     const long long sms = std::max(1, resident / MW_IEEE_X_MIN_BLOCKS);
     int nrun = 1;
     double best = 0.0;
-    for (int n = (nx + kXRunBlocksMax * kWSlots - 1) / (kXRunBlocksMax * kWSlots);
-         n <= (nx + kWSlots - 3) / (kWSlots - 2); ++n) {
+    const int least = (int)(((long long)nx + kXRunBlocksMax * kWSlots - 1) / (kXRunBlocksMax * kWSlots));
+    const int most = (int)(((long long)nx + kWSlots - 3) / (kWSlots - 2));
+    for (int n = least; n <= most; n += std::max(1, n / 32)) {
       const int blocks = run_blocks((nx + n - 1) / n);
       const long long ctas = ((long long)n * rows + kXWarps - 1) / kXWarps;
       const double cost = (double)((ctas + sms - 1) / sms) * (blocks + 1.0 / 3);

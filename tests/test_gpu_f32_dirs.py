@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
+from pyminiweather_gb300 import _native
 from pyminiweather_gb300.data import initialize_fields
 from pyminiweather_gb300.ensemble import Ensemble, member_params
 from pyminiweather_gb300.ics import init
@@ -93,3 +94,39 @@ def test_ensemble_members_vs_oracle(z_tile):
         o.evolve(3)
         assert max(normwise(ens.member_state(e).double().cpu().numpy(), o.state, interior=False)) <= TOL, e
         assert max(normwise(ens.member_state_tmp(e).double().cpu().numpy(), o.state_tmp, interior=False)) <= TOL, e
+
+
+def by_stages(p, f, nsteps):
+    """Time steps issued stage by stage (mw_dirstage_f32), z then x first; returns state and state_tmp."""
+    s, t, a = f.state.clone(), f.state_tmp.clone(), torch.zeros_like(f.state)
+    bg = [_native.ptr(b) for b in f.backgrounds()]
+    for n in range(nsteps):
+        for d in (1, 0) if n % 2 == 0 else (0, 1):
+            for frc, out, div in ((s, a, 3), (a, t, 2), (t, s, 1)):
+                _native.call("mw_dirstage_f32", f.nx, f.nz, p["dx"], p["dz"], p["dt"], *bg, _native.ptr(f.src_w),
+                             _native.ptr(s), _native.ptr(frc), _native.ptr(out), p["dt"] / div, d, 1,
+                             _native.stream_handle())
+    return s, t
+
+
+@pytest.mark.parametrize("nx,nz,same", [(66, 600000, False), (43_000_001, 1, True)])
+def test_long_columns_and_rows_vs_stages(nx, nz, same):
+    """A column of many tiles; a row too long for the direction kernels, which is stepped stage by stage."""
+    if torch.cuda.mem_get_info()[0] < 12 * 4 * (nx + 4) * (nz + 4) * 4:
+        pytest.skip("not enough device memory")
+    p = dict(make_params(nx, nz, "thermal", xlen=20.0 * nx, zlen=1e4 if nz > 1 else 20.0))
+    f = initialize_fields(p, dtype=torch.float32)
+    init(f, p)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for q, amp in enumerate((1e-3, 5.0, 2.0, 0.5)):
+        f.state[q] += amp * torch.randn(f.shape[1:], device="cuda", generator=g)
+    ref, ref_tmp = by_stages(p, f, 2)
+    reset_direction()
+    evolve(p, f, None, dt=p["dt"], nsteps=2)
+    for got, want in ((f.state, ref), (f.state_tmp, ref_tmp)):
+        got, want = got[:, 2:-2, 2:-2], want[:, 2:-2, 2:-2]
+        if same:
+            assert torch.equal(got, want)
+        else:
+            for q in range(4):
+                assert (got[q] - want[q]).abs().max() <= TOL * want[q].abs().max(), q
