@@ -111,6 +111,41 @@ inline double ieee_hv(double d, double dt_full) { return std::fmax(12.0 * kHvBet
 
 inline bool valid_f64_mode(int m) { return m == MW_F64_NATIVE || m == MW_F64_SPLIT || m == MW_F64_IEEE; }
 
+// Internal launch flag: the launch may start while the one before it on the
+// stream is finishing (programmatic dependence).  Only behind another launch of
+// the same call: what a kernel reads before overlap_wait(), the backgrounds, is
+// then complete.  Never taken from a caller's flags (user_flags).
+constexpr unsigned kFlagOverlap = 1u << 31;
+inline unsigned user_flags(unsigned flags) { return flags & ~kFlagOverlap; }
+
+#ifdef __CUDACC__
+// Before anything the launch before may have written is touched (no effect in a plain launch).
+__device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next launch may come in, once every CTA of this one has got here or ended.
+// Not called early in a kernel whose CTAs do not fill the SMs evenly: the next
+// one's CTAs take what is free beside them, and stay where that was (FP64 stage
+// launches at 992x992, called at the head: 911 us a step, not at all: 643, plain
+// launches 657).
+__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+int launch_overlapping(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlap,
+                       const char* what, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return e == cudaSuccess ? MW_OK : fail(MW_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
+}
+#endif
+
 // Rows per z CTA for a single-grid launch: the largest tile up to max_rows
 // that still gives about two CTAs per SM (152 SMs), at least 8 rows.
 inline int z_tile_rows(int nx, int nz, int cols_per_cta, int max_rows) {

@@ -1049,6 +1049,7 @@ static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, doubl
                      const double* hytc, const double* hyi, const double* hyti, const double* hypi,
                      const double* src_w, double* state, double* state_tmp, double* scratch, int nsteps, int* reverse,
                      int f64_mode, unsigned flags, cudaStream_t s) {
+  flags = user_flags(flags);
   LinePlan plan;
   if (f64_mode == MW_F64_IEEE)
     if (const int st = line_ieee_plan(nx, nz, &plan)) return st;
@@ -1069,10 +1070,14 @@ static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, doubl
     }
     return MW_OK;
   }
+  unsigned overlap = 0;
   return run_steps<double>(dt, state, state_tmp, scratch, nsteps, reverse,
                            [&](const double* init, double* forcing, double* out, double dts, int dir, int k) {
-                             return stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init,
-                                              forcing, out, dts, dir, f64_mode, flags, s, split_step_fmt(k));
+                             const int st = stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init,
+                                                      forcing, out, dts, dir, f64_mode, flags | overlap, s,
+                                                      split_step_fmt(k));
+                             overlap = kFlagOverlap;  // the call's first launch waits for what came before the call
+                             return st;
                            });
 }
 
@@ -1120,7 +1125,7 @@ extern "C" int mw_dirstage_f64(int nx, int nz, double dx, double dz, double dt_f
              "MW_FLAG_PAIRS_OUT needs init == forcing (the first RK stage)");
   const int fmt = (flags & MW_FLAG_PAIRS_OUT) ? 1 : ((flags & MW_FLAG_PAIRS_IN) ? 2 : 0);
   return stage_f64(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, src_w, init, forcing, out, dt_stage,
-                   direction, f64_mode, flags & ~pairs, (cudaStream_t)stream, fmt);
+                   direction, f64_mode, user_flags(flags & ~pairs), (cudaStream_t)stream, fmt);
 }
 
 extern "C" int mw_dirstage_f32(int nx, int nz, double dx, double dz, double dt_full, const double* hyc,

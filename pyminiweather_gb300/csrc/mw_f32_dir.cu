@@ -49,6 +49,11 @@ constexpr int kAhead = 9;      // rows loaded ahead
 constexpr int kLag = 6;        // row r of the state comes in when row r - 6 of the result goes out
 constexpr int kZTileMax = 512; // rows per z CTA
 constexpr int kXWarps = 4;     // warps per x CTA
+// Launches of at most this many CTAs let the next one in at their head: both
+// then find an SM per CTA (100x50: 15.9 against 16.9 us a step).  A larger one's
+// CTAs would share SMs with the next one's, which stay there (2501x1251: 98 us a
+// step with every launch doing so, 79 with none).
+constexpr unsigned kFewCtas = 76;
 
 // Constants of one direction of one grid.
 struct Consts {
@@ -223,7 +228,7 @@ struct SmemZ {
 // it the extra stores bound the pass and the compact loop does better (190
 // against 198 us).
 template <int NC, bool SRC, bool TMP>
-__device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, SmemZ<NC>& sm, Row* tab, bool wait) {
+__device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, SmemZ<NC>& sm, Row* tab) {
   const int a0 = max(z0 - 6, 0), last = z1 - 1 + kLag;  // first row in; last iteration
   const int t = threadIdx.x, nz = a.nz;
   for (int i = t; i <= last - a0 + 5; i += NC) {  // interface a0 - 6 + i, clamped where nothing uses it
@@ -235,8 +240,8 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
     sm.hr[t] = MW_AT(a.hyc, h, nz + 2 * kHs) / MW_AT(a.hyc, src, nz + 2 * kHs);
   }
   __syncthreads();
-  if (wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  overlap_wait();
+  if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   const int c = cb * NC + t;
   // the wall halo rows (arrays that ask for them): of the initial state here, and of the x-halo columns of
   // both arrays from the halo columns' own first and last rows
@@ -343,11 +348,11 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
 }
 
 template <bool SRC, bool TMP>
-__global__ void __launch_bounds__(kZCols, 4) k_dir_z_f32(const __grid_constant__ Args a, int tile, int tile0, bool wait) {
+__global__ void __launch_bounds__(kZCols, 4) k_dir_z_f32(const __grid_constant__ Args a, int tile, int tile0) {
   extern __shared__ __align__(16) unsigned char smem_f32[];
   SmemZ<kZCols>& sm = *reinterpret_cast<SmemZ<kZCols>*>(smem_f32);
   const int z0 = (tile0 + blockIdx.y) * tile;
-  z_march<kZCols, SRC, TMP>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1), wait);
+  z_march<kZCols, SRC, TMP>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1));
 }
 
 // ---- x ---------------------------------------------------------------------
@@ -517,7 +522,7 @@ __device__ __forceinline__ void x_halo_in(const Args& a, int k) {
 // works on one.
 template <int V, bool SRC>
 __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_constant__ Args a, int nrun, int len,
-                                                              long long total, bool wait) {
+                                                              long long total) {
   extern __shared__ __align__(16) unsigned char smem_f32[];
   XBuf<V>* buf = reinterpret_cast<XBuf<V>*>(smem_f32) + 2 * (threadIdx.x >> 5);
   const long long w = (long long)blockIdx.x * kXWarps + (threadIdx.x >> 5), nw = (long long)gridDim.x * kXWarps;
@@ -525,8 +530,8 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
   int k = (int)(g0 / nrun), rn = (int)(g0 - (long long)k * nrun);
   Row row = {0.f, 0.f, 0.f, 0.f};
   if (g0 < g1) row = row_x(a.k, MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
-  if (wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  overlap_wait();
+  if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   if (g0 >= g1) return;
   x_load<V>(a, k, rn * len, min(len, a.nx - rn * len), buf[0]);
   int cur = 0;
@@ -630,7 +635,7 @@ __global__ void __launch_bounds__(kEnsZCols, 8) k_ens_z_f32(EnsStageT<float> es)
     int z0, z1;
     ens_part_rows(es, item.y / ncb, it % es.z_parts, a.nz, z0, z1);
     if (z0 >= z1) continue;
-    z_march<kEnsZCols, false, TMP>(a, cb, z0, z1, sm, reinterpret_cast<Row*>(&sm + 1), false);
+    z_march<kEnsZCols, false, TMP>(a, cb, z0, z1, sm, reinterpret_cast<Row*>(&sm + 1));
   }
   ens_finish(es.cursor);
 }
@@ -686,23 +691,6 @@ int device(Device** out) {
   return MW_OK;
 }
 
-template <typename K, typename... A>
-int launch(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlap, const char* what,
-           const A&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = overlap ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  return e == cudaSuccess ? MW_OK : fail(MW_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
-}
-
 }  // namespace f32
 
 int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double dt, const F32DirArgs& d, int direction,
@@ -738,8 +726,7 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
     const size_t smem = (v == 8 ? sizeof(XBuf<8>) : sizeof(XBuf<4>)) * 2 * kXWarps;
     auto kern = v == 8 ? (a.srcw ? k_dir_x_f32<8, true> : k_dir_x_f32<8, false>)
                        : (a.srcw ? k_dir_x_f32<4, true> : k_dir_x_f32<4, false>);
-    return launch(kern, dim3(grid), 32 * kXWarps, smem, stream, overlap, "FP32 x direction", a, nrun, lenc, total,
-                  overlap);
+    return launch_overlapping(kern, dim3(grid), 32 * kXWarps, smem, stream, overlap, "FP32 x direction", a, nrun, lenc, total);
   }
   // Rows per z CTA: a CTA marches its tile and 12 rows more; an iteration takes
   // ~300 cycles alone on its SM and ~150 more for every CTA beyond two.
@@ -763,8 +750,8 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
     const dim3 grid((unsigned)ncb, (unsigned)std::min(ntiles - t0, 65535));
     auto kern = a.srcw ? (a.s2 ? k_dir_z_f32<true, true> : k_dir_z_f32<true, false>)
                        : (a.s2 ? k_dir_z_f32<false, true> : k_dir_z_f32<false, false>);
-    st = launch(kern, grid, kZCols, z_smem(kZCols, tile), stream,
-                overlap && t0 == 0, "FP32 z direction", a, tile, t0, overlap && t0 == 0);
+    st = launch_overlapping(kern, grid, kZCols, z_smem(kZCols, tile), stream,
+                overlap && t0 == 0, "FP32 z direction", a, tile, t0);
     if (st) return st;
   }
   return MW_OK;

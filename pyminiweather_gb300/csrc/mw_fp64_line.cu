@@ -46,7 +46,6 @@ struct LineParams {
   long long plane;
   double HV, IHV;        // HV = -12 hv of the direction and 1 / HV
   double c[3], dt[3];    // per stage HV dt_stage / (12 d) and dt_stage
-  bool wait;             // launched while the kernel before it may still run
 };
 
 #define MW_LG(p, off) MW_AT((p), (off), 4 * P.plane)
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       rz[j].PC1 = rz[j].P * c_pow_g.c[1] * rz[j].IRT12;
     }
   }
-  if (P.wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+  overlap_wait();
   if (DIR == MW_DIR_Z) __syncthreads();  // hr
   {
     const int ca = whole ? 0 : (DIR == MW_DIR_X ? p0 - 6 : max(p0 - 6, 0));
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     // The next kernel may come in now: its CTAs take what is free beside this
     // one's, and earlier that is unevenly much (256x128: 60 us a step with this at
     // the head of the kernel, 41 here, 47 without overlap).
-    if (s == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (s == 2) overlap_next();
     double* g = s == 0 ? a.s1 : (s == 1 ? a.s2 : a.out);
     if (g)
       each_cell<DIR>(P, l0, nl, p0, p1, [&](int q, int ll, int c, long long o) {
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
 }
 
 template <int DIR, int SL>
-int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, cudaStream_t stream) {
+int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, bool overlap, cudaStream_t stream) {
   static std::atomic<int> done[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(MW_ERR_CUDA, "cudaGetDevice failed");
@@ -291,19 +290,7 @@ int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, cudaS
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "line kernel shared memory: %s", cudaGetErrorString(e));
     if (dev >= 0 && dev < 64) done[dev].store(1, std::memory_order_relaxed);
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = P.wait ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_line_ieee<DIR, SL>, P);
-  if (e != cudaSuccess) return fail(MW_ERR_CUDA, "line kernel launch: %s", cudaGetErrorString(e));
-  return MW_OK;
+  return launch_overlapping(k_line_ieee<DIR, SL>, dim3((unsigned)ctas), threads, smem, stream, overlap, "line kernel", P);
 }
 
 int line_sms(int* out) {
@@ -399,7 +386,6 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
     P.dt[s] = dt / (3 - s);
     P.c[s] = P.dt[s] / (12.0 * d) * P.HV;
   }
-  P.wait = overlap;
   const LineSpread& sp = isx ? plan.x : plan.z;
   MW_REQUIRE(sp.pieces == 1 || a.in != a.out, MW_ERR_ALIAS, "a direction of cut lines needs another array for its result");
   P.log_lines = sp.log_lines;
@@ -411,10 +397,10 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
   const int threads = 32 * (P.runs << P.log_lines);
   const int ctas = ((P.nlines + (1 << P.log_lines) - 1) >> P.log_lines) * P.pieces;
   const size_t smem = (size_t)P.lp * sizeof(double) * 8 << P.log_lines;
-  if (isx) return sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, stream)
-                               : launch_line_t<MW_DIR_X, 2>(P, ctas, threads, smem, stream);
-  return sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, stream)
-                      : launch_line_t<MW_DIR_Z, 2>(P, ctas, threads, smem, stream);
+  if (isx) return sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, overlap, stream)
+                               : launch_line_t<MW_DIR_X, 2>(P, ctas, threads, smem, overlap, stream);
+  return sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, overlap, stream)
+                      : launch_line_t<MW_DIR_Z, 2>(P, ctas, threads, smem, overlap, stream);
 }
 
 #if MW_CHECK

@@ -49,6 +49,7 @@
 #include "mw_ensemble.cuh"
 #include "mw_fp64_flux.cuh"
 #include "mw_fp64_math.cuh"
+#include "mw_pow.cuh"
 
 namespace mw {
 namespace ieee {
@@ -140,7 +141,8 @@ __device__ __forceinline__ void x_warp_walk(const Args& a, int nrun, int len, lo
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   // values of the block of row k whose slot 0 is cell i0: cells i0-1+lane, i0+31+lane and (lanes 0, 1)
-  // i0+63+lane; slots beyond the run hold valid values that nothing uses
+  // i0+63+lane; slots beyond the run hold valid values that nothing uses.  Plain loads: with launches that
+  // overlap, the launch before may write the forcing while this kernel is already resident (no ld.global.nc).
   auto load = [&](int k, int i0, double v[3][4]) {
     const long long row = (long long)(k + kHs) * a.pitch;
 #pragma unroll
@@ -148,7 +150,7 @@ __device__ __forceinline__ void x_warp_walk(const Args& a, int nrun, int len, lo
       if (j < 2 || lane < 2) {
         const long long col = wrap_x(min(i0 - 1 + 32 * j + lane, a.nx + 1), a.nx) + kHs;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[j][q] = __ldg(&MW_F(a, q * a.plane + row + col));
+        for (int q = 0; q < 4; ++q) v[j][q] = MW_F(a, q * a.plane + row + col);
       }
     }
   };
@@ -253,17 +255,27 @@ __global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Ar
                                                                                long long g1) {
   __shared__ SmemXW sm;
   __shared__ RowP rows[kXRowsMax];
+  __shared__ PowTables pow_tables;
   const long long b0 = g0 + (long long)blockIdx.x * kXWarps, b1 = min(b0 + kXWarps, g1);
   const int row0 = (int)(b0 / nrun), nrows = (int)((b1 - 1) / nrun) - row0 + 1;  // nrows <= kXRowsMax
   const int w = threadIdx.x >> 5;
+  auto table = [&]() {
+    load_pow_tables(pow_tables);
+    __syncthreads();
+    for (int r = threadIdx.x; r < nrows; r += kXT) {
+      const double rt = MW_AT(a.hytc, row0 + r + kHs, a.nz + 2 * kHs);
+      rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow_gamma(rt, pow_tables), a.HV,
+                             a.IHV);
+    }
+    __syncthreads();
+  };
+  // overlapped with the launch before, the table comes before the wait; else it is formed under the first loads
+  const bool early = a.flags & kFlagOverlap;
+  if (early) table();
+  overlap_wait();
   x_warp_walk(a, nrun, len, min(b0 + w, b1), min(b0 + w + 1, b1), [&](int k) -> const RowP& { return rows[k - row0]; },
               a.flags & MW_FLAG_WRITE_HALO, sm.sS[w], [&]() {
-                for (int r = threadIdx.x; r < nrows; r += kXT) {
-                  const double rt = MW_AT(a.hytc, row0 + r + kHs, a.nz + 2 * kHs);
-                  rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow(rt, kGamma),
-                                         a.HV, a.IHV);
-                }
-                __syncthreads();
+                if (!early) table();
               });
 }
 
@@ -283,6 +295,7 @@ __device__ __forceinline__ void z_tile(const Args& a, int cb, int z0, int z1, bo
                               a.IHV);
   }
   __syncthreads();
+  overlap_wait();
   const int c = cb * NC + threadIdx.x;  // interior column
   if ((hbot || htop) && cb == 0 && threadIdx.x < 4)
     write_z_halo_column(a, threadIdx.x < 2 ? threadIdx.x : a.nx + threadIdx.x, hbot, htop);
@@ -556,20 +569,18 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     const long long g0 = (long long)r0 * nrun, g1 = (long long)r1 * nrun;
     const long long grid = (g1 - g0 + kXWarps - 1) / kXWarps;
     MW_REQUIRE(grid <= 0x7fffffffLL, MW_ERR_SHAPE, "grid too large for the x direction-stage launch");
-    k_stage_x_ieee_w<<<(unsigned)grid, kXT, 0, stream>>>(a, nrun, len, g0, g1);
+    return launch_overlapping(k_stage_x_ieee_w, dim3((unsigned)grid), kXT, 0, stream, flags & kFlagOverlap,
+                              "x IEEE-FP64 direction-stage", a, nrun, len, g0, g1);
   } else {
     const int ntiles = (rows + a.z_tile - 1) / a.z_tile;
     for (int t0 = 0; t0 < ntiles; t0 += 65535) {
       dim3 grid((nx + kZT - 1) / kZT, (unsigned)std::min(ntiles - t0, 65535));
-      k_stage_z_ieee<<<grid, kZT, 0, stream>>>(a, t0);
-      if (t0 + 65535 < ntiles) {
-        const int st = check_launch("z IEEE-FP64 direction-stage launch");
-        if (st) return st;
-      }
+      const int st = launch_overlapping(k_stage_z_ieee, grid, kZT, 0, stream, (flags & kFlagOverlap) && t0 == 0,
+                                        "z IEEE-FP64 direction-stage", a, t0);
+      if (st) return st;
     }
   }
-  return check_launch(direction == MW_DIR_X ? "x IEEE-FP64 direction-stage launch"
-                                            : "z IEEE-FP64 direction-stage launch");
+  return MW_OK;
 }
 
 #if MW_CHECK

@@ -126,6 +126,7 @@ extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_
   int st = mw_step_f64(nx, nz, dx, dz, dt_full, dt, hyc, hytc, hyi, hyti, hypi, src_w, state, state_tmp, scratch, 0,
                        reverse, f64_mode, flags, stream);
   if (st) return st;
+  flags = user_flags(flags);
   MW_REQUIRE(h_in && h_out, MW_ERR_INVALID_ARG, "host state arrays must not be NULL");
   const Geom g = make_geom(nx, nz);
   const size_t bytes = sizeof(double) * 4 * (size_t)g.plane;

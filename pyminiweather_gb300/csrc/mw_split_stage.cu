@@ -17,6 +17,7 @@
 
 #include "mw_common.cuh"
 #include "mw_ensemble.cuh"
+#include "mw_pow.cuh"
 #include "mw_split.cuh"
 #include "mw_split2.cuh"
 #include "mw_split_flux.cuh"

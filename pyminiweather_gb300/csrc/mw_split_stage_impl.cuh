@@ -150,11 +150,12 @@ struct SmemXW {
   dw2 sS[kXWarps][2][kWVals + 1];  // [warp][pair][staged cell]
   dw2 sF[kXWarps][2][32];          // [warp][pair][interface]
   RowS row[kXRowsMax];
+  PowTables pow_tables;
 };
 
-__device__ __forceinline__ RowS x_row_consts(const SplitArgs& a, int k) {
+__device__ __forceinline__ RowS x_row_consts(const SplitArgs& a, int k, const PowTables& pow_tables) {
   const double hrt = MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs);
-  return row_consts(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), hrt, kC0 * pow(hrt, kGamma));
+  return row_consts(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), hrt, kC0 * pow_gamma(hrt, pow_tables));
 }
 
 // row_at(k): the row constants of row k.  prologue() runs once, after the
@@ -175,15 +176,16 @@ __device__ __forceinline__ void x_warp_segments(const SplitArgs& a, int nseg, lo
   // lanes 0..11, one value each (variable lane & 3 of cell x0+30+(lane>>2)),
   // so their conversion costs the warp one value's instructions, not four.
   const int xq = lane & 3, xj = lane >> 2;
+  // plain loads: with launches that overlap, the launch before may write the forcing while this one is resident
   auto load = [&](int kk, int x0, double v0[4], double& v1) {
     const sidx row = (sidx)(kk + kHs) * a.pitch;
     const int c0 = x0 - 2 + lane, c1 = x0 + 30 + xj;
     if (c0 <= a.nx + 1) {
       const sidx col = wrap_x(c0, a.nx) + kHs;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v0[q] = __ldg(&MW_AT(a.forcing, q * a.plane + row + col, 4 * (long long)a.plane));
+      for (int q = 0; q < 4; ++q) v0[q] = MW_AT(a.forcing, q * a.plane + row + col, 4 * (long long)a.plane);
     }
-    if (lane < 12 && c1 <= a.nx + 1) v1 = __ldg(&MW_AT(a.forcing, xq * a.plane + row + wrap_x(c1, a.nx) + kHs, 4 * (long long)a.plane));
+    if (lane < 12 && c1 <= a.nx + 1) v1 = MW_AT(a.forcing, xq * a.plane + row + wrap_x(c1, a.nx) + kHs, 4 * (long long)a.plane);
   };
   double v0[4] = {0, 0, 0, 0}, v1 = 0.0;
   load(k, sg * kWCells, v0, v1);
@@ -271,6 +273,7 @@ __device__ __forceinline__ void z_march(const SplitArgs& a, int cb, int kbeg, in
     sm.row[r] = row_consts(MW_AT(a.hyi, k, a.nz + 1), MW_AT(a.hyti, k, a.nz + 1), MW_AT(a.hypi, k, a.nz + 1));
   }
   __syncthreads();
+  overlap_wait();
   const int c = cb * NT + threadIdx.x;
   if ((hbot || htop) && cb == 0 && threadIdx.x < 4)
     write_z_halo_column(a, threadIdx.x < 2 ? threadIdx.x : a.nx + threadIdx.x, hbot, htop);
@@ -351,12 +354,20 @@ __global__ void __launch_bounds__(kXThreads, MW_XSPLIT_MIN_BLOCKS) k_stage_x_spl
   const int row0 = (int)(g0 / nseg), nrows = (int)((g1 - 1) / nseg) - row0 + 1;  // nrows <= kXRowsMax (host)
   const int w = threadIdx.x >> 5;
   const long long n = g1 - g0;
-  // the row-constant table (an FP64 pow per row) is formed while the warps'
-  // first loads are in flight
+  // the row-constant table (an FP64 power per row): before the wait where the
+  // launch overlaps the one before, else while the warps' first loads are in flight
+  auto table = [&]() {
+    load_pow_tables(sm.pow_tables);
+    __syncthreads();
+    for (int r = threadIdx.x; r < nrows; r += kXThreads) sm.row[r] = x_row_consts(a, row0 + r, sm.pow_tables);
+    __syncthreads();
+  };
+  const bool early = a.flags & kFlagOverlap;
+  if (early) table();
+  overlap_wait();
   x_warp_segments<FMT>(a, nseg, g0 + n * w / kXWarps, g0 + n * (w + 1) / kXWarps,
                        [&](int k) { return sm.row[k - row0]; }, a.flags & MW_FLAG_WRITE_HALO, sm, [&]() {
-                         for (int r = threadIdx.x; r < nrows; r += kXThreads) sm.row[r] = x_row_consts(a, row0 + r);
-                         __syncthreads();
+                         if (!early) table();
                        });
 }
 
@@ -572,7 +583,8 @@ int launch_stage_split_fmt(int nx, int nz, double dx, double dz, double dt_full,
 #endif
     grid = std::max<long long>(grid, (rows + kXRowsMax - 3) / (kXRowsMax - 2));
     MW_REQUIRE(grid <= 0x7fffffffLL, MW_ERR_SHAPE, "grid too large for the x direction-stage launch");
-    k_stage_x_split<FMT><<<(unsigned)grid, kXThreads, 0, stream>>>(a, nseg, total, (long long)r0 * nseg);
+    return launch_overlapping(k_stage_x_split<FMT>, dim3((unsigned)grid), kXThreads, 0, stream, flags & kFlagOverlap,
+                              "x split direction-stage", a, nseg, total, (long long)r0 * nseg);
   } else {
     const int ncb = (nx + kZThreads - 1) / kZThreads;
     const long long units = (long long)ncb * rows;
@@ -581,9 +593,9 @@ int launch_stage_split_fmt(int nx, int nz, double dx, double dz, double dt_full,
     long long grid = resident * ((units + (long long)kZTileMax * resident - 1) / ((long long)kZTileMax * resident));
     grid = std::max<long long>(1, std::min<long long>(grid, units / kZMinRows));
     MW_REQUIRE(grid <= 0x7fffffffLL, MW_ERR_SHAPE, "grid too large for the z direction-stage launch");
-    k_stage_z_split<FMT><<<(unsigned)grid, kZThreads, 0, stream>>>(a, ncb, r0, r1);
+    return launch_overlapping(k_stage_z_split<FMT>, dim3((unsigned)grid), kZThreads, 0, stream, flags & kFlagOverlap,
+                              "z split direction-stage", a, ncb, r0, r1);
   }
-  return check_launch(direction == MW_DIR_X ? "x split direction-stage launch" : "z split direction-stage launch");
 }
 
 // fmt: kF64, kToPair (forcing == init, out as pairs) or kFromPair (forcing as pairs).
