@@ -30,6 +30,7 @@
 
 #include "mw_common.cuh"
 #include "mw_fp64_math.cuh"
+#include "mw_pow.cuh"
 
 namespace mw {
 namespace {
@@ -49,6 +50,7 @@ struct VjpArgs {
   double* gdst;
   double* ws;       // 8 x n_interfaces: Abar[4], Dbar[4]
   long long nif;    // interfaces per variable plane of ws
+  double kc, ke;    // the gather's factors of the transposed interpolation (of 12 x it, over 12) and third difference
 };
 
 __device__ __forceinline__ int wrap_x(int j, int nx) { return j < 0 ? j + nx : (j >= nx ? j - nx : j); }
@@ -80,6 +82,7 @@ __constant__ double kE[4] = {-1.0, 3.0, -3.0, 1.0};
 // Interface adjoints.  x: interface (k, i), i in [0, nx]; z: (k, c), k in [0, nz].
 template <int DIR>
 __global__ void k_vjp_iface(VjpArgs a) {
+  overlap_wait();
   const long long n = a.nif;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -153,13 +156,16 @@ __global__ void k_vjp_iface(VjpArgs a) {
 template <int DIR>
 __device__ __forceinline__ void gather_general(const VjpArgs& a, int k, int i, double acc[4]) {
   const long long n = a.nif;
+  auto tap = [&](int q, int j, long long o) {
+    return a.kc * (kC[j] * MW_WS(a, q * n + o)) + a.ke * (kE[j] * MW_WS(a, (4 + q) * n + o));
+  };
   if (DIR == MW_DIR_X) {
     for (int j = 0; j < 4; ++j)
       for (int m = -1; m <= 1; ++m) {
         const int f = i + 2 - j + m * a.nx;  // interface whose tap j is cell i
         if (f < 0 || f > a.nx) continue;
         const long long o = (long long)k * (a.nx + 1) + f;
-        for (int q = 0; q < 4; ++q) acc[q] += kC[j] * MW_WS(a, q * n + o) + kE[j] * MW_WS(a, (4 + q) * n + o);
+        for (int q = 0; q < 4; ++q) acc[q] += tap(q, j, o);
       }
   } else {
     // taps t = f - 2 + j of interface f in [0, nz]; t maps to row k directly,
@@ -168,7 +174,7 @@ __device__ __forceinline__ void gather_general(const VjpArgs& a, int k, int i, d
       if (f < 0 || f > a.nz) continue;
       const int j = k - f + 2;
       const long long o = (long long)f * a.nx + i;
-      for (int q = 0; q < 4; ++q) acc[q] += kC[j] * MW_WS(a, q * n + o) + kE[j] * MW_WS(a, (4 + q) * n + o);
+      for (int q = 0; q < 4; ++q) acc[q] += tap(q, j, o);
     }
     auto halo_taps = [&](int t, double wq[4]) {  // weight of halo row t on row k
       const int src = t < 0 ? 0 : a.nz - 1;
@@ -187,7 +193,7 @@ __device__ __forceinline__ void gather_general(const VjpArgs& a, int k, int i, d
         if (f < 0 || f > a.nz) continue;
         const long long o = (long long)f * a.nx + i;
         for (int q = 0; q < 4; ++q)
-          acc[q] += wq[q] * (kC[j] * MW_WS(a, q * n + o) + kE[j] * MW_WS(a, (4 + q) * n + o));
+          acc[q] += wq[q] * tap(q, j, o);
       }
     }
   }
@@ -202,6 +208,7 @@ __device__ __forceinline__ void gather_general(const VjpArgs& a, int k, int i, d
 // the others take the general rule.  In z the gravity term follows.
 template <int DIR>
 __global__ void __launch_bounds__(128) k_vjp_gather(VjpArgs a) {
+  overlap_wait();
   const long long n = a.nif;
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   if (ii >= a.pitch) return;
@@ -227,9 +234,9 @@ __global__ void __launch_bounds__(128) k_vjp_gather(VjpArgs a) {
         const double D2 = MW_WS(a, (4 + q) * n + o0 + 2 * st), D3 = MW_WS(a, (4 + q) * n + o0 + 3 * st);
         // cell i is tap j of interface f = i + 2 - j, so kC = (-1, 7, 7, -1) / 12 and
         // kE = (-1, 3, -3, 1) act on the interfaces i + 2, i + 1, i, i - 1 = (A3, A2, A1, A0)
-        const double ca = fma(7.0, A1 + A2, -(A0 + A3)) * (1.0 / 12.0);
+        const double ca = fma(7.0, A1 + A2, -(A0 + A3));
         const double ce = fma(3.0, D2 - D1, D0 - D3);
-        acc[q] = ca + ce;
+        acc[q] = fma(a.kc * (1.0 / 12.0), ca, a.ke * ce);
       }
     } else {
       gather_general<DIR>(a, k, i, acc);
@@ -262,13 +269,16 @@ struct RowV {
 
 __global__ void k_vjp_rows_ieee(int nz, const double* hyc, const double* hytc, const double* hyi, const double* hyti,
                                 const double* hypi, RowV* t) {
+  __shared__ PowTables pow_tables;
+  load_pow_tables(pow_tables);
+  __syncthreads();
   const int n = 2 * nz + 5;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     double r, rt, Q;
     if (j < nz + 2 * kHs) {
       r = MW_AT(hyc, j, nz + 2 * kHs);
       rt = MW_AT(hytc, j, nz + 2 * kHs);
-      Q = kGamma * kC0 * pow(rt, kGamma - 1.0);
+      Q = kGamma * (kC0 * pow_gamma(rt, pow_tables)) / rt;  // gamma C0 (rho theta)^(gamma - 1)
     } else {  // hy_pressure_int = C0 hy_dens_theta_int^gamma (ics/initial.py:105)
       const int k = j - (nz + 2 * kHs);
       r = MW_AT(hyi, k, nz + 1);
@@ -280,13 +290,14 @@ __global__ void k_vjp_rows_ieee(int nz, const double* hyc, const double* hytc, c
   }
 }
 
-// J(f)^T of one interface in the fewest FP64 operations (~43 against ~300
+// J(f)^T of one interface in the fewest FP64 operations (~35 against ~300
 // for k_vjp_iface, the same Jacobian): taps s, G = g(f) - g(f-1), the row
-// constants rv; Ab = J^T (cd G) and Db = hvcd G, with (rho w)' and d3[DENS]
-// held at zero at the z walls.  The lanes in `mask` call it together.
+// constants rv; Ab = J^T G and Db = G (the gather applies their factors cd and
+// hvcd), with (rho w)' and d3[DENS] held at zero at the z walls.  The lanes in
+// `mask` call it together.
 template <int DIR>
-__device__ __forceinline__ void jt_ieee(const double s[4][4], const double dg[4], const RowV& rv, double cd,
-                                        double hvcd, bool wall, unsigned mask, double Ab[4], double Db[4]) {
+__device__ __forceinline__ void jt_ieee(const double s[4][4], const double Fb[4], const RowV& rv, bool wall,
+                                        unsigned mask, double Ab[4], double Db[4]) {
   double A[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) A[q] = ieee::interp12(s[q][0], s[q][1], s[q][2], s[q][3]);
@@ -305,12 +316,8 @@ __device__ __forceinline__ void jt_ieee(const double s[4][4], const double dg[4]
       if (big) dp = rv.Q * exp((kGamma - 1.0) * log1p(d));
     }
   }
-  double Fb[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    Fb[q] = cd * dg[q];
-    Db[q] = hvcd * dg[q];
-  }
+  for (int q = 0; q < 4; ++q) Db[q] = Fb[q];
   if (DIR == MW_DIR_X) {
     const double y = fma(Fb[1], u, fma(Fb[2], w, Fb[3] * th));  // Fb1 u + Fb2 w + Fb3 th
     Ab[DENS] = -(u * y);
@@ -387,19 +394,19 @@ __device__ __forceinline__ void store_cell(const VjpArgs& a, long long o, const 
 }
 
 // The transposed taps of interfaces p0-1+l .. p0+2+l (slots l .. l+3) on their cell.
-__device__ __forceinline__ double gather4(const double* ab, const double* db, int l) {
-  const double ca = fma(7.0, ab[l + 1] + ab[l + 2], -(ab[l] + ab[l + 3])) * (1.0 / 12.0);
+__device__ __forceinline__ double gather4(const VjpArgs& a, const double* ab, const double* db, int l) {
+  const double ca = fma(7.0, ab[l + 1] + ab[l + 2], -(ab[l] + ab[l + 3]));
   const double ce = fma(3.0, db[l + 2] - db[l + 1], db[l] - db[l + 3]);
-  return ca + ce;
+  return fma(a.kc * (1.0 / 12.0), ca, a.ke * ce);
 }
 
 __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV* rows, int nseg, long long total) {
   __shared__ SmemFX sm;
+  overlap_wait();
   zero_frame(a);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long b0 = total * blockIdx.x / gridDim.x, b1 = total * (blockIdx.x + 1) / gridDim.x;
   const long long g0 = b0 + (b1 - b0) * w / kFXWarps, g1 = b0 + (b1 - b0) * (w + 1) / kFXWarps;
-  const double cd = a.dt_stage / a.d, hvcd = -a.hv * cd;
   auto col = [&](int p) { return ((p % a.nx) + a.nx) % a.nx + kHs; };  // periodic
   for (long long g = g0; g < g1; ++g) {
     const int k = (int)(g / nseg), p0 = (int)(g - (long long)k * nseg) * kFVCells;
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
         dg[q] = sm.g[w][q][lane + 1] - sm.g[w][q][lane];
       }
       const RowV rv = MW_AT(rows, k + kHs, 2 * a.nz + 5);
-      jt_ieee<MW_DIR_X>(s, dg, rv, cd, hvcd, false, 0xffffffffu, Ab, Db);
+      jt_ieee<MW_DIR_X>(s, dg, rv, false, 0xffffffffu, Ab, Db);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         sm.ab[w][q][lane] = Ab[q];
@@ -436,7 +443,7 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
     if (lane < kFVCells && t < a.nx) {
       double acc[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = gather4(sm.ab[w][q], sm.db[w][q], lane);
+      for (int q = 0; q < 4; ++q) acc[q] = gather4(a, sm.ab[w][q], sm.db[w][q], lane);
       store_cell(a, row + t + kHs, acc);
     }
     __syncwarp();
@@ -448,8 +455,8 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
 // fused z kernel over tiles of 4 columns x 29 rows staged through shared
 // memory was slower at 512 x 256: 39.6 against 18.8 + 17.7 us per call.)
 __global__ void k_vjp_iface_ieee_z(VjpArgs a, const RowV* rows) {
+  overlap_wait();
   const long long n = a.nif;
-  const double cd = a.dt_stage / a.d, hvcd = -a.hv * cd;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
     const long long idx = base + threadIdx.x;
@@ -464,7 +471,7 @@ __global__ void k_vjp_iface_ieee_z(VjpArgs a, const RowV* rows) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) dg[q] = (k < a.nz ? gval(a, q, k, c) : 0.0) - (k > 0 ? gval(a, q, k - 1, c) : 0.0);
     const RowV rv = MW_AT(rows, a.nz + 2 * kHs + k, 2 * a.nz + 5);
-    jt_ieee<MW_DIR_Z>(s, dg, rv, cd, hvcd, k == 0 || k == a.nz, mask, Ab, Db);
+    jt_ieee<MW_DIR_Z>(s, dg, rv, k == 0 || k == a.nz, mask, Ab, Db);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       MW_WS(a, q * n + idx) = Ab[q];
@@ -524,8 +531,8 @@ extern "C" size_t mw_dirstage_vjp_workspace_bytes(int nx, int nz) {
 static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const double* hyc, const double* hytc,
                      const double* hyi, const double* hyti, const double* hypi, const double* forcing,
                      const double* g_out, const double* g_base_a, const double* g_base_b, int add_g_out,
-                     double* g_dst, double dt_stage, int direction, int f64_mode, bool table_ready, void* workspace,
-                     size_t workspace_bytes, void* stream) {
+                     double* g_dst, double dt_stage, int direction, int f64_mode, bool table_ready, bool follows,
+                     void* workspace, size_t workspace_bytes, void* stream) {
   int st = check_grid(nx, nz);
   if (st) return st;
   MW_REQUIRE(finite_pos(dx) && finite_pos(dz) && finite_pos(dt_full), MW_ERR_INVALID_ARG,
@@ -574,13 +581,20 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
   a.gdst = g_dst;
   a.ws = (double*)workspace;
   a.nif = n_interfaces(nx, nz, direction);
+  const bool ieee = f64_mode == MW_F64_IEEE;  // its interface adjoints carry no factors
+  a.kc = ieee ? dt_stage / a.d : 1.0;
+  a.ke = ieee ? -a.hv * a.kc : 1.0;
   cudaStream_t s = (cudaStream_t)stream;
   RowV* rows = (RowV*)((double*)workspace + ieee_rows_off(nx, nz));
-  if (f64_mode == MW_F64_IEEE && !table_ready) {
-    k_vjp_rows_ieee<<<grid_for(2 * nz + 5, 128), 128, 0, s>>>(nz, hyc, hytc, hyi, hyti, hypi, rows);
-    if ((st = check_launch("vjp row-table launch"))) return st;
+  // Every launch of the call but its first may come in while the one before it ends (each waits before it touches
+  // anything); `follows`: a launch of the same call came before this stage.
+  if (ieee && !table_ready) {
+    st = launch_overlapping(k_vjp_rows_ieee, dim3(grid_for(2 * nz + 5, 128)), 128, 0, s, false, "vjp row table", nz, hyc,
+                            hytc, hyi, hyti, hypi, rows);
+    if (st) return st;
+    follows = true;
   }
-  if (f64_mode == MW_F64_IEEE && direction == MW_DIR_X) {  // one fused launch, a grid of resident CTAs at most
+  if (ieee && direction == MW_DIR_X) {  // one fused launch, a grid of resident CTAs at most
     int per_sm = 0, sms = 0, dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vjp_ieee_x, kFXThreads, 0);
@@ -590,25 +604,16 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
     const int nseg = (nx + kFVCells - 1) / kFVCells;
     const long long total = (long long)nseg * nz;
     const long long grid = std::max(1LL, std::min(resident, (total + kFXWarps - 1) / kFXWarps));
-    k_vjp_ieee_x<<<(unsigned)grid, kFXThreads, 0, s>>>(a, rows, nseg, total);
-    return check_launch("vjp launch");
+    return launch_overlapping(k_vjp_ieee_x, dim3((unsigned)grid), kFXThreads, 0, s, follows, "vjp", a, rows, nseg, total);
   }
-  if (f64_mode == MW_F64_IEEE) {
-    k_vjp_iface_ieee_z<<<grid_for(a.nif, 128), 128, 0, s>>>(a, rows);
-    if ((st = check_launch("vjp interface launch"))) return st;
-    k_vjp_gather<MW_DIR_Z><<<gather_grid(g), 128, 0, s>>>(a);
-    return check_launch("vjp gather launch");
-  }
-  if (direction == MW_DIR_X) {
-    k_vjp_iface<MW_DIR_X><<<grid_for(a.nif, 128), 128, 0, s>>>(a);
-    if ((st = check_launch("vjp interface launch"))) return st;
-    k_vjp_gather<MW_DIR_X><<<gather_grid(g), 128, 0, s>>>(a);
-  } else {
-    k_vjp_iface<MW_DIR_Z><<<grid_for(a.nif, 128), 128, 0, s>>>(a);
-    if ((st = check_launch("vjp interface launch"))) return st;
-    k_vjp_gather<MW_DIR_Z><<<gather_grid(g), 128, 0, s>>>(a);
-  }
-  return check_launch("vjp gather launch");
+  if (ieee)
+    st = launch_overlapping(k_vjp_iface_ieee_z, dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a, rows);
+  else
+    st = launch_overlapping(direction == MW_DIR_X ? k_vjp_iface<MW_DIR_X> : k_vjp_iface<MW_DIR_Z>,
+                            dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a);
+  if (st) return st;
+  return launch_overlapping(direction == MW_DIR_X ? k_vjp_gather<MW_DIR_X> : k_vjp_gather<MW_DIR_Z>, gather_grid(g), 128,
+                            0, s, true, "vjp gather", a);
 }
 
 extern "C" int mw_dirstage_vjp_f64(int nx, int nz, double dx, double dz, double dt_full, const double* hyc,
@@ -618,7 +623,7 @@ extern "C" int mw_dirstage_vjp_f64(int nx, int nz, double dx, double dz, double 
                                    int direction, int f64_mode, void* workspace, size_t workspace_bytes,
                                    void* stream) {
   return vjp_stage(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, forcing, g_out, g_base_a, g_base_b, add_g_out,
-                   g_dst, dt_stage, direction, f64_mode, false, workspace, workspace_bytes, stream);
+                   g_dst, dt_stage, direction, f64_mode, false, false, workspace, workspace_bytes, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -641,21 +646,21 @@ extern "C" int mw_step_vjp_f64(int nx, int nz, double dx, double dz, double dt_f
   const int dirs[2] = {reverse ? MW_DIR_X : MW_DIR_Z, reverse ? MW_DIR_Z : MW_DIR_X};
   const double* cur = g_out;
   int st;
-  bool ready = false;  // split / IEEE modes: the background table is written by the first stage call
+  bool ready = false;  // a stage came before: the background table (split / IEEE modes) is written by the first
   for (int d = 1; d >= 0; --d) {
     const double* S = stages + (3 * d) * n;
     const double* s1 = S + n;
     const double* s2 = S + 2 * n;
     double* out = d == 1 ? gC : g_in;
     if ((st = vjp_stage(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, s2, cur, nullptr, nullptr, 0, gA, dt,
-                        dirs[d], f64_mode, ready, workspace, workspace_bytes, stream)))
+                        dirs[d], f64_mode, ready, ready, workspace, workspace_bytes, stream)))
       return st;
     ready = true;
     if ((st = vjp_stage(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, s1, gA, nullptr, nullptr, 0, gB, dt / 2,
-                        dirs[d], f64_mode, ready, workspace, workspace_bytes, stream)))
+                        dirs[d], f64_mode, ready, ready, workspace, workspace_bytes, stream)))
       return st;
     if ((st = vjp_stage(nx, nz, dx, dz, dt_full, hyc, hytc, hyi, hyti, hypi, S, gB, cur, gA, 1, out, dt / 3, dirs[d],
-                        f64_mode, ready, workspace, workspace_bytes, stream)))
+                        f64_mode, ready, ready, workspace, workspace_bytes, stream)))
       return st;
     cur = out;
   }
