@@ -23,9 +23,9 @@
 // taps.  MW_F64_IEEE (the fewest FP64 operations: values scaled by 12, 1/rho
 // by a Newton step, dp/d(rho theta) = gamma P_row (1 + delta)^(gamma-1) /
 // (rho theta)_bg by its binomial series, per-row constants from a table in the
-// workspace) runs the same two kernels in z and, in x, one kernel that computes
-// each warp segment's interface adjoints into shared memory and gathers them
-// there.
+// workspace) runs one kernel in either direction, which computes the interface
+// adjoints of a warp's segment (x) or a CTA's tile (z) into shared memory and
+// gathers them there.
 #include <algorithm>
 
 #include "mw_common.cuh"
@@ -149,6 +149,14 @@ __global__ void k_vjp_iface(VjpArgs a) {
   }
 }
 
+// g_dst of one value from its gathered adjoint: + g_out (add_gout), + the bases, which may be far larger, last.
+__device__ __forceinline__ void store_value(const VjpArgs& a, long long oq, double v) {
+  if (a.add_gout) v += MW_AT(a.gout, oq, 4 * a.plane);
+  if (a.base_a) v += MW_AT(a.base_a, oq, 4 * a.plane);
+  if (a.base_b) v += MW_AT(a.base_b, oq, 4 * a.plane);
+  MW_AT(a.gdst, oq, 4 * a.plane) = v;
+}
+
 // Cell gather: gdst = base_a + base_b + add_gout * gout + sbar (interior); halo cells of gdst = 0.
 // The adjoint of interior cell (k, i) gathered from the interface adjoints
 // of its taps by the general rule: periodic wrap in x, the wall rule's halo
@@ -244,11 +252,7 @@ __global__ void __launch_bounds__(128) k_vjp_gather(VjpArgs a) {
     if (DIR == MW_DIR_Z) acc[DENS] -= a.dt_stage * kGrav * gval(a, WMOM, k, i);
     for (int q = 0; q < 4; ++q) {
       const long long o = q * a.plane + idx;
-      double v = acc[q];
-      if (a.add_gout) v += MW_AT(a.gout, o, 4 * a.plane);
-      if (a.base_a) v += MW_AT(a.base_a, o, 4 * a.plane);
-      if (a.base_b) v += MW_AT(a.base_b, o, 4 * a.plane);
-      MW_AT(a.gdst, o, 4 * a.plane) = v;
+      store_value(a, o, acc[q]);
     }
   }
 }
@@ -359,51 +363,31 @@ struct SmemFX {
   double db[kFXWarps][4][32];     // Db
 };
 
-// g_dst's halo cells: zero (the frame, strided over every thread of the launch).
+// g_dst's halo cells: zero (its rows strided over the CTAs of the launch).
 __device__ __forceinline__ void zero_frame(const VjpArgs& a) {
   const int rows = a.nz + 2 * kHs;
-  const long long hrow = 2LL * kHs * a.pitch;               // the halo rows' cells
-  const long long frame = hrow + 2LL * kHs * a.nz;          // + the halo columns of the interior rows
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < frame; e += step) {
-    long long o;
-    if (e < hrow) {
-      const int r = (int)(e / a.pitch), c = (int)(e % a.pitch);
-      o = (long long)(r < kHs ? r : rows - 2 * kHs + r) * a.pitch + c;
-    } else {
-      const long long e2 = e - hrow;
-      const int k = (int)(e2 / (2 * kHs)), h = (int)(e2 % (2 * kHs));
-      o = (long long)(k + kHs) * a.pitch + (h < kHs ? h : a.nx + h);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    const bool all = r < kHs || r >= a.nz + kHs;  // a halo row, or the halo columns of an interior one
+    const int n = all ? a.pitch : 2 * kHs;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+      const long long o = (long long)r * a.pitch + (all || t < kHs ? t : a.nx + t);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) MW_AT(a.gdst, q * a.plane + o, 4 * a.plane) = 0.0;
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) MW_AT(a.gdst, q * a.plane + o, 4 * a.plane) = 0.0;
   }
 }
 
-// g_dst of one cell from its gathered adjoints acc: + g_out (add_gout), + the bases.
-__device__ __forceinline__ void store_cell(const VjpArgs& a, long long o, const double acc[4]) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const long long oq = q * a.plane + o;
-    double v = acc[q];
-    if (a.add_gout) v += MW_AT(a.gout, oq, 4 * a.plane);
-    if (a.base_a) v += MW_AT(a.base_a, oq, 4 * a.plane);
-    if (a.base_b) v += MW_AT(a.base_b, oq, 4 * a.plane);
-    MW_AT(a.gdst, oq, 4 * a.plane) = v;
-  }
-}
-
-// The transposed taps of interfaces p0-1+l .. p0+2+l (slots l .. l+3) on their cell.
-__device__ __forceinline__ double gather4(const VjpArgs& a, const double* ab, const double* db, int l) {
-  const double ca = fma(7.0, ab[l + 1] + ab[l + 2], -(ab[l] + ab[l + 3]));
-  const double ce = fma(3.0, db[l + 2] - db[l + 1], db[l] - db[l + 3]);
+// The transposed taps of interface adjoints A0 .. A3, D0 .. D3 (interfaces i - 1 .. i + 2) on cell i.
+__device__ __forceinline__ double gather4(const VjpArgs& a, double A0, double A1, double A2, double A3, double D0,
+                                          double D1, double D2, double D3) {
+  const double ca = fma(7.0, A1 + A2, -(A0 + A3));
+  const double ce = fma(3.0, D2 - D1, D0 - D3);
   return fma(a.kc * (1.0 / 12.0), ca, a.ke * ce);
 }
 
 __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV* rows, int nseg, long long total) {
   __shared__ SmemFX sm;
   overlap_wait();
-  zero_frame(a);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long b0 = total * blockIdx.x / gridDim.x, b1 = total * (blockIdx.x + 1) / gridDim.x;
   const long long g0 = b0 + (b1 - b0) * w / kFXWarps, g1 = b0 + (b1 - b0) * (w + 1) / kFXWarps;
@@ -443,41 +427,168 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
     if (lane < kFVCells && t < a.nx) {
       double acc[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = gather4(a, sm.ab[w][q], sm.db[w][q], lane);
-      store_cell(a, row + t + kHs, acc);
+      for (int q = 0; q < 4; ++q) {
+        const double* ab = sm.ab[w][q] + lane;
+        const double* db = sm.db[w][q] + lane;
+        acc[q] = gather4(a, ab[0], ab[1], ab[2], ab[3], db[0], db[1], db[2], db[3]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + row + t + kHs, acc[q]);
     }
     __syncwarp();
   }
+  zero_frame(a);
 }
 
-// z: the interface adjoints of k_vjp_iface (same Jacobian, same workspace
-// layout) by jt_ieee, one thread per interface; k_vjp_gather follows.  (A
-// fused z kernel over tiles of 4 columns x 29 rows staged through shared
-// memory was slower at 512 x 256: 39.6 against 18.8 + 17.7 us per call.)
-__global__ void k_vjp_iface_ieee_z(VjpArgs a, const RowV* rows) {
-  overlap_wait();
-  const long long n = a.nif;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const long long idx = base + threadIdx.x;
-    const unsigned mask = __ballot_sync(0xffffffffu, idx < n);  // base is uniform over the block
-    if (idx >= n) continue;
-    const int k = (int)(idx / a.nx), c = (int)(idx % a.nx);
-    double s[4][4], dg[4], Ab[4], Db[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[q][j] = zval(a, q, k - 2 + j, c + kHs);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) dg[q] = (k < a.nz ? gval(a, q, k, c) : 0.0) - (k > 0 ? gval(a, q, k - 1, c) : 0.0);
-    const RowV rv = MW_AT(rows, a.nz + 2 * kHs + k, 2 * a.nz + 5);
-    jt_ieee<MW_DIR_Z>(s, dg, rv, k == 0 || k == a.nz, mask, Ab, Db);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      MW_WS(a, q * n + idx) = Ab[q];
-      MW_WS(a, (4 + q) * n + idx) = Db[q];
+// ---- IEEE-FP64 stage adjoint, z: one kernel ---------------------------------
+// A CTA takes 32 columns of up to kFZRows rows.  Its warps first compute the
+// tile's rows + 3 interface adjoints, each warp a stretch of consecutive
+// interfaces down its 32 columns (the four taps and g move along in
+// registers, one new row of each per interface), into shared memory; then,
+// registers, one new row of each per interface), into shared memory; then,
+// after the one barrier, each gathers a stretch of rows the same way (one new
+// interface per row).
+//
+// Bound: FP64 (512 x 256, a stage without bases: 2375 instructions on the
+// fullest SM at 16 cycles each, 38000 of its 53500 active cycles; the rest is
+// the first and last loads and stores, which all warps meet together).  30.8 us
+// a stage at 512 x 256, with the bases counted in, against 14.8 + 21 us for
+// the interface adjoints and the gather as two kernels with the 8 values per
+// interface in memory between them.  Sixteen warps a CTA: 33 us.  Rows read
+// one interface ahead: no gain.
+constexpr int kFZRows = 29;  // 32 interfaces: 64 KB of shared memory
+constexpr int kFZThreads = 256;
+constexpr int kFZWarps = kFZThreads / 32;
+
+inline int fz_smem(int rows) { return (int)sizeof(double) * 8 * 32 * (rows + 3); }
+
+// The wall rule's halo taps on row k (0 or nz - 1, or both): halo row t passes weight wq of its adjoint to row `src`.
+__device__ __forceinline__ void gather_wall(const VjpArgs& a, const double* ws, int f0, int k, double acc[4]) {
+  for (int t = -2; t <= a.nz + 1; t = t == -1 ? a.nz : t + 1) {
+    const int src = t < 0 ? 0 : a.nz - 1;
+    if (src != k) continue;
+    const double wu = MW_VC(a, hyc, t + kHs) / MW_VC(a, hyc, src + kHs);
+    for (int j = 0; j < 4; ++j) {
+      const int f = t + 2 - j;
+      if (f < 0 || f > a.nz) continue;
+      const double* c = ws + (f - f0) * 256;
+      for (int q = 0; q < 4; ++q) {
+        if (q == WMOM) continue;
+        acc[q] += (q == UMOM ? wu : 1.0) * (a.kc * (kC[j] * c[q * 32]) + a.ke * (kE[j] * c[(4 + q) * 32]));
+      }
     }
   }
+}
+
+__global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV* rows, int tile_rows) {
+  extern __shared__ double fz_ws[];  // [interface][Ab 0..3, Db 0..3][column]
+  overlap_wait();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nxt = (a.nx + 31) / 32, nzt = (a.nz + tile_rows - 1) / tile_rows;
+  for (long long tile = blockIdx.x; tile < (long long)nxt * nzt; tile += gridDim.x) {
+    const int k0 = (int)(tile / nxt) * tile_rows, k1 = min(a.nz, k0 + tile_rows);
+    const int c = (int)(tile % nxt) * 32 + lane;
+    const bool in = c < a.nx;
+    const int col = min(c, a.nx - 1) + kHs;  // columns past the grid repeat the last one and are not stored
+    const int fa = max(0, k0 - 1), fb = min(a.nz, k1 + 1);  // interfaces fa .. fb
+    double* ws = fz_ws + lane;
+    {
+      const int n = fb - fa + 1, f0 = fa + n * w / kFZWarps, f1 = fa + n * (w + 1) / kFZWarps;
+      double s[4][4], gl[4];
+      if (f0 < f1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+          for (int j = 1; j < 4; ++j) s[q][j] = zval(a, q, f0 - 3 + j, col);
+          gl[q] = f0 > 0 ? gval(a, q, f0 - 1, col - kHs) : 0.0;
+        }
+      }
+      for (int f = f0; f < f1; ++f) {
+        double dg[4], Ab[4], Db[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          s[q][0] = s[q][1];
+          s[q][1] = s[q][2];
+          s[q][2] = s[q][3];
+          s[q][3] = zval(a, q, f + 1, col);
+          const double gr = f < a.nz ? gval(a, q, f, col - kHs) : 0.0;
+          dg[q] = gr - gl[q];
+          gl[q] = gr;
+        }
+        const RowV rv = MW_AT(rows, a.nz + 2 * kHs + f, 2 * a.nz + 5);
+        jt_ieee<MW_DIR_Z>(s, dg, rv, f == 0 || f == a.nz, 0xffffffffu, Ab, Db);
+        double* o = ws + (f - fa) * 256;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          o[q * 32] = Ab[q];
+          o[(4 + q) * 32] = Db[q];
+        }
+      }
+    }
+    __syncthreads();
+    {
+      const int n = k1 - k0, r0 = k0 + n * w / kFZWarps, r1 = k0 + n * (w + 1) / kFZWarps;
+      double A[4][4], D[4][4];
+      // interface f of the tile; one outside [0, nz] has no adjoint
+      auto load = [&](int f, int j) {
+        const bool has = f >= 0 && f <= a.nz;
+        const double* p = ws + (f - fa) * 256;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          A[q][j] = has ? p[q * 32] : 0.0;
+          D[q][j] = has ? p[(4 + q) * 32] : 0.0;
+        }
+      };
+      if (r0 < r1) {
+        load(r0 - 1, 1);
+        load(r0, 2);
+        load(r0 + 1, 3);
+      }
+      for (int k = r0; k < r1; ++k) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            A[q][j] = A[q][j + 1];
+            D[q][j] = D[q][j + 1];
+          }
+        load(k + 2, 3);
+        double acc[4];
+        const long long o = (long long)(k + kHs) * a.pitch + col;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          acc[q] = gather4(a, A[q][0], A[q][1], A[q][2], A[q][3], D[q][0], D[q][1], D[q][2], D[q][3]);
+        if (k == 0 || k == a.nz - 1) gather_wall(a, ws, fa, k, acc);
+        acc[DENS] = fma(-a.dt_stage * kGrav, gval(a, WMOM, k, col - kHs), acc[DENS]);
+        if (in)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + o, acc[q]);
+      }
+    }
+    __syncthreads();
+  }
+  zero_frame(a);
+}
+
+// Rows of a tile of k_vjp_ieee_z: those with the fewest rounds of a warp's work,
+// interfaces and rows counted alike (about 40 FP64 operations each) and one
+// more per tile for its loads, on the SM with the most tiles; of equals the
+// tallest, which recompute the fewest interfaces.  512 x 256: 29 rows, 144 tiles,
+// 30.8 us.  From a third to twice the charge per tile: the same times within 1 %
+// from 100 x 50 to 640 x 448.
+inline int fz_rows(int nx, int nz, int sms) {
+  const long long nxt = (nx + 31) / 32;
+  int best = std::min(nz, kFZRows);
+  double cost = 0;
+  for (int r = 1; r <= std::min(nz, kFZRows); ++r) {
+    const long long nzt = (nz + r - 1) / r, per_sm = (nxt * nzt + sms - 1) / sms;
+    const double c = per_sm * ((r + 3 + 7) / 8 + (r + 7) / 8 + 1.0);
+    if (r == 1 || c <= cost) {
+      cost = c;
+      best = r;
+    }
+  }
+  return best;
 }
 
 // k_vjp_gather: 128 columns per CTA, the rows strided over grid.y.
@@ -606,11 +717,20 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
     const long long grid = std::max(1LL, std::min(resident, (total + kFXWarps - 1) / kFXWarps));
     return launch_overlapping(k_vjp_ieee_x, dim3((unsigned)grid), kFXThreads, 0, s, follows, "vjp", a, rows, nseg, total);
   }
-  if (ieee)
-    st = launch_overlapping(k_vjp_iface_ieee_z, dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a, rows);
-  else
-    st = launch_overlapping(direction == MW_DIR_X ? k_vjp_iface<MW_DIR_X> : k_vjp_iface<MW_DIR_Z>,
-                            dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a);
+  if (ieee) {
+    int sms = 0, dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_vjp_ieee_z, cudaFuncAttributeMaxDynamicSharedMemorySize, fz_smem(kFZRows));
+    if (e != cudaSuccess) return fail(MW_ERR_CUDA, "vjp setup: %s", cudaGetErrorString(e));
+    const int tile_rows = fz_rows(nx, nz, sms);
+    const long long tiles = (long long)((nx + 31) / 32) * ((nz + tile_rows - 1) / tile_rows);
+    return launch_overlapping(k_vjp_ieee_z, dim3((unsigned)std::min(tiles, 1LL << 30)), kFZThreads, fz_smem(tile_rows), s,
+                              follows, "vjp", a, rows, tile_rows);
+  }
+  st = launch_overlapping(direction == MW_DIR_X ? k_vjp_iface<MW_DIR_X> : k_vjp_iface<MW_DIR_Z>,
+                          dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a);
   if (st) return st;
   return launch_overlapping(direction == MW_DIR_X ? k_vjp_gather<MW_DIR_X> : k_vjp_gather<MW_DIR_Z>, gather_grid(g), 128,
                             0, s, true, "vjp gather", a);
