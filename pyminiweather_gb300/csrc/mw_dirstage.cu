@@ -1051,9 +1051,9 @@ static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, doubl
                      int f64_mode, unsigned flags, cudaStream_t s) {
   flags = user_flags(flags);
   LinePlan plan;
-  if (f64_mode == MW_F64_IEEE)
-    if (const int st = line_ieee_plan(nx, nz, &plan)) return st;
+  if (const int st = line_plan_of(f64_mode, nx, nz, &plan)) return st;
   if (plan.fits) {
+    const auto launch_line = f64_mode == MW_F64_SPLIT ? launch_line_split : launch_line_ieee;
     const bool halo = flags & MW_FLAG_WRITE_HALO;
     LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, state, state, nullptr, nullptr, halo ? state : nullptr,
                halo ? state_tmp : nullptr};
@@ -1062,8 +1062,8 @@ static int steps_f64(int nx, int nz, double dx, double dz, double dt_full, doubl
         a.s2 = n + 1 == nsteps && d == 1 ? state_tmp : nullptr;  // what the call leaves in state_tmp
         a.in = plan.cut && d == 1 ? scratch : state;  // cut lines: state -> scratch -> state, else in place
         a.out = plan.cut && d == 0 ? scratch : state;
-        const int st = launch_line_ieee(plan, nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
-                                        n + d > 0, s);
+        const int st = launch_line(plan, nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
+                                   n + d > 0, s);
         if (st) return st;
       }
       *reverse = *reverse ? 0 : 1;
@@ -1290,13 +1290,14 @@ extern "C" int mw_step_record_f64(int nx, int nz, double dx, double dz, double d
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "stage copy: %s", cudaGetErrorString(e));
   const int dirs[2] = {reverse ? MW_DIR_X : MW_DIR_Z, reverse ? MW_DIR_Z : MW_DIR_X};
   LinePlan plan;
-  if (f64_mode == MW_F64_IEEE && (st = line_ieee_plan(nx, nz, &plan))) return st;
+  if ((st = line_plan_of(f64_mode, nx, nz, &plan))) return st;
   if (plan.fits) {
+    const auto launch_line = f64_mode == MW_F64_SPLIT ? launch_line_split : launch_line_ieee;
     for (int d = 0; d < 2; ++d) {
       double* S = stages + 3 * d * n;
       const LineArgs a{hyc, hytc, hyi, hyti, hypi, src_w, S, d == 0 ? stages + 3 * n : state_out, S + n, S + 2 * n,
                        nullptr, nullptr};
-      if ((st = launch_line_ieee(plan, nx, nz, dx, dz, dt_full, dt, a, dirs[d], d > 0, s))) return st;
+      if ((st = launch_line(plan, nx, nz, dx, dz, dt_full, dt, a, dirs[d], d > 0, s))) return st;
     }
     return MW_OK;
   }

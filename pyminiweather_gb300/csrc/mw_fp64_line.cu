@@ -25,6 +25,7 @@
 #include "mw_common.cuh"
 #include "mw_fp64_flux.cuh"
 #include "mw_fp64_line.cuh"
+#include "mw_line.cuh"
 #include "mw_pow.cuh"
 
 namespace mw {
@@ -32,23 +33,10 @@ namespace ieee {
 
 // Most warps per CTA with SL slots per lane (as their registers allow).
 __host__ __device__ constexpr int line_warps(int sl) { return sl == 1 ? 20 : 16; }
-constexpr int kLineMax = 8;            // most lines per CTA
-constexpr size_t kLineSmem = 200 << 10;
-
-struct LineParams {
-  LineArgs a;
-  int n, nlines;         // cells per line, lines
-  int log_lines, runs;   // lines per CTA (a power of two), runs per line
-  int run;               // cells per run
-  int pieces, piece;     // pieces per line, cells per piece
-  int lp;                // shared-memory pitch of a line
-  int pitch;
-  long long plane;
+struct LineParams : LineGeom {
   double HV, IHV;        // HV = -12 hv of the direction and 1 / HV
   double c[3], dt[3];    // per stage HV dt_stage / (12 d) and dt_stage
 };
-
-#define MW_LG(p, off) MW_AT((p), (off), 4 * P.plane)
 
 // Line l of variable q in one of the two buffers.
 __device__ __forceinline__ double* line_at(const LineParams& P, double* buf, int q, int l) {
@@ -71,47 +59,6 @@ __device__ __forceinline__ void put(double* line, int q, int c, int n, bool whol
       for (int h = 0; h < 2; ++h) line[h - 2] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[h] : v);
     if (c == n - 1)
       for (int h = 0; h < 2; ++h) line[n + h] = q == WMOM ? 0.0 : (q == UMOM ? v * hr[2 + h] : v);
-  }
-}
-
-// The halo cells that cell c of a line is the source of, in a global array.
-template <int DIR>
-__device__ __forceinline__ void halo_out(const LineParams& P, double* g, int line, int c, const double v[4],
-                                         const double* hr) {
-  const int n = P.n;
-  if (DIR == MW_DIR_X) {
-    const long long row = (long long)(line + kHs) * P.pitch;
-    for (int q = 0; q < 4; ++q) {
-      if (c < kHs) MW_LG(g, q * P.plane + row + n + kHs + c) = v[q];
-      if (c >= n - kHs) MW_LG(g, q * P.plane + row + c - n + kHs) = v[q];
-    }
-  } else {
-    for (int q = 0; q < 4; ++q)
-      for (int h = 0; h < 4; ++h)
-        if (c == (h < 2 ? 0 : n - 1))
-          MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + line) =
-              q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
-  }
-}
-
-// Cells [ca, cb) of the CTA's lines, between a global array and shared memory
-// (x: periodic).  x: a warp per line and variable; z: consecutive threads take
-// the CTA's columns of a row.
-template <int DIR, typename Fn>
-__device__ __forceinline__ void each_cell(const LineParams& P, int l0, int nl, int ca, int cb, Fn fn) {
-  if (DIR == MW_DIR_X) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int ql = w; ql < 4 * nl; ql += nw) {
-      const int q = ql / nl, l = ql - q * nl;
-      const long long o = q * P.plane + (long long)(l0 + l + kHs) * P.pitch + kHs;
-      for (int c = ca + lane; c < cb; c += 32) fn(q, l, c, o + (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c)));
-    }
-  } else {
-    for (int q = 0; q < 4; ++q)
-      for (int i = threadIdx.x; i < ((cb - ca) << P.log_lines); i += blockDim.x) {
-        const int l = i & ((1 << P.log_lines) - 1), c = ca + (i >> P.log_lines);
-        if (l < nl) fn(q, l, c, q * P.plane + (long long)(c + kHs) * P.pitch + l0 + l + kHs);
-      }
   }
 }
 
@@ -263,20 +210,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
         MW_LG(g, o) = line_at(P, dst, q, ll)[c];
       });
   }
-  // the four x-halo columns of the wall halo rows, from the halo columns' own first and last rows
-  if (DIR == MW_DIR_Z && blockIdx.x == 0 && threadIdx.x < 8) {
-    double* g = threadIdx.x < 4 ? a.halo_in : a.halo_tmp;
-    const int col = (threadIdx.x & 2) ? P.nlines + (threadIdx.x & 3) : (threadIdx.x & 1);
-    if (g)
-      for (int e = 0; e < 2; ++e) {
-        double v[4];
-        for (int q = 0; q < 4; ++q) v[q] = MW_LG(g, q * P.plane + (long long)(e ? n + kHs - 1 : kHs) * P.pitch + col);
-        for (int q = 0; q < 4; ++q)
-          for (int h = 2 * e; h < 2 * e + 2; ++h)
-            MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + col) =
-                q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
-      }
-  }
+  if (DIR == MW_DIR_Z && blockIdx.x == 0 && threadIdx.x < 8) halo_corners(P, hr);
 }
 
 template <int DIR, int SL>
@@ -293,19 +227,8 @@ int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, bool 
   return launch_overlapping(k_line_ieee<DIR, SL>, dim3((unsigned)ctas), threads, smem, stream, overlap, "line kernel", P);
 }
 
-int line_sms(int* out) {
-  static std::atomic<int> cache[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return fail(MW_ERR_CUDA, "cudaGetDevice failed");
-  const bool cached = dev >= 0 && dev < 64;
-  if (cached && (*out = cache[dev].load(std::memory_order_relaxed)) > 0) return MW_OK;
-  const cudaError_t e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return fail(MW_ERR_CUDA, "device query: %s", cudaGetErrorString(e));
-  if (cached) cache[dev].store(*out, std::memory_order_relaxed);
-  return MW_OK;
-}
-
-constexpr int run_cells(int sl) { return 32 * sl - 2; }
+// two slots of a run repeat its neighbours' (x pass of mw_fp64_stage.cu)
+constexpr LineKind kIeeeLines = {2, {line_warps(1), line_warps(2)}, {96, 128}, 2, 64, 0, 0.0};
 
 constexpr int kMaxPieces = 16;
 
@@ -321,28 +244,44 @@ constexpr int kMaxPieces = 16;
 // slots per lane with less than two warps per partition wait on their own
 // latency.  The factors near 1 break ties: more resident CTAs (their heads and
 // tails fill one another), fewer pieces, fewer CTAs, in z whole sectors.
-LineSpread spread_lines(int n, int nlines, bool isx, int sms) {
+//
+// The double-FP32 form's warps hide one another's latency instead, and its time
+// follows the warps of the SM with the most CTAs, partition by partition, and
+// part of a CTA's own for its head and tail, less where more CTAs are resident
+// to fill them.  CTAs of under four warps leave partitions idle, and single
+// columns use a quarter of a sector.  Over every spread of eleven grids from
+// 100x50 to 1250x799, both directions in turn, the rule takes one within 2 % of
+// the fastest but for 300x150, x (4 %): 512x256, x: whole rows in 17 warps 46.7 us
+// a step, five pieces of four warps 43.1; 880x620, z: twelve pieces of two columns
+// in four warps 122 us, of one column in two warps 129, three in 14 warps 150.
+LineSpread spread_lines(const LineKind& kind, int n, int nlines, bool isx, int sms) {
   LineSpread best;
   double least = 0.0;
-  for (int sl = 1; sl <= 2; ++sl)
+  for (int sl = 1; sl <= kind.max_slots; ++sl)
     for (int pieces = 1; pieces == 1 || (pieces <= kMaxPieces && (n + pieces - 1) / pieces >= 24); ++pieces) {
       const int piece = (n + pieces - 1) / pieces;
       if ((n + piece - 1) / piece != pieces) continue;  // an empty last piece
       const int range = pieces == 1 ? n : piece + 8;
       if (pieces > 1 && range >= n) break;
-      const int runs = (range + run_cells(sl) - 1) / run_cells(sl);
+      const int cells = 32 * sl - kind.shared_slots, runs = (range + cells - 1) / cells;
       const int lp = (pieces == 1 ? n + 2 * kHs : piece + 12) | 1;
       for (int lg = 0; (1 << lg) <= kLineMax; ++lg) {
         const int warps = runs << lg;
-        const size_t smem = (size_t)lp * sizeof(double) * 8 << lg;
-        if (warps > line_warps(sl) || smem > kLineSmem) break;
-        const int resident = std::min((int)(65536 / ((sl == 1 ? 96 : 128) * 32 * warps)), (int)((220 << 10) / smem));
+        const size_t smem = line_smem(kind, lp, lg, isx);
+        if (warps > kind.warps[sl - 1] || smem > kLineSmem) break;
+        const int resident = std::min((int)(65536 / (kind.regs[sl - 1] * 32 * warps)), (int)((220 << 10) / smem));
         const double load = (double)((nlines + (1 << lg) - 1) >> lg) * pieces / sms;
         const double turns = std::min(std::ceil(load / resident) * resident, load + 0.5 * resident) * warps / 4.0;
         const double once = std::ceil(load) * warps / 4.0;
-        double cost = sl * (load <= resident ? 0.1 * once + 0.9 * std::ceil(once) : turns);
-        cost *= (1.0 + 0.1 / resident) * (1.0 + 0.001 * load) * (pieces > 1 ? 1.01 : 1.0) *
-                (!isx && lg == 0 ? 1.03 : 1.0) * (sl == 2 && once < 2.0 ? 1.3 : 1.0);
+        double cost;
+        if (kind.tail > 0.0) {
+          cost = (once + kind.tail * std::max(warps, 4)) * (1.0 + 0.3 / resident) * (1.0 + 0.001 * pieces) *
+                 (warps < 4 ? 1.1 : 1.0) * (!isx && lg == 0 ? 1.2 : 1.0);
+        } else {
+          cost = sl * (load <= resident ? 0.1 * once + 0.9 * std::ceil(once) : turns);
+          cost *= (1.0 + 0.1 / resident) * (1.0 + 0.001 * load) * (pieces > 1 ? 1.01 : 1.0) *
+                  (!isx && lg == 0 ? 1.03 : 1.0) * (sl == 2 && once < 2.0 ? 1.3 : 1.0);
+        }
         if (best.sl == 0 || cost < least) {
           least = cost;
           const int run = (range + runs - 1) / runs;
@@ -355,16 +294,34 @@ LineSpread spread_lines(int n, int nlines, bool isx, int sms) {
 
 }  // namespace ieee
 
+int line_sms(int* out) {
+  static std::atomic<int> cache[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fail(MW_ERR_CUDA, "cudaGetDevice failed");
+  const bool cached = dev >= 0 && dev < 64;
+  if (cached && (*out = cache[dev].load(std::memory_order_relaxed)) > 0) return MW_OK;
+  const cudaError_t e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return fail(MW_ERR_CUDA, "device query: %s", cudaGetErrorString(e));
+  if (cached) cache[dev].store(*out, std::memory_order_relaxed);
+  return MW_OK;
+}
+
+LinePlan line_plan(const LineKind& kind, int nx, int nz, int sms) {
+  LinePlan p;
+  p.x = ieee::spread_lines(kind, nx, nz, true, sms);
+  p.z = ieee::spread_lines(kind, nz, nx, false, sms);
+  p.fits = p.x.sl > 0 && p.z.sl > 0;
+  p.cut = p.x.pieces > 1 || p.z.pieces > 1;
+  return p;
+}
+
 int line_ieee_plan(int nx, int nz, LinePlan* plan) {
   using namespace ieee;
   *plan = LinePlan();
   if ((long long)nx * nz > kLineCellsMax) return MW_OK;
   int sms = 0, st = line_sms(&sms);
   if (st) return st;
-  plan->x = spread_lines(nx, nz, true, sms);
-  plan->z = spread_lines(nz, nx, false, sms);
-  plan->fits = plan->x.sl > 0 && plan->z.sl > 0;
-  plan->cut = plan->x.pieces > 1 || plan->z.pieces > 1;
+  *plan = line_plan(kIeeeLines, nx, nz, sms);
   return MW_OK;
 }
 
@@ -374,11 +331,6 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
   LineParams P;
   P.a = a;
   const bool isx = direction == MW_DIR_X;
-  const Geom g = make_geom(nx, nz);
-  P.n = isx ? nx : nz;
-  P.nlines = isx ? nz : nx;
-  P.pitch = g.pitch;
-  P.plane = g.plane;
   const double d = isx ? dx : dz;
   P.HV = ieee_hv(d, dt_full);
   P.IHV = 1.0 / P.HV;
@@ -388,15 +340,9 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
   }
   const LineSpread& sp = isx ? plan.x : plan.z;
   MW_REQUIRE(sp.pieces == 1 || a.in != a.out, MW_ERR_ALIAS, "a direction of cut lines needs another array for its result");
-  P.log_lines = sp.log_lines;
-  P.pieces = sp.pieces;
-  P.piece = sp.piece;
-  P.run = sp.run;
-  P.runs = sp.runs;
-  P.lp = sp.lp;
-  const int threads = 32 * (P.runs << P.log_lines);
-  const int ctas = ((P.nlines + (1 << P.log_lines) - 1) >> P.log_lines) * P.pieces;
-  const size_t smem = (size_t)P.lp * sizeof(double) * 8 << P.log_lines;
+  int ctas, threads;
+  set_line_geom(&P, sp, nx, nz, isx, &ctas, &threads);
+  const size_t smem = line_smem(kIeeeLines, P.lp, P.log_lines, isx);
   if (isx) return sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, overlap, stream)
                                : launch_line_t<MW_DIR_X, 2>(P, ctas, threads, smem, overlap, stream);
   return sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, overlap, stream)

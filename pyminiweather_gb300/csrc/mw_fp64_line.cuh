@@ -13,6 +13,11 @@ namespace mw {
 // 237 / 279, 990x495 354 / 387, 992x992 659 / 661, 1200x600 482 / 469).
 constexpr long long kLineCellsMax = 600000;
 
+// The double-FP32 form's (100x50 14 / 61, 300x150 18 / 73, 512x256 38 / 70, 700x500
+// 85 / 110, 880x620 120 / 134, 900x620 125 / 138; 600x1000 146 / 139, 1100x700
+// 170 / 166, 1250x799 213 / 201).
+constexpr long long kSplitLineCellsMax = 580000;
+
 struct LineArgs {
   const double* hyc;
   const double* hytc;
@@ -44,11 +49,39 @@ struct LinePlan {
 };
 int line_ieee_plan(int nx, int nz, LinePlan* plan);
 
+// What the spread of a form's lines depends on.
+struct LineKind {
+  int max_slots;        // slots per lane, at most
+  int warps[2];         // most warps per CTA with one and two slots
+  int regs[2];          // registers per thread with one and two slots
+  int shared_slots;     // slots of a run that its neighbour has too
+  int cell_bytes;       // shared memory per cell
+  int row_bytes;        // and per cell of a column's row table (z)
+  double tail;          // cost of a CTA's head and tail per warp (0: the IEEE form's rule)
+};
+inline size_t line_smem(const LineKind& kind, int lp, int log_lines, bool isx) {
+  return ((size_t)lp * kind.cell_bytes << log_lines) + (isx ? 0 : (size_t)lp * kind.row_bytes);
+}
+LinePlan line_plan(const LineKind& kind, int nx, int nz, int sms);
+int line_sms(int* out);  // SMs of the current device
+
+// The same of the double-FP32 form (mw_split_line.cu).
+int line_split_plan(int nx, int nz, LinePlan* plan);
+int launch_line_split(const LinePlan& plan, int nx, int nz, double dx, double dz, double dt_full, double dt,
+                      const LineArgs& a, int direction, bool overlap, cudaStream_t stream);
+
 // One direction of one step of size dt.  overlap: the kernel may start while
 // the one before it on the stream is finishing, and waits for it before it
 // touches the state; only for a launch behind another line kernel of the same
 // call (what it reads before the wait, the backgrounds, is then complete).
 int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz, double dt_full, double dt,
                      const LineArgs& a, int direction, bool overlap, cudaStream_t stream);
+
+// The plan of a form that has line kernels (else one that fits no grid).
+inline int line_plan_of(int f64_mode, int nx, int nz, LinePlan* plan) {
+  *plan = LinePlan();
+  return f64_mode == MW_F64_IEEE ? line_ieee_plan(nx, nz, plan)
+                                 : (f64_mode == MW_F64_SPLIT ? line_split_plan(nx, nz, plan) : MW_OK);
+}
 
 }  // namespace mw

@@ -1,0 +1,104 @@
+// mw_line.cuh -- what the line kernels of the IEEE-FP64 (mw_fp64_line.cu) and
+// double-FP32 (mw_split_line.cu) forms share: which cells a CTA holds, and the
+// passes over them between global and shared memory.
+#pragma once
+
+#include "mw_common.cuh"
+#include "mw_fp64_line.cuh"
+
+namespace mw {
+namespace {
+
+constexpr int kLineMax = 8;            // most lines per CTA
+constexpr size_t kLineSmem = 200 << 10;
+
+struct LineGeom {
+  LineArgs a;
+  int n, nlines;         // cells per line, lines
+  int log_lines, runs;   // lines per CTA (a power of two), runs per line
+  int run;               // cells per run
+  int pieces, piece;     // pieces per line, cells per piece
+  int lp;                // shared-memory pitch of a line
+  int pitch;
+  long long plane;
+};
+
+// The geometry of a direction's launch, its CTAs and threads per CTA.
+inline void set_line_geom(LineGeom* P, const LineSpread& sp, int nx, int nz, bool isx, int* ctas, int* threads) {
+  const Geom g = make_geom(nx, nz);
+  P->n = isx ? nx : nz;
+  P->nlines = isx ? nz : nx;
+  P->pitch = g.pitch;
+  P->plane = g.plane;
+  P->log_lines = sp.log_lines;
+  P->pieces = sp.pieces;
+  P->piece = sp.piece;
+  P->run = sp.run;
+  P->runs = sp.runs;
+  P->lp = sp.lp;
+  *threads = 32 * (sp.runs << sp.log_lines);
+  *ctas = ((P->nlines + (1 << sp.log_lines) - 1) >> sp.log_lines) * sp.pieces;
+}
+
+#define MW_LG(p, off) MW_AT((p), (off), 4 * P.plane)
+
+// The halo cells that cell c of a line is the source of, in a global array.
+template <int DIR>
+__device__ __forceinline__ void halo_out(const LineGeom& P, double* g, int line, int c, const double v[4],
+                                         const double* hr) {
+  const int n = P.n;
+  if (DIR == MW_DIR_X) {
+    const long long row = (long long)(line + kHs) * P.pitch;
+    for (int q = 0; q < 4; ++q) {
+      if (c < kHs) MW_LG(g, q * P.plane + row + n + kHs + c) = v[q];
+      if (c >= n - kHs) MW_LG(g, q * P.plane + row + c - n + kHs) = v[q];
+    }
+  } else {
+    for (int q = 0; q < 4; ++q)
+      for (int h = 0; h < 4; ++h)
+        if (c == (h < 2 ? 0 : n - 1))
+          MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + line) =
+              q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
+  }
+}
+
+// Cells [ca, cb) of the CTA's lines, between a global array and shared memory
+// (x: periodic).  x: a warp per line and variable; z: consecutive threads take
+// the CTA's columns of a row.
+template <int DIR, typename Fn>
+__device__ __forceinline__ void each_cell(const LineGeom& P, int l0, int nl, int ca, int cb, Fn fn) {
+  if (DIR == MW_DIR_X) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int ql = w; ql < 4 * nl; ql += nw) {
+      const int q = ql / nl, l = ql - q * nl;
+      const long long o = q * P.plane + (long long)(l0 + l + kHs) * P.pitch + kHs;
+      for (int c = ca + lane; c < cb; c += 32) fn(q, l, c, o + (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c)));
+    }
+  } else {
+    for (int q = 0; q < 4; ++q)
+      for (int i = threadIdx.x; i < ((cb - ca) << P.log_lines); i += blockDim.x) {
+        const int l = i & ((1 << P.log_lines) - 1), c = ca + (i >> P.log_lines);
+        if (l < nl) fn(q, l, c, q * P.plane + (long long)(c + kHs) * P.pitch + l0 + l + kHs);
+      }
+  }
+}
+
+// The four x-halo columns of the wall halo rows, from the halo columns' own first and last rows (8 threads).
+__device__ __forceinline__ void halo_corners(const LineGeom& P, const double* hr) {
+  const LineArgs& a = P.a;
+  const int n = P.n;
+  double* g = threadIdx.x < 4 ? a.halo_in : a.halo_tmp;
+  const int col = (threadIdx.x & 2) ? P.nlines + (threadIdx.x & 3) : (threadIdx.x & 1);
+  if (g)
+    for (int e = 0; e < 2; ++e) {
+      double v[4];
+      for (int q = 0; q < 4; ++q) v[q] = MW_LG(g, q * P.plane + (long long)(e ? n + kHs - 1 : kHs) * P.pitch + col);
+      for (int q = 0; q < 4; ++q)
+        for (int h = 2 * e; h < 2 * e + 2; ++h)
+          MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + col) =
+              q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
+    }
+}
+
+}  // namespace
+}  // namespace mw

@@ -216,6 +216,32 @@ __device__ __forceinline__ RowS row_consts(double hy_r, double hy_rt, double P) 
   return r;
 }
 
+// out = init + c12 (F(i) - F(i+1)): one FP64 add (merging the pair, scaled by
+// 2^-896) and one FP64 FMA per value; c12s = c12 * 2^896 undoes the scale.
+__device__ __forceinline__ double update(double init, dw dF, double c12s) { return fma(c12s, to_f64_scaled(dF), init); }
+
+// The same of the four variables.  One test per cell for non-finite increments:
+// h - h is 0 for finite h and NaN otherwise; only then are the four values
+// merged with the per-value check.
+__device__ __forceinline__ void update_f64(const double iv[4], const dw2 dF[2], double c12s, double v[4]) {
+  const dw d[4] = {lo_of(dF[0]), hi_of(dF[0]), lo_of(dF[1]), hi_of(dF[1])};
+  const float2 z = f2add(f2sub(dF[0].h, dF[0].h), f2sub(dF[1].h, dF[1].h));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = fma(c12s, to_f64_scaled_finite(d[q]), iv[q]);
+  if (!(z.x + z.y == 0.0f)) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = update(iv[q], d[q], c12s);
+  }
+}
+
+// The same in pair arithmetic, init and result as pairs.
+__device__ __forceinline__ void update_pairs(const dw2 ip[2], const dw2 dF[2], dw c, dw2 r[2]) {
+  const dw2 cv = splat(c);
+  const float2 cn = f2splat(-c.h);
+#pragma unroll
+  for (int pr = 0; pr < 2; ++pr) r[pr] = add2(ip[pr], mul2n(dF[pr], cv, cn));
+}
+
 __device__ __forceinline__ int wrap_x(int j, int nx) { return j < 0 ? j + nx : (j >= nx ? j - nx : j); }
 
 __device__ __forceinline__ void pack4(const double v[4], dw2 out[2]) {

@@ -91,10 +91,6 @@ __device__ __forceinline__ void write_z_halo_column(const SplitArgs& a, int col,
   }
 }
 
-// out = init + c12 (F(i) - F(i+1)): one FP64 add (merging the pair, scaled by
-// 2^-896) and one FP64 FMA per value; c12s = c12 * 2^896 undoes the scale.
-__device__ __forceinline__ double update(double init, dw dF, double c12s) { return fma(c12s, to_f64_scaled(dF), init); }
-
 // ---------------------------------------------------------------------------
 // Tiles.  Both the single-grid kernels and the persistent ensemble kernels
 // call these; every thread of the CTA must call them (they contain barriers).
@@ -105,35 +101,24 @@ struct SmemZ {
 
 // out = init + c12 (F(i) - F(i+1)) for the four variables (paired differences,
 // then per value one FP64 add merging the pair and one FP64 FMA).
-// One test per cell for non-finite increments: h - h is 0 for finite h and
-// NaN otherwise; only then are the four values merged with the per-value check.
 // kToPair: out = init + c12 (F(i) - F(i+1)) in pair arithmetic from the
 // init pairs ip (the forcing's own pairs), stored as (h, l) floats.
 template <int FMT>
 __device__ __forceinline__ void store_update(const SplitArgs& a, sidx o, const double iv[4], const dw2 ip[2],
                                              dw2 dF[2]) {
   if (FMT == kToPair) {
-    const dw c = ld(a.c12);
-    const dw2 cv = splat(c);
-    const float2 cn = f2splat(-c.h);
     float2* out = reinterpret_cast<float2*>(a.out);
+    dw2 r[2];
+    update_pairs(ip, dF, ld(a.c12), r);
 #pragma unroll
     for (int pr = 0; pr < 2; ++pr) {
-      const dw2 r = add2(ip[pr], mul2n(dF[pr], cv, cn));
-      MW_AT(out, (2 * pr) * a.plane + o, 4 * (long long)a.plane) = make_float2(r.h.x, r.l.x);
-      MW_AT(out, (2 * pr + 1) * a.plane + o, 4 * (long long)a.plane) = make_float2(r.h.y, r.l.y);
+      MW_AT(out, (2 * pr) * a.plane + o, 4 * (long long)a.plane) = make_float2(r[pr].h.x, r[pr].l.x);
+      MW_AT(out, (2 * pr + 1) * a.plane + o, 4 * (long long)a.plane) = make_float2(r[pr].h.y, r[pr].l.y);
     }
     return;
   }
-  const dw d[4] = {lo_of(dF[0]), hi_of(dF[0]), lo_of(dF[1]), hi_of(dF[1])};
-  const float2 z = f2add(f2sub(dF[0].h, dF[0].h), f2sub(dF[1].h, dF[1].h));
   double v[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = fma(a.c12s, to_f64_scaled_finite(d[q]), iv[q]);
-  if (!(z.x + z.y == 0.0f)) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = update(iv[q], d[q], a.c12s);
-  }
+  update_f64(iv, dF, a.c12s, v);
 #pragma unroll
   for (int q = 0; q < 4; ++q) MW_AT(a.out, q * a.plane + o, 4 * (long long)a.plane) = v[q];
 }
