@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     }
   }
   overlap_wait();
+  if (gridDim.x <= kLineFewCtas) overlap_next();
   if (DIR == MW_DIR_Z) __syncthreads();  // hr
   {
     const int ca = whole ? 0 : (DIR == MW_DIR_X ? p0 - 6 : max(p0 - 6, 0));
@@ -200,10 +201,7 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       }
     }
     __syncthreads();
-    // The next kernel may come in now: its CTAs take what is free beside this
-    // one's, and earlier that is unevenly much (256x128: 60 us a step with this at
-    // the head of the kernel, 41 here, 47 without overlap).
-    if (s == 2) overlap_next();
+    if (s == 2) overlap_next();  // at the latest (kLineFewCtas)
     double* g = s == 0 ? a.s1 : (s == 1 ? a.s2 : a.out);
     if (g)
       each_cell<DIR>(P, l0, nl, p0, p1, [&](int q, int ll, int c, long long o) {

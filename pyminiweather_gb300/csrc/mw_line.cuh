@@ -11,6 +11,13 @@ namespace {
 
 constexpr int kLineMax = 8;            // most lines per CTA
 constexpr size_t kLineSmem = 200 << 10;
+// A launch of at most this many CTAs, about one per SM, lets the next one in at
+// its head, whose row constants then cost no time (us a step, eight in a call:
+// IEEE form 100x50 24.2 -> 22.8, 150x75 26.0 -> 23.6, double-FP32 14.3 -> 13.3); a
+// larger one only after its last stage: the next one's CTAs take what is free
+// beside its own, and earlier that is unevenly much (256x128, IEEE: 60 us a step
+// with the trigger at the head, 41 here, 47 without overlap).
+constexpr unsigned kLineFewCtas = 152;
 
 struct LineGeom {
   LineArgs a;

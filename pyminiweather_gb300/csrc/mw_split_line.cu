@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32, 1) k_line_split(const __grid
     __syncthreads();  // hr
   }
   overlap_wait();
+  if (gridDim.x <= kLineFewCtas) overlap_next();
   {
     const int ca = whole ? 0 : (DIR == MW_DIR_X ? p0 - 6 : max(p0 - 6, 0));
     const int cb = whole ? n : (DIR == MW_DIR_X ? p1 + 6 : min(p1 + 6, n));
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32, 1) k_line_split(const __grid
       }
     }
     __syncthreads();
-    if (s == 2) overlap_next();  // as in mw_fp64_line.cu
+    if (s == 2) overlap_next();  // at the latest (kLineFewCtas)
     double* g = s == 0 ? a.s1 : (s == 1 ? a.s2 : a.out);
     if (g) {
       each_cell4<DIR>(P, l0, nl, p0, p1, [&](int ll, int c, long long o) {
