@@ -64,6 +64,7 @@ int oob_count_ieee_stage(unsigned long long* out, bool reset);
 int oob_count_ieee_line(unsigned long long* out, bool reset);
 int oob_count_split_line(unsigned long long* out, bool reset);
 int oob_count_f32_dir(unsigned long long* out, bool reset);
+int oob_count_f32_line(unsigned long long* out, bool reset);
 int oob_count_dirstage(unsigned long long* out, bool reset);
 int oob_count_aux(unsigned long long* out, bool reset);
 int oob_count_adjoint(unsigned long long* out, bool reset);
@@ -83,6 +84,7 @@ extern "C" int mw_debug_oob_count(unsigned long long* count, int reset) {
       (st = mw::oob_count_ieee_stage(count, reset != 0)) || (st = mw::oob_count_ieee_line(count, reset != 0)) ||
       (st = mw::oob_count_split_line(count, reset != 0)) ||
       (st = mw::oob_count_dirstage(count, reset != 0)) || (st = mw::oob_count_f32_dir(count, reset != 0)) ||
+      (st = mw::oob_count_f32_line(count, reset != 0)) ||
       (st = mw::oob_count_aux(count, reset != 0)) || (st = mw::oob_count_adjoint(count, reset != 0)) ||
       (st = mw::oob_count_capi(count, reset != 0)))
     return st;

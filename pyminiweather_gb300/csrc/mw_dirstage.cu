@@ -6,9 +6,11 @@
 // update.  Halo cells are never read: the periodic (x) and wall (z) rules of
 // ics/bcs.py are applied to the indices / values as they are loaded.
 //
-// Native FP64 and FP32 forms (the IEEE-FP64 form with the fewest operations
-// is in mw_fp64_stage.cu, the split form in mw_split_stage.cu); this file
-// also holds the stage and step entry points of every form.
+// Native FP64 form and single FP32 stages (the IEEE-FP64 form with the fewest
+// operations is in mw_fp64_stage.cu and mw_fp64_line.cu, the split form in
+// mw_split_stage.cu and mw_split_line.cu, the FP32 form's steps in
+// mw_f32_dir.cu); this file also holds the stage and step entry points of every
+// form.
 // x pass (plain loads): a CTA walks a run of 255-cell chunks of one row.
 // Thread t evaluates the flux at interface x0+t into shared memory; after one
 // barrier thread t updates cell x0+t from interfaces t and t+1.  Interface
@@ -239,8 +241,7 @@ __device__ __forceinline__ void write_z_halo_column(const StageArgs<T>& a, int c
 }
 
 // ---------------------------------------------------------------------------
-// Tiles, called by the single-grid kernels and the persistent ensemble
-// kernels alike; every thread of the CTA must call them (they contain barriers).
+// Tiles; every thread of the CTA must call them (they contain barriers).
 template <typename T>
 struct SmemXT {
   T sF[4][kXThreads];
@@ -1170,6 +1171,8 @@ extern "C" int mw_step_f32(int nx, int nz, double dx, double dz, double dt_full,
   cudaStream_t s = (cudaStream_t)stream;
   const bool halo = flags & MW_FLAG_WRITE_HALO;
   const bool fits = f32_dir_fits(nx);
+  LinePlan plan;
+  if ((st = line_f32_plan(nx, nz, &plan))) return st;
   if (!fits)
     st = run_steps<float>(dt, state, state_tmp, scratch, nsteps, reverse,
                           [&](const float* init, float* forcing, float* out, double dts, int dir, int) {
@@ -1177,13 +1180,15 @@ extern "C" int mw_step_f32(int nx, int nz, double dx, double dz, double dt_full,
                                                                  src_w, init, forcing, out, dts, dir, flags, s);
                           });
   for (int n = 0; fits && n < nsteps; ++n) {
-    for (int d = 0; d < 2; ++d) {  // state -> scratch -> state
-      const F32DirArgs a{hyc, hytc, hyi, hyti, hypi, src_w, d ? scratch : state, d ? state : scratch,
+    for (int d = 0; d < 2; ++d) {  // state -> scratch -> state; line kernels of whole lines in place
+      const bool cut = !plan.fits || plan.cut;
+      const int dir = (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z;
+      const F32DirArgs a{hyc, hytc, hyi, hyti, hypi, src_w, cut && d ? scratch : state, cut && !d ? scratch : state,
                          n + 1 == nsteps && d == 1 ? state_tmp : nullptr, halo ? state : nullptr,
                          halo ? state_tmp : nullptr};
-      if ((st = launch_dir_f32(nx, nz, dx, dz, dt_full, dt, a, (*reverse != 0) == (d == 0) ? MW_DIR_X : MW_DIR_Z,
-                               n + d > 0, s)))
-        return st;
+      st = plan.fits ? launch_line_f32(plan, nx, nz, dx, dz, dt_full, dt, a, dir, n + d > 0, s)
+                     : launch_dir_f32(nx, nz, dx, dz, dt_full, dt, a, dir, n + d > 0, s);
+      if (st) return st;
     }
     *reverse = *reverse ? 0 : 1;
   }

@@ -13,7 +13,7 @@ struct F32DirArgs {
   const double* hypi;
   const double* srcw;  // optional forcing of w
   const float* in;     // the direction's initial state
-  float* out;          // its result; must not overlap `in`
+  float* out;          // its result; must not overlap `in` (launch_dir_f32)
   float* s2;           // second stage (optional)
   float* halo_in;      // optional: arrays that get the direction's halo of the initial state
   float* halo_tmp;     // and of the second stage
@@ -44,5 +44,12 @@ inline bool f32_dir_fits(int nx) { return 25LL * 4 * (nx + 4LL) < (1LL << 32); }
 // (mw_fp64_line.cuh).
 int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double dt, const F32DirArgs& d, int direction,
                    bool overlap, cudaStream_t stream);
+
+// The same by line kernels (mw_f32_line.cu), for grids whose lines fit a CTA;
+// `out` may be `in` where the plan does not cut the lines.
+struct LinePlan;
+int line_f32_plan(int nx, int nz, LinePlan* plan);
+int launch_line_f32(const LinePlan& plan, int nx, int nz, double dx, double dz, double dt_full, double dt,
+                    const F32DirArgs& d, int direction, bool overlap, cudaStream_t stream);
 
 }  // namespace mw

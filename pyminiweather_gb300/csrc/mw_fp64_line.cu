@@ -251,7 +251,9 @@ constexpr int kMaxPieces = 16;
 // 100x50 to 1250x799, both directions in turn, the rule takes one within 2 % of
 // the fastest but for 300x150, x (4 %): 512x256, x: whole rows in 17 warps 46.7 us
 // a step, five pieces of four warps 43.1; 880x620, z: twelve pieces of two columns
-// in four warps 122 us, of one column in two warps 129, three in 14 warps 150.
+// in four warps 122 us, of one column in two warps 129, three in 14 warps 150.  The
+// FP32 form takes the same rule (within 3 % of the fastest spread from 100x50 to
+// 1000x1000).
 LineSpread spread_lines(const LineKind& kind, int n, int nlines, bool isx, int sms) {
   LineSpread best;
   double least = 0.0;

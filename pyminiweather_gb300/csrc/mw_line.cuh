@@ -19,8 +19,7 @@ constexpr size_t kLineSmem = 200 << 10;
 // with the trigger at the head, 41 here, 47 without overlap).
 constexpr unsigned kLineFewCtas = 152;
 
-struct LineGeom {
-  LineArgs a;
+struct LineShape {
   int n, nlines;         // cells per line, lines
   int log_lines, runs;   // lines per CTA (a power of two), runs per line
   int run;               // cells per run
@@ -29,9 +28,12 @@ struct LineGeom {
   int pitch;
   long long plane;
 };
+struct LineGeom : LineShape {
+  LineArgs a;
+};
 
-// The geometry of a direction's launch, its CTAs and threads per CTA.
-inline void set_line_geom(LineGeom* P, const LineSpread& sp, int nx, int nz, bool isx, int* ctas, int* threads) {
+// The shape of a direction's launch, its CTAs and threads per CTA.
+inline void set_line_geom(LineShape* P, const LineSpread& sp, int nx, int nz, bool isx, int* ctas, int* threads) {
   const Geom g = make_geom(nx, nz);
   P->n = isx ? nx : nz;
   P->nlines = isx ? nz : nx;
@@ -87,6 +89,26 @@ __device__ __forceinline__ void each_cell(const LineGeom& P, int l0, int nl, int
         const int l = i & ((1 << P.log_lines) - 1), c = ca + (i >> P.log_lines);
         if (l < nl) fn(q, l, c, q * P.plane + (long long)(c + kHs) * P.pitch + l0 + l + kHs);
       }
+  }
+}
+
+// Cells [ca, cb) of the CTA's lines, each by one thread: fn(line, cell, offset in a plane of a global array).
+template <int DIR, typename Fn>
+__device__ __forceinline__ void each_cell4(const LineShape& P, int l0, int nl, int ca, int cb, Fn fn) {
+  const int len = cb - ca;
+  for (int i = threadIdx.x; i < (DIR == MW_DIR_X ? len * nl : len << P.log_lines); i += blockDim.x) {
+    int l, c;
+    if (DIR == MW_DIR_X) {
+      l = i / len;
+      c = ca + i - l * len;
+    } else {
+      l = i & ((1 << P.log_lines) - 1);
+      c = ca + (i >> P.log_lines);
+      if (l >= nl) continue;
+    }
+    const int cw = DIR == MW_DIR_Z ? c : (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c));
+    fn(l, c, DIR == MW_DIR_X ? (long long)(l0 + l + kHs) * P.pitch + kHs + cw
+                             : (long long)(cw + kHs) * P.pitch + l0 + l + kHs);
   }
 }
 

@@ -61,26 +61,6 @@ __device__ __forceinline__ void put_pairs(dw2* line, size_t pl, int c, int n, bo
   }
 }
 
-// Cells [ca, cb) of the CTA's lines, each by one thread: fn(line, cell, offset in a plane of a global array).
-template <int DIR, typename Fn>
-__device__ __forceinline__ void each_cell4(const LineGeom& P, int l0, int nl, int ca, int cb, Fn fn) {
-  const int len = cb - ca;
-  for (int i = threadIdx.x; i < (DIR == MW_DIR_X ? len * nl : len << P.log_lines); i += blockDim.x) {
-    int l, c;
-    if (DIR == MW_DIR_X) {
-      l = i / len;
-      c = ca + i - l * len;
-    } else {
-      l = i & ((1 << P.log_lines) - 1);
-      c = ca + (i >> P.log_lines);
-      if (l >= nl) continue;
-    }
-    const int cw = DIR == MW_DIR_Z ? c : (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c));
-    fn(l, c, DIR == MW_DIR_X ? (long long)(l0 + l + kHs) * P.pitch + kHs + cw
-                             : (long long)(cw + kHs) * P.pitch + l0 + l + kHs);
-  }
-}
-
 template <int DIR>
 __global__ void __launch_bounds__(kSplitWarps * 32, 1) k_line_split(const __grid_constant__ SplitLineParams P) {
   extern __shared__ __align__(16) unsigned char smem_line[];
