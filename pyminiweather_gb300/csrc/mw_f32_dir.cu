@@ -71,6 +71,10 @@ __device__ __forceinline__ void copy4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copies_wait() {
@@ -124,13 +128,17 @@ struct SmemZ {
 
 // Rows [z0, z1) of the columns [cb NC, cb NC + NC); every thread of the CTA
 // calls it (one barrier after the row table is formed).  tab: z1 - z0 + 17 rows
-// of shared memory.
+// of shared memory.  SRC: the forcing of w comes through a ring of its own (srcs,
+// kRing rows of NC) beside the state's: read where the three stages add it, it
+// stood in each one's way (2501x1251: 175 us a step against 79 without forcing,
+// 113 here).
 // TMP: the second stage is stored too.  Without it the march is unrolled by four
 // (8192x2048: 145 against 169 us, the streams' rows keep their registers); with
 // it the extra stores bound the pass and the compact loop does better (190
 // against 198 us).
 template <int NC, bool SRC, bool TMP>
-__device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, SmemZ<NC>& sm, Row* tab) {
+__device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, SmemZ<NC>& sm, Row* tab,
+                                        double* srcs = nullptr) {
   const int a0 = max(z0 - 6, 0), last = z1 - 1 + kLag;  // first row in; last iteration
   const int t = threadIdx.x, nz = a.nz;
   for (int i = t; i <= last - a0 + 5; i += NC) {  // interface a0 - 6 + i, clamped where nothing uses it
@@ -186,6 +194,7 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
     if (r < nz && r <= z1 + 5) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) copy4(&sm.ring[r & (kRing - 1)][q][t], elem(a.in, q, off_in));
+      if (SRC) copy8(&srcs[(r & (kRing - 1)) * NC + t], &MW_AT(a.srcw, (long long)r * a.nx + cc, (long long)a.nx * nz));
     }
     off_in += pitch4;
     copies_commit();
@@ -218,8 +227,7 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
       commit<W>(st[s], p, idx, sm.hr);
       if (SRC) {
         const int k = idx - 2;
-        if (k >= 0 && k < nz)
-          p.o.b.x = fmaf(a.k.dt[s], split::d2f(MW_AT(a.srcw, (long long)k * a.nx + cc, (long long)a.nx * nz)), p.o.b.x);
+        if (k >= a0 && k < nz) p.o.b.x = fmaf(a.k.dt[s], split::d2f(srcs[(k & (kRing - 1)) * NC + t]), p.o.b.x);
       }
       return p.o;
     };
@@ -254,14 +262,21 @@ __global__ void __launch_bounds__(kZCols, 4) k_dir_z_f32(const __grid_constant__
   extern __shared__ __align__(16) unsigned char smem_f32[];
   SmemZ<kZCols>& sm = *reinterpret_cast<SmemZ<kZCols>*>(smem_f32);
   const int z0 = (tile0 + blockIdx.y) * tile;
-  z_march<kZCols, SRC, TMP>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, reinterpret_cast<Row*>(&sm + 1));
+  Row* tab = reinterpret_cast<Row*>(&sm + 1);
+  z_march<kZCols, SRC, TMP>(a, blockIdx.x, z0, min(z0 + tile, a.nz), sm, tab, reinterpret_cast<double*>(tab + tile + 17));
 }
 
 // ---- x ---------------------------------------------------------------------
-template <int V>
+template <int V, bool SRC = false>
 struct XBuf {
-  float v[4][32 * V + 4];  // cells c0 - 6 + j of a run
+  float v[4][32 * V + 4];               // cells c0 - 6 + j of a run
+  double src[SRC ? 32 * V + 2 : 1];     // their forcing of w
 };
+template <int V>
+struct XBuf<V, false> {
+  float v[4][32 * V + 4];
+};
+static_assert(sizeof(XBuf<4, true>) % 16 == 0 && sizeof(XBuf<8, true>) % 16 == 0, "buffers are read in float4");
 constexpr int x_run_max(int V) { return 32 * V - 12; }
 
 __device__ __forceinline__ Vars shfl_up(const Vars& v) {
@@ -276,8 +291,8 @@ __device__ __forceinline__ Vars shfl_down(const Vars& v) {
 }
 
 // Copies of the cells c0 - 6 .. c0 + len + 5 of row k (periodic) into b, one group.
-template <int V>
-__device__ __forceinline__ void x_load(const Args& a, int k, int c0, int len, XBuf<V>& b) {
+template <int V, bool SRC = false>
+__device__ __forceinline__ void x_load(const Args& a, int k, int c0, int len, XBuf<V, SRC>& b) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)(k + kHs) * a.pitch + kHs;
   if (c0 >= 6 && c0 + len + 6 <= a.nx) {
@@ -287,6 +302,8 @@ __device__ __forceinline__ void x_load(const Args& a, int k, int c0, int len, XB
       if (j < len + 12)
 #pragma unroll
         for (int q = 0; q < 4; ++q) copy4(&b.v[q][j], &MW_G(a.in, q * a.plane + row + (c0 - 6) + j));
+      if constexpr (SRC)
+        if (j < len + 12) copy8(&b.src[j], &MW_AT(a.srcw, (long long)k * a.nx + (c0 - 6) + j, (long long)a.nx * a.nz));
     }
   } else {
     for (int j = lane; j < len + 12; j += 32) {
@@ -299,6 +316,7 @@ __device__ __forceinline__ void x_load(const Args& a, int k, int c0, int len, XB
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) copy4(&b.v[q][j], &MW_G(a.in, q * a.plane + row + c));
+      if constexpr (SRC) copy8(&b.src[j], &MW_AT(a.srcw, (long long)k * a.nx + c, (long long)a.nx * a.nz));
     }
   }
   copies_commit();
@@ -334,7 +352,8 @@ __device__ __forceinline__ void x_stage(Vars (&v)[V], const Vars (&S)[V], const 
 // The run of `len` cells from c0 of row k, staged in b (which it reuses for its
 // results); every lane of the warp calls it.
 template <int V, bool SRC>
-__device__ __forceinline__ void x_run(const Args& a, int k, int c0, int len, const Row& row, XBuf<V>& b) {
+__device__ __forceinline__ void x_run(const Args& a, int k, int c0, int len, const Row& row,
+                                      XBuf<V, SRC>& b) {
   const int lane = threadIdx.x & 31;
   const long long go = (long long)(k + kHs) * a.pitch + kHs + c0;
   Vars S[V], v[V];
@@ -351,15 +370,9 @@ __device__ __forceinline__ void x_run(const Args& a, int k, int c0, int len, con
 #pragma unroll
   for (int j = 0; j < V; ++j) v[j] = S[j];
   float src[V];
-  if (SRC) {
+  if constexpr (SRC) {  // the cells beyond the run and its neighbours' are not used
 #pragma unroll
-    for (int j = 0; j < V; ++j) {
-      const int c = c0 - 6 + V * lane + j;
-      // cells beyond the row ends belong to the periodic image
-      int cw = V * lane + j < len + 12 ? c % a.nx : 0;
-      if (cw < 0) cw += a.nx;
-      src[j] = split::d2f(MW_AT(a.srcw, (long long)k * a.nx + cw, (long long)a.nx * a.nz));
-    }
+    for (int j = 0; j < V; ++j) src[j] = split::d2f(b.src[V * lane + j]);
   }
   auto stage_out = [&](float* g, bool halo) {  // cells c0 .. c0 + len - 1 of v through b to g
     __syncwarp();
@@ -426,7 +439,7 @@ template <int V, bool SRC>
 __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_constant__ Args a, int nrun, int len,
                                                               long long total) {
   extern __shared__ __align__(16) unsigned char smem_f32[];
-  XBuf<V>* buf = reinterpret_cast<XBuf<V>*>(smem_f32) + 2 * (threadIdx.x >> 5);
+  XBuf<V, SRC>* buf = reinterpret_cast<XBuf<V, SRC>*>(smem_f32) + 2 * (threadIdx.x >> 5);
   const long long w = (long long)blockIdx.x * kXWarps + (threadIdx.x >> 5), nw = (long long)gridDim.x * kXWarps;
   const long long g0 = total * w / nw, g1 = total * (w + 1) / nw;
   int k = (int)(g0 / nrun), rn = (int)(g0 - (long long)k * nrun);
@@ -435,7 +448,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
   overlap_wait();
   if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   if (g0 >= g1) return;
-  x_load<V>(a, k, rn * len, min(len, a.nx - rn * len), buf[0]);
+  x_load<V, SRC>(a, k, rn * len, min(len, a.nx - rn * len), buf[0]);
   int cur = 0;
   for (long long g = g0; g < g1; ++g) {
     const int kc = k, c0 = rn * len;
@@ -445,7 +458,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
     }
     __syncwarp();  // the other buffer's results are read
     if (g + 1 < g1) {
-      x_load<V>(a, k, rn * len, min(len, a.nx - rn * len), buf[cur ^ 1]);
+      x_load<V, SRC>(a, k, rn * len, min(len, a.nx - rn * len), buf[cur ^ 1]);
       copies_wait<1>();
     } else {
       copies_wait<0>();
@@ -542,7 +555,10 @@ __global__ void __launch_bounds__(kEnsZCols, 8) k_ens_z_f32(EnsStageT<float> es)
   ens_finish(es.cursor);
 }
 
-size_t z_smem(int nc, int tile) { return (nc == kZCols ? sizeof(SmemZ<kZCols>) : sizeof(SmemZ<kEnsZCols>)) + sizeof(Row) * (tile + 17); }
+size_t z_smem(int nc, int tile, bool src = false) {
+  return (nc == kZCols ? sizeof(SmemZ<kZCols>) : sizeof(SmemZ<kEnsZCols>)) + sizeof(Row) * (tile + 17) +
+         (src ? sizeof(double) * kRing * nc : 0);
+}
 
 // The kernels' shared-memory limits, raised once per device; the device's SMs
 // and resident CTAs per SM of the two passes.
@@ -571,12 +587,13 @@ int device(Device** out) {
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<false, false>, zs);
   if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<false, true>, zs);
-  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, false>, zs);
-  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, true>, zs);
+  const size_t zs_src = z_smem(kZCols, kZTileMax, true);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, false>, zs_src);
+  if (e == cudaSuccess) e = raise_smem(k_dir_z_f32<true, true>, zs_src);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<4, false>, xs4);
-  if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<4, true>, xs4);
+  if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<4, true>, sizeof(XBuf<4, true>) * 2 * kXWarps);
   if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<8, false>, xs8);
-  if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<8, true>, xs8);
+  if (e == cudaSuccess) e = raise_smem(k_dir_x_f32<8, true>, sizeof(XBuf<8, true>) * 2 * kXWarps);
   if (e == cudaSuccess) e = raise_smem(k_ens_x_f32, xs8);
   if (e == cudaSuccess) e = raise_smem(k_ens_z_f32<false>, z_smem(kEnsZCols, kEnsZTileMax));
   if (e == cudaSuccess) e = raise_smem(k_ens_z_f32<true>, z_smem(kEnsZCols, kEnsZTileMax));
@@ -615,7 +632,8 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
     const long long total = (long long)nrun * nz;
     const int resident = dev->x_ctas[v == 8] * sms;
     const unsigned grid = (unsigned)std::min<long long>(resident, (total + kXWarps - 1) / kXWarps);
-    const size_t smem = (v == 8 ? sizeof(XBuf<8>) : sizeof(XBuf<4>)) * 2 * kXWarps;
+    const size_t smem = (a.srcw ? (v == 8 ? sizeof(XBuf<8, true>) : sizeof(XBuf<4, true>))
+                                : (v == 8 ? sizeof(XBuf<8>) : sizeof(XBuf<4>))) * 2 * kXWarps;
     auto kern = v == 8 ? (a.srcw ? k_dir_x_f32<8, true> : k_dir_x_f32<8, false>)
                        : (a.srcw ? k_dir_x_f32<4, true> : k_dir_x_f32<4, false>);
     return launch_overlapping(kern, dim3(grid), 32 * kXWarps, smem, stream, overlap, "FP32 x direction", a, nrun, lenc, total);
@@ -642,7 +660,7 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
     const dim3 grid((unsigned)ncb, (unsigned)std::min(ntiles - t0, 65535));
     auto kern = a.srcw ? (a.s2 ? k_dir_z_f32<true, true> : k_dir_z_f32<true, false>)
                        : (a.s2 ? k_dir_z_f32<false, true> : k_dir_z_f32<false, false>);
-    st = launch_overlapping(kern, grid, kZCols, z_smem(kZCols, tile), stream,
+    st = launch_overlapping(kern, grid, kZCols, z_smem(kZCols, tile, a.srcw != nullptr), stream,
                 overlap && t0 == 0, "FP32 z direction", a, tile, t0);
     if (st) return st;
   }
