@@ -3,8 +3,9 @@
 
 Workload: the collision case on an 8192 x 4096 grid (two cos^2 bubbles of
 +-20 K, 20 km x 10 km, cfl 1.5, max_speed 450).  One step is one full time
-step: two directions x three RK stages = six fused direction-stage kernel
-launches over the whole grid.  The state (1.07 GB per FP64 array) is far
+step: two directions x three RK stages, in the FP64 forms one fused kernel
+launch per direction-stage over the whole grid (six a step), in the FP32 form
+one per direction (two a step).  The state (1.07 GB per FP64 array) is far
 larger than the 129 MB L2, so no flush is needed between steps.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb300|reference]
@@ -13,7 +14,8 @@ The headline is the IEEE-FP64 form (f64_mode "fp64": every floating-point
 operation an IEEE FP64 add, multiply or FMA), timed over K calls of the public
 step (evolve -> mw_step_f64).  The per-kernel figures of the roofline come from
 a second pass that issues the step's six launches one by one through
-mw_dirstage_f64 (the same kernels on the same arrays) with an event after each.
+mw_dirstage_f64 (the same kernels on the same arrays) with an event after each;
+the FP32 form's two have no entry point of their own and are timed as a step.
 The other forms are reported on the same line: "fp64_dw" (the split form:
 FP64 storage, double-FP32 arithmetic of ~47 significant bits -- not IEEE
 FP64), "fp64_native" (IEEE FP64 with the reference's formulas as written),
@@ -50,6 +52,9 @@ UNIT = "cell-steps/s"
 # reads 4 (init is the forcing) and writes 4; stages 2 and 3 read 8, write 4.
 VALUES_PER_STAGE = (8, 12, 12)
 STATE_VALUES_PER_CELL_STEP = 2 * sum(VALUES_PER_STAGE)  # 64
+# The FP32 form's three stages of a direction share one launch: each direction
+# reads 4 values and writes 4, the step's last one stores state_tmp as well.
+F32_VALUES_PER_CELL_STEP = 2 * 8 + 4  # 20
 # FP64 operations the GB300 SM retires per clock (DFMA, DADD or DMUL; the
 # profiler's peak_sustained for sm__sass_thread_inst_executed_op_dfma_pred_on).
 FP64_OPS_PER_CLOCK_PER_SM = 2.0
@@ -65,7 +70,7 @@ KERNELS = {
     "fp64": {0: "k_stage_x_ieee_w", 1: "k_stage_z_ieee"},
     "split": {0: "k_stage_x_split", 1: "k_stage_z_split"},
     "native": {0: "k_stage_x<double,NATIVE64>", 1: "k_stage_z<double,NATIVE64>"},
-    "fp32": {0: "k_stage_x_f32_bulk", 1: "k_stage_z_f32_bulk"},
+    "fp32": {0: "k_dir_x_f32", 1: "k_dir_z_f32"},
 }
 
 
@@ -216,14 +221,13 @@ def make_params(nx, nz, ic, mode="fp64"):
 
 class StageRunner:
     """Issues a time step stage by stage through the C ABI -- the six launches
-    mw_step_* makes, with the same storage formats (the split form keeps its
+    mw_step_f64 makes of a grid too large for the line kernels, with the same storage formats (the split form keeps its
     first RK stage's result as pairs: MW_FLAG_PAIRS_OUT / _IN) -- recording a
     CUDA event on the launching stream after each launch."""
 
     def __init__(self, torch, native, p, f):
         self.torch, self.n, self.p, self.f = torch, native, p, f
         self.reverse = 0
-        self.fp64 = f.dtype == torch.float64
         self.mode = native.F64_MODES[p["f64_mode"]]
         self.hb = [native.ptr(a) for a in f.backgrounds()]
         self.stream = native.stream_handle(f.device)
@@ -232,13 +236,10 @@ class StageRunner:
     def stage(self, init, forcing, out, dts, d, k):
         n, p, f = self.n, self.p, self.f
         args = (f.nx, f.nz, p["dx"], p["dz"], p["dt"], *self.hb, None, init, forcing, out, dts, d)
-        if self.fp64:
-            flags = n.MW_FLAG_WRITE_HALO
-            if self.mode == n.MW_F64_SPLIT:
-                flags |= (n.MW_FLAG_PAIRS_OUT, n.MW_FLAG_PAIRS_IN, 0)[k]
-            n.call("mw_dirstage_f64", *args, self.mode, flags, self.stream)
-        else:
-            n.call("mw_dirstage_f32", *args, n.MW_FLAG_WRITE_HALO, self.stream)
+        flags = n.MW_FLAG_WRITE_HALO
+        if self.mode == n.MW_F64_SPLIT:
+            flags |= (n.MW_FLAG_PAIRS_OUT, n.MW_FLAG_PAIRS_IN, 0)[k]
+        n.call("mw_dirstage_f64", *args, self.mode, flags, self.stream)
 
     def step(self, events=None):
         dt = self.p["dt"]
@@ -333,6 +334,22 @@ def roofline(per, cells, bytes_per_value, peak, peak_kind, names, table, sm_mhz=
     return rl
 
 
+def roofline_f32(ms_per_step, cells, peak, peak_kind, table):
+    """HBM roofline of the FP32 step's two launches together, from the public
+    step's time (the x and the z launch each move 32 B a cell, the step's last
+    one 16 more)."""
+    algo = cells * 4 * F32_VALUES_PER_CELL_STEP
+    names = [KERNELS["fp32"][d] for d in (0, 1)]
+    out = {"bound": "hbm", "kernel": " + ".join(names), "achieved": round(algo / (ms_per_step * 1e-3) / 1e9, 1),
+           "peak": peak, "unit": "GB/s", "frac": round(algo / (ms_per_step * 1e-3) / 1e9 / peak, 4),
+           "peak_kind": peak_kind, "algorithmic_bytes_per_launch": algo / 2, "avg_launch_ms": round(ms_per_step / 2, 4),
+           "kernel_timing": "the public step (mw_step_f32, two launches), CUDA events on the launching stream"}
+    per_cell = [table.get(n, {}).get("dram_bytes_per_cell_launch") for n in names]
+    if all(b is not None for b in per_cell):
+        out["traffic"] = cells * sum(per_cell) / 2
+    return out
+
+
 def fp64_probe(torch, native, dev, repeats=5):
     """FP64 pipe throughput of this GPU, measured: mw_fp64_throughput (8
     independent FMA chains per thread, 4 CTAs of 256 threads per SM), the
@@ -416,15 +433,17 @@ def form_leg(torch, native, args, mode, dtype, peak, peak_kind, table, sm_mhz, s
     f = initialize_fields(p, dtype=dtype)
     init(f, p)
     ms = step_run(torch, p, f, steps, warmup)
-    init(f, p)
-    per = stage_pass(torch, native, p, f, steps, warmup)
     fp64 = dtype == torch.float64
-    names = KERNELS[mode if fp64 else "fp32"]
+    if fp64:
+        init(f, p)
+        per = stage_pass(torch, native, p, f, steps, warmup)
+        rl = roofline(per, cells, 8, peak, peak_kind, KERNELS[mode], table, sm_mhz)
+        rl["public_step_frac"] = round(cells * STATE_VALUES_PER_CELL_STEP * 8 / (ms / steps * 1e-3) / 1e9 / peak, 4)
+    else:
+        rl = roofline_f32(ms / steps, cells, peak, peak_kind, table)
     out = {"value": job_value(1, cells, steps, ms), "ms_per_step": ms / steps, "steps": steps,
            "dtype": DTYPES[mode] if fp64 else "f32 perturbation fields (FP64 backgrounds, IC and reductions)",
-           "roofline": roofline(per, cells, 8 if fp64 else 4, peak, peak_kind, names, table, sm_mhz)}
-    out["roofline"]["public_step_frac"] = round(
-        cells * STATE_VALUES_PER_CELL_STEP * (8 if fp64 else 4) / (ms / steps * 1e-3) / 1e9 / peak, 4)
+           "roofline": rl}
     del f
     torch.cuda.empty_cache()
     return out
@@ -452,12 +471,13 @@ def ensemble_run(torch, steps, warmup, dtype, mode, peak, ops_per_cell_stage=Non
     ms = e0.elapsed_time(e1)
     n = 2 * reps
     value = ens.cells() * n / (ms * 1e-3)
-    bpc = STATE_VALUES_PER_CELL_STEP * (8 if dtype == torch.float64 else 4)
+    # FP32: a replay's two steps are one call, whose last launch alone stores state_tmp
+    bpc = STATE_VALUES_PER_CELL_STEP * 8 if dtype == torch.float64 else (F32_VALUES_PER_CELL_STEP - 2) * 4
     out = {"value": value, "unit": UNIT, "ms_per_step": ms / n, "steps": n, "members": ens.n_members(),
            "cells": ens.cells(), "cuda_graph": True,
            "dtype": DTYPES[mode] if dtype == torch.float64 else "f32",
            # FP64 forms: + the row-constant table, once per replay of 2 steps
-           "launches_per_step": 6.5 if dtype == torch.float64 else 6,
+           "launches_per_step": 6.5 if dtype == torch.float64 else 2,
            "roofline": {"bound": "hbm", "bytes_per_cell_step": bpc, "achieved": round(value * bpc / 1e9, 1),
                         "peak": peak, "unit": "GB/s", "frac": round(value * bpc / 1e9 / peak, 4)},
            "tuning": {k: tuned[k] for k in ("z_tile", "grid_x", "grid_z")}}
@@ -663,7 +683,6 @@ def run_gb300(args):
     f32 = args.mode == "fp32"
     p = make_params(args.nx, args.nz, args.ic, "fp64" if f32 else args.mode)
     f = initialize_fields(p, dtype=torch.float32 if f32 else torch.float64)
-    vbytes = 4 if f32 else 8
     init(f, p)
     torch.cuda.synchronize()
     m0 = compute_stats(p, f)[0]
@@ -693,15 +712,18 @@ def run_gb300(args):
                     if link["h2d"] and link["d2h"] else None}
     # per-kernel durations: the step's six launches issued one by one through
     # the C ABI (same kernels, same arrays, same storage formats), an event after each
-    init(f, p)
-    per = stage_pass(torch, _native, p, f, args.steps, args.warmup, dist)
-    rl = roofline(per, cells, vbytes, peak, peak_kind, KERNELS[args.mode], table, clk.get("sm_mhz"))
-    rl["kernel_timing"] = "the public step's six launches issued one by one (mw_dirstage_f64), CUDA events on the " \
-                          "launching stream"
-    step_gbs = cells * STATE_VALUES_PER_CELL_STEP * vbytes / (ms / args.steps * 1e-3) / 1e9
+    bpc = F32_VALUES_PER_CELL_STEP * 4 if f32 else STATE_VALUES_PER_CELL_STEP * 8
+    if f32:
+        rl = roofline_f32(ms / args.steps, cells, peak, peak_kind, table)
+    else:
+        init(f, p)
+        per = stage_pass(torch, _native, p, f, args.steps, args.warmup, dist)
+        rl = roofline(per, cells, 8, peak, peak_kind, KERNELS[args.mode], table, clk.get("sm_mhz"))
+        rl["kernel_timing"] = "the public step's six launches issued one by one (mw_dirstage_f64), CUDA events on " \
+                              "the launching stream"
+    step_gbs = cells * bpc / (ms / args.steps * 1e-3) / 1e9
     rl["public_step"] = {"achieved": round(step_gbs, 1), "frac": round(step_gbs / peak, 4),
-                         "note": "%d algorithmic B per cell-step over the public step's time"
-                                 % (STATE_VALUES_PER_CELL_STEP * vbytes)}
+                         "note": "%d algorithmic B per cell-step over the public step's time" % bpc}
     probe = fp64_probe(torch, _native, dev) if rl.get("fp64_pipe") or not args.no_extras else None
     with_measured_fp64(rl, probe)
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -709,8 +731,8 @@ def run_gb300(args):
             "vs_baseline": None, "dtype": DTYPES[args.mode],
             "data": "synthetic (the reference's analytic collision initial condition)",
             "config": config_dict(args), "f64_mode": args.mode,
-            "roofline": rl, "clocks": clk, "gpu_launches": 6 * args.steps,
-            "mass_drift": (m1 - m0) / m0, "bytes_per_cell_step": STATE_VALUES_PER_CELL_STEP * vbytes}
+            "roofline": rl, "clocks": clk, "gpu_launches": (2 if f32 else 6) * args.steps,
+            "mass_drift": (m1 - m0) / m0, "bytes_per_cell_step": bpc}
     if probe:
         line["fp64_peak_measured"] = probe
     if rl.get("fp64_pipe"):

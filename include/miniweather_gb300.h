@@ -75,8 +75,8 @@ enum mw_f64_mode {
                               (needs init == forcing) */
 #define MW_FLAG_PAIRS_IN 16u  /* mw_dirstage_f64, split form: read `forcing` as such pairs.
                               With these two flags a caller can issue a split-form step
-                              stage by stage with the launches mw_step_f64 makes (to
-                              time them one by one); the pair arrays are not FP64 data */
+                              stage by stage with the launches mw_step_f64 makes on grids
+                              of more than 580000 cells (to time them one by one); the pair arrays are not FP64 data */
 
 /* Background profile of the initial condition. */
 enum mw_background {
@@ -120,8 +120,10 @@ int mw_dirstage_f32(int nx, int nz, double dx, double dz, double dt_full, const 
  * *reverse is a host int updated in place.  Per direction the three RK stages
  * run with dt/3, dt/2, dt:
  *   scratch = S + dt/3 L(S);  state_tmp = S + dt/2 L(scratch);  S = S + dt L(state_tmp)
- * so state_tmp ends holding what the reference's state_tmp holds.  scratch is
- * a third state-sized array (the fused kernel cannot update in place); its
+ * so state_tmp ends holding what the reference's state_tmp holds.  A direction's
+ * stages are one launch each or share one, as the form and the grid allow (the
+ * FP32 form, and FP64 grids whose lines fit a CTA: two launches a step).  scratch
+ * is a third state-sized array (the fused kernel cannot update in place); its
  * contents after the call are unspecified (in the split form each 8-byte slot
  * holds the first stage's result as a pair of floats, not a double).  dt is
  * evolve's time step; dt_full is params["dt"], the hyperviscosity time scale
@@ -137,8 +139,8 @@ int mw_step_f64(int nx, int nz, double dx, double dz, double dt_full, double dt,
  * is copied into state, the step runs as mw_step_f64 with nsteps = 1, and the
  * resulting state is copied into h_out (which may equal h_in).  Enqueued on
  * `stream`; h_out is complete once the stream is.  In the IEEE-FP64 and split
- * forms the copies overlap the computation by nbands row bands (at most 64 and
- * at most nz / 16); the results are those of copy-in, mw_step_f64, copy-out
+ * forms the copies overlap the computation by nbands row bands (at most 64, at
+ * most nz / 16 and at most one per 2^19 cells); the results are those of copy-in, mw_step_f64, copy-out
  * bit for bit.
  * h_in / h_out should be page-locked for the copies to run asynchronously.
  * Calls on one device share internal copy and compute streams (the x stages
@@ -213,8 +215,8 @@ int mw_ensemble_plan_info(int n_members, const mw_ens_member* members, int z_til
  * step call at a time: calls that use one plan must be ordered (one stream). */
 int mw_ensemble_plan(int n_members, const mw_ens_member* members, int z_tile, void* plan_device, size_t plan_bytes,
                      mw_ens_plan_info* info, void* stream);
-/* nsteps time steps of every member: 6 persistent launches per step, grid_x
- * and grid_z CTAs (0 = one full-occupancy wave); the FP64 call first writes
+/* nsteps time steps of every member: persistent launches, 6 per step (FP64) or
+ * 2 (FP32), grid_x and grid_z CTAs (0 = one full-occupancy wave); the FP64 call first writes
  * the plan's row-constant table (one more launch per call).  The direction order follows
  * *reverse as in mw_step_f64 (all members alike).  FP64 storage supports
  * f64_mode MW_F64_IEEE and MW_F64_SPLIT. */

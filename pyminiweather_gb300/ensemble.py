@@ -3,8 +3,8 @@
 No counterpart in the reference, which runs one grid per process: here many
 members -- each a full simulation with its own nx, nz, dx, dz, dt and initial
 bubbles -- share three flat state buffers and advance with one persistent
-kernel launch per direction-stage (six per step) walking a work list over all
-members (mw_ensemble_step_*).  `graph()` captures two steps (both direction
+kernel launch per direction-stage (FP64, six per step) or per direction (FP32,
+two per step) walking a work list over all members (mw_ensemble_step_*).  `graph()` captures two steps (both direction
 orders) in a CUDA graph; `autotune()` picks the z tile height and the
 persistent grid sizes by timing candidates on the ensemble itself.
 

@@ -1,7 +1,8 @@
 """Time stepping: the GPU counterpart of pyminiweather/solve/step.py:18-143.
 
-evolve() advances the state by whole time steps through mw_step_* (six fused
-direction-stage launches per step).  discrete_step() runs one direction-stage
+evolve() advances the state by whole time steps through mw_step_* (a fused
+launch per direction-stage, or per direction where a launch can hold its three
+stages).  discrete_step() runs one direction-stage
 through mw_dirstage_*.  Both write the halo cells of each forcing array as
 set_bc_x / set_bc_z do, so `fields.state` and `fields.state_tmp` hold, halo
 included, what the reference leaves in them.
@@ -121,8 +122,8 @@ def evolve(params: Dict, fields, mesh=None, dt: float = 1e-4, nsteps: int = 1) -
 # the x stages of a band run on a second stream beside the z stages of the
 # others, so the short banded launches fill each other's tails, and both forms
 # do best with 32 bands: the split form is bound by the copies (9.3 ms per
-# step), the IEEE-FP64 form by its compute (20.4 ms against 19.4 ms for the
-# step alone; 22.0 ms in 8 bands, 29.9 ms unbanded).
+# step), the IEEE-FP64 form by its compute (17.4 ms against 16.1 ms for the
+# step alone).  The library uses fewer where a band would have under 2^19 cells.
 HOST_STEP_BANDS = {"split": 32, "fp64": 32}
 
 
