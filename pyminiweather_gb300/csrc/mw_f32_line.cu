@@ -24,7 +24,7 @@ namespace f32 {
 namespace {
 
 constexpr int kF32Warps = 32;  // most per CTA, at up to 64 registers a thread
-constexpr LineKind kF32Lines = {1, {kF32Warps, 0}, {64, 0}, 1, 32, sizeof(Row), 0.4};
+constexpr LineKind kF32Lines = {1, 1, {0, kF32Warps, 0}, {0, 64, 0}, 1, 32, sizeof(Row), 0.4};
 
 struct LineF32Params : LineShape {
   F32DirArgs a;

@@ -12,8 +12,8 @@
 // of them.  On a small grid the stage kernels (mw_fp64_stage.cu) therefore pay
 // for every row a thread marches and for the row tables a CTA forms: 30 us a z
 // stage and 18 us an x stage at 100 x 50.  Here a cell is one lane's work: the
-// cells of a line are cut into runs of at most 32 SL - 2, a warp per run (slots
-// as in the x pass of mw_fp64_stage.cu), spread so that the SM partitions get
+// cells of a line are cut into runs of at most 32 SL - 2 (14 in half slots), a
+// warp per run (slots as in the x pass of mw_fp64_stage.cu), spread so that the SM partitions get
 // equal numbers of warps, and the constants of an interface's row live in the
 // registers of the lane that needs them (z) or are formed once per line (x).
 // Lines may be cut into pieces, each CTA computing four cells more on either
@@ -32,7 +32,7 @@ namespace mw {
 namespace ieee {
 
 // Most warps per CTA with SL slots per lane (as their registers allow).
-__host__ __device__ constexpr int line_warps(int sl) { return sl == 1 ? 20 : 16; }
+__host__ __device__ constexpr int line_warps(int sl) { return sl == 0 ? 24 : (sl == 1 ? 20 : 16); }
 struct LineParams : LineGeom {
   double HV, IHV;        // HV = -12 hv of the direction and 1 / HV
   double c[3], dt[3];    // per stage HV dt_stage / (12 d) and dt_stage
@@ -62,9 +62,39 @@ __device__ __forceinline__ void put(double* line, int q, int c, int n, bool whol
   }
 }
 
+// flux_x or flux_z (mw_fp64_flux.cuh) by the two halves of a warp: A and D of (DENS, UMOM) in lanes 0 .. 15, of
+// (WMOM, RHOT) of the same interfaces in lanes 16 .. 31, F likewise; the same operations on each value.
+template <int DIR>
+__device__ __forceinline__ void flux_halves(const double A[2], const double D[2], const RowD& r, double HV, double IHV,
+                                            bool wall, double F[2]) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, lo = lane & 15, hi = lo | 16;
+  const bool up = lane >= 16;
+  const double AD = __shfl_sync(kAll, A[0], lo), AT = __shfl_sync(kAll, A[1], hi);
+  double m = DIR == MW_DIR_X ? __shfl_sync(kAll, A[1], lo) : __shfl_sync(kAll, A[0], hi);  // the direction's momentum
+  double d0 = D[0];
+  if (DIR == MW_DIR_Z && wall) {
+    m = 0.0;
+    if (!up) d0 = 0.0;
+  }
+  const double u = m * rcp(fma(HV, AD, r.R), kAll);
+  const double p = pressure(AT, r, DIR == MW_DIR_X ? D[1] : d0, kAll);
+  const double t = AT + r.RT12;
+  if (DIR == MW_DIR_X) {
+    F[0] = fma(up ? u : IHV, up ? A[0] : m, d0);
+    F[1] = fma(up ? t : m, u, up ? D[1] : p);
+  } else {
+    F[0] = fma(up ? u : IHV, m, up ? p : d0);
+    F[1] = fma(u, up ? t : A[1], D[1]);
+  }
+}
+
+// SL slots per lane; SL = 0: the lanes of a warp's two halves share sixteen slots, two variables each, which shortens
+// a stage's chain of FP64 instructions (25 instead of 41) where a grid leaves SM partitions idle.
 template <int DIR, int SL>
 __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __grid_constant__ LineParams P) {
   constexpr unsigned kAll = 0xffffffffu;
+  constexpr int NS = SL == 0 ? 1 : SL, NV = SL == 0 ? 2 : 4;  // slots and variables of a lane
   extern __shared__ __align__(16) unsigned char smem_line[];
   __shared__ RowD rows[kLineMax];
   __shared__ double hr[4];
@@ -82,12 +112,13 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
   double* buf[2] = {reinterpret_cast<double*>(smem_line) + (whole ? kHs : 6 - p0),
                     reinterpret_cast<double*>(smem_line) + (size_t)4 * nl_cta * P.lp + (whole ? kHs : 6 - p0)};
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int sub = SL == 0 ? lane & 15 : lane, q0 = SL == 0 ? (lane >> 4) * 2 : 0;  // the lane's slot and first variable
   const int l = w / P.runs, rn = w - l * P.runs;   // the warp's line and run
   const int c0 = first(0) + rn * P.run, c1 = min(c0 + P.run, past(0));
   const bool live = l < nl && c0 < c1;
 
   // row constants and wall ratios (backgrounds only: the kernel before it does not write them)
-  RowD rz[SL];
+  RowD rz[NS];
   if (DIR == MW_DIR_X) {
     load_pow_tables(pow_tables);
     double r = 0.0, rt = 1.0;
@@ -106,8 +137,8 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       hr[threadIdx.x] = MW_AT(a.hyc, h, n + 2 * kHs) / MW_AT(a.hyc, src, n + 2 * kHs);
     }
 #pragma unroll
-    for (int j = 0; j < SL; ++j) {
-      const int i = min(max(c0 - 1 + 32 * j + lane, 0), n);
+    for (int j = 0; j < NS; ++j) {
+      const int i = min(max(c0 - 1 + 32 * j + sub, 0), n);
       const double rt12 = 12.0 * MW_AT(a.hyti, i, n + 1);
       rz[j].R = MW_AT(a.hyi, i, n + 1) * (12.0 * P.HV);
       rz[j].RT12 = rt12;
@@ -126,10 +157,10 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
       put<DIR>(line_at(P, buf[0], q, ll), q, c, n, whole, MW_LG(a.in, o), hr);
     });
   }
-  double sw[SL];
+  double sw[NS];
 #pragma unroll
-  for (int j = 0; j < SL; ++j) {
-    int c = c0 - 2 + 32 * j + lane;  // the cell this slot updates
+  for (int j = 0; j < NS; ++j) {
+    int c = c0 - 2 + 32 * j + sub;  // the cell this slot updates
     sw[j] = 0.0;
     if (a.srcw && live && c >= c0 && c < c1) {
       if (DIR == MW_DIR_X) c = c < 0 ? c + n : (c >= n ? c - n : c);
@@ -139,29 +170,29 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
   }
   __syncthreads();
 
-  double sv[SL][4];  // the direction's initial state at the updated cells
+  double sv[NS][NV];  // the direction's initial state at the updated cells
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
     double* src = buf[s & 1];
     double* dst = buf[(s + 1) & 1];
     if (live) {
-      double A[SL][4], D[SL][4], F[SL][4], wgt[SL];
-      const int prev = (lane + 31) & 31;
+      double A[NS][NV], D[NS][NV], F[NS][NV], wgt[NS];
+      const int prev = SL == 0 ? (lane & 16) | ((lane + 15) & 15) : (lane + 31) & 31;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double* ln = line_at(P, src, q, l);
-        double e[SL], qv[SL];
+      for (int q = 0; q < NV; ++q) {
+        const double* ln = line_at(P, src, q0 + q, l);
+        double e[NS], qv[NS];
 #pragma unroll
-        for (int j = 0; j < SL; ++j) {
+        for (int j = 0; j < NS; ++j) {
           // slots beyond the stage's cells repeat its last ones (not used)
-          const int i = min(max(c0 - 1 + 32 * j + lane, first(s) - 1), past(s));
+          const int i = min(max(c0 - 1 + 32 * j + sub, first(s) - 1), past(s));
           const double sm = ln[i - 1];
           cell_eq(sm, ln[i], ln[i + 1], e[j], qv[j]);
           if (s == 0) sv[j][q] = sm;
-          if (q == DENS) wgt[j] = sm;
+          if (q == DENS) wgt[j] = SL == 0 ? line_at(P, src, DENS, l)[i - 1] : sm;
         }
 #pragma unroll
-        for (int j = 0; j < SL; ++j) {
+        for (int j = 0; j < NS; ++j) {
           // slot j - 1's: lane 31 hands its slot of the group before to lane 0; slot 0 has none (not used)
           const double ep = __shfl_sync(kAll, j > 0 && lane == 31 ? e[j > 0 ? j - 1 : 0] : e[j], prev);
           const double qp = __shfl_sync(kAll, j > 0 && lane == 31 ? qv[j > 0 ? j - 1 : 0] : qv[j], prev);
@@ -170,32 +201,43 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
         }
       }
 #pragma unroll
-      for (int j = 0; j < SL; ++j) {
-        const int i = c0 - 1 + 32 * j + lane;
-        if (DIR == MW_DIR_X)
+      for (int j = 0; j < NS; ++j) {
+        const int i = c0 - 1 + 32 * j + sub;
+        if constexpr (SL == 0)
+          flux_halves<DIR>(A[j], D[j], DIR == MW_DIR_X ? rows[l] : rz[j], P.HV, P.IHV, i <= 0 || i >= n, F[j]);
+        else if (DIR == MW_DIR_X)
           flux_x(A[j], D[j], rows[l], P.HV, P.IHV, kAll, F[j]);
         else
           flux_z(A[j], D[j], rz[j], P.HV, P.IHV, i <= 0 || i >= n, kAll, F[j]);
       }
 #pragma unroll
-      for (int j = 0; j < SL; ++j) {
-        const int c = c0 - 2 + 32 * j + lane;
-        double v[4];
+      for (int j = 0; j < NS; ++j) {
+        const int c = c0 - 2 + 32 * j + sub;
+        double v[NV];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < NV; ++q) {
           const double Fp = __shfl_sync(kAll, j > 0 && lane == 31 ? F[j > 0 ? j - 1 : 0][q] : F[j][q], prev);
           v[q] = fma(P.c[s], Fp - F[j][q], sv[j][q]);
         }
-        if (DIR == MW_DIR_Z) v[WMOM] = fma(-P.dt[s] * kGrav, wgt[j], v[WMOM]);
-        if (a.srcw) v[WMOM] = fma(P.dt[s], sw[j], v[WMOM]);
-        if (c >= max(c0, first(s)) && c < min(c1, past(s))) {
+        // of a warp's lower half this is no variable: its values are left as they are
+        double& vw = v[SL == 0 ? 0 : WMOM];
+        const bool has_w = SL != 0 || q0 == WMOM;
+        if (DIR == MW_DIR_Z) {
+          const double g = fma(-P.dt[s] * kGrav, wgt[j], vw);
+          vw = has_w ? g : vw;
+        }
+        if (a.srcw) {
+          const double f = fma(P.dt[s], sw[j], vw);
+          vw = has_w ? f : vw;
+        }
+        if (c >= max(c0, first(s)) && c < min(c1, past(s)) && (SL != 0 || sub >= 2)) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) put<DIR>(line_at(P, dst, q, l), q, c, n, whole, v[q], hr);
+          for (int q = 0; q < NV; ++q) put<DIR>(line_at(P, dst, q0 + q, l), q0 + q, c, n, whole, v[q], hr);
           const bool edge = c < p0 || c >= p1 ? false : DIR == MW_DIR_X ? (c < kHs || c >= n - kHs) : (c == 0 || c == n - 1);
           if (edge) {
             const int line = DIR == MW_DIR_X ? l0 + l : l0 + l + kHs;
-            if (s == 0 && a.halo_in) halo_out<DIR>(P, a.halo_in, line, c, sv[j], hr);
-            if (s == 1 && a.halo_tmp) halo_out<DIR>(P, a.halo_tmp, line, c, v, hr);
+            if (s == 0 && a.halo_in) halo_out<DIR, NV>(P, a.halo_in, line, c, sv[j], hr, q0);
+            if (s == 1 && a.halo_tmp) halo_out<DIR, NV>(P, a.halo_tmp, line, c, v, hr, q0);
           }
         }
       }
@@ -226,9 +268,12 @@ int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, bool 
 }
 
 // two slots of a run repeat its neighbours' (x pass of mw_fp64_stage.cu)
-constexpr LineKind kIeeeLines = {2, {line_warps(1), line_warps(2)}, {96, 128}, 2, 64, 0, 0.0};
+constexpr LineKind kIeeeLines = {0, 2, {line_warps(0), line_warps(1), line_warps(2)}, {80, 96, 128}, 2, 64, 0, 0.0};
 
 constexpr int kMaxPieces = 16;
+// A warp of half slots against one of whole ones: 0.61 in FP64 instructions, more in time (us a step, one a call:
+// 60x30 27.9 -> 23.5, 100x50 26.7 -> 23.4; where partitions get two warps for one it loses, 200x100 31.0 -> 36.2).
+constexpr double kHalfCost = 0.75;
 
 // The spread with the least time.  An SM that gets m CTAs of W warps with SL
 // slots per lane gives its four partitions m W SL / 4 slot groups each, every
@@ -257,19 +302,19 @@ constexpr int kMaxPieces = 16;
 LineSpread spread_lines(const LineKind& kind, int n, int nlines, bool isx, int sms) {
   LineSpread best;
   double least = 0.0;
-  for (int sl = 1; sl <= kind.max_slots; ++sl)
+  for (int sl = kind.min_slots; sl <= kind.max_slots; ++sl)
     for (int pieces = 1; pieces == 1 || (pieces <= kMaxPieces && (n + pieces - 1) / pieces >= 24); ++pieces) {
       const int piece = (n + pieces - 1) / pieces;
       if ((n + piece - 1) / piece != pieces) continue;  // an empty last piece
       const int range = pieces == 1 ? n : piece + 8;
       if (pieces > 1 && range >= n) break;
-      const int cells = 32 * sl - kind.shared_slots, runs = (range + cells - 1) / cells;
+      const int cells = (sl == 0 ? 16 : 32 * sl) - kind.shared_slots, runs = (range + cells - 1) / cells;
       const int lp = (pieces == 1 ? n + 2 * kHs : piece + 12) | 1;
       for (int lg = 0; (1 << lg) <= kLineMax; ++lg) {
         const int warps = runs << lg;
         const size_t smem = line_smem(kind, lp, lg, isx);
-        if (warps > kind.warps[sl - 1] || smem > kLineSmem) break;
-        const int resident = std::min((int)(65536 / (kind.regs[sl - 1] * 32 * warps)), (int)((220 << 10) / smem));
+        if (warps > kind.warps[sl] || smem > kLineSmem) break;
+        const int resident = std::min((int)(65536 / (kind.regs[sl] * 32 * warps)), (int)((220 << 10) / smem));
         const double load = (double)((nlines + (1 << lg) - 1) >> lg) * pieces / sms;
         const double turns = std::min(std::ceil(load / resident) * resident, load + 0.5 * resident) * warps / 4.0;
         const double once = std::ceil(load) * warps / 4.0;
@@ -278,11 +323,11 @@ LineSpread spread_lines(const LineKind& kind, int n, int nlines, bool isx, int s
           cost = (once + kind.tail * std::max(warps, 4)) * (1.0 + 0.3 / resident) * (1.0 + 0.001 * pieces) *
                  (warps < 4 ? 1.1 : 1.0) * (!isx && lg == 0 ? 1.2 : 1.0);
         } else {
-          cost = sl * (load <= resident ? 0.1 * once + 0.9 * std::ceil(once) : turns);
+          cost = (sl == 0 ? kHalfCost : sl) * (load <= resident ? 0.1 * once + 0.9 * std::ceil(once) : turns);
           cost *= (1.0 + 0.1 / resident) * (1.0 + 0.001 * load) * (pieces > 1 ? 1.01 : 1.0) *
                   (!isx && lg == 0 ? 1.03 : 1.0) * (sl == 2 && once < 2.0 ? 1.3 : 1.0);
         }
-        if (best.sl == 0 || cost < least) {
+        if (best.runs == 0 || cost < least) {
           least = cost;
           const int run = (range + runs - 1) / runs;
           best = {sl, lg, pieces, piece, (range + run - 1) / run, run, lp};
@@ -310,7 +355,7 @@ LinePlan line_plan(const LineKind& kind, int nx, int nz, int sms) {
   LinePlan p;
   p.x = ieee::spread_lines(kind, nx, nz, true, sms);
   p.z = ieee::spread_lines(kind, nz, nx, false, sms);
-  p.fits = p.x.sl > 0 && p.z.sl > 0;
+  p.fits = p.x.runs > 0 && p.z.runs > 0;
   p.cut = p.x.pieces > 1 || p.z.pieces > 1;
   return p;
 }
@@ -343,10 +388,13 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
   int ctas, threads;
   set_line_geom(&P, sp, nx, nz, isx, &ctas, &threads);
   const size_t smem = line_smem(kIeeeLines, P.lp, P.log_lines, isx);
-  if (isx) return sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>(P, ctas, threads, smem, overlap, stream)
-                               : launch_line_t<MW_DIR_X, 2>(P, ctas, threads, smem, overlap, stream);
-  return sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>(P, ctas, threads, smem, overlap, stream)
-                      : launch_line_t<MW_DIR_Z, 2>(P, ctas, threads, smem, overlap, stream);
+  const auto launch = isx ? (sp.sl == 0   ? launch_line_t<MW_DIR_X, 0>
+                             : sp.sl == 1 ? launch_line_t<MW_DIR_X, 1>
+                                          : launch_line_t<MW_DIR_X, 2>)
+                          : (sp.sl == 0   ? launch_line_t<MW_DIR_Z, 0>
+                             : sp.sl == 1 ? launch_line_t<MW_DIR_Z, 1>
+                                          : launch_line_t<MW_DIR_Z, 2>);
+  return launch(P, ctas, threads, smem, overlap, stream);
 }
 
 #if MW_CHECK

@@ -37,7 +37,7 @@ struct LineArgs {
   double* halo_tmp;    // and of the second stage
 };
 
-// How a direction's lines are spread over CTAs: slots per lane, lines per CTA
+// How a direction's lines are spread over CTAs (fits where runs > 0): slots per lane, lines per CTA
 // (log2), pieces per line and cells per piece, runs (warps) per line and cells
 // per run, and a line's pitch in shared memory.
 struct LineSpread {
@@ -55,9 +55,10 @@ int line_ieee_plan(int nx, int nz, LinePlan* plan);
 
 // What the spread of a form's lines depends on.
 struct LineKind {
-  int max_slots;        // slots per lane, at most
-  int warps[2];         // most warps per CTA with one and two slots
-  int regs[2];          // registers per thread with one and two slots
+  int min_slots;        // slots per lane, at least and at most (0: half a slot, the variables in two halves of a warp)
+  int max_slots;
+  int warps[3];         // most warps per CTA with none, one and two slots
+  int regs[3];          // registers per thread with none, one and two slots
   int shared_slots;     // slots of a run that its neighbour has too
   int cell_bytes;       // shared memory per cell
   int row_bytes;        // and per cell of a column's row table (z)

@@ -51,23 +51,23 @@ inline void set_line_geom(LineShape* P, const LineSpread& sp, int nx, int nz, bo
 
 #define MW_LG(p, off) MW_AT((p), (off), 4 * P.plane)
 
-// The halo cells that cell c of a line is the source of, in a global array.
-template <int DIR>
-__device__ __forceinline__ void halo_out(const LineGeom& P, double* g, int line, int c, const double v[4],
-                                         const double* hr) {
+// The halo cells that cell c of a line is the source of, in a global array; v[0 .. NV): variables q0 onwards.
+template <int DIR, int NV = 4>
+__device__ __forceinline__ void halo_out(const LineGeom& P, double* g, int line, int c, const double* v,
+                                         const double* hr, int q0 = 0) {
   const int n = P.n;
   if (DIR == MW_DIR_X) {
     const long long row = (long long)(line + kHs) * P.pitch;
-    for (int q = 0; q < 4; ++q) {
-      if (c < kHs) MW_LG(g, q * P.plane + row + n + kHs + c) = v[q];
-      if (c >= n - kHs) MW_LG(g, q * P.plane + row + c - n + kHs) = v[q];
+    for (int q = q0; q < q0 + NV; ++q) {
+      if (c < kHs) MW_LG(g, q * P.plane + row + n + kHs + c) = v[q - q0];
+      if (c >= n - kHs) MW_LG(g, q * P.plane + row + c - n + kHs) = v[q - q0];
     }
   } else {
-    for (int q = 0; q < 4; ++q)
+    for (int q = q0; q < q0 + NV; ++q)
       for (int h = 0; h < 4; ++h)
         if (c == (h < 2 ? 0 : n - 1))
           MW_LG(g, q * P.plane + (long long)(h < 2 ? h : n + h) * P.pitch + line) =
-              q == WMOM ? 0.0 : (q == UMOM ? v[q] * hr[h] : v[q]);
+              q == WMOM ? 0.0 : (q == UMOM ? v[q - q0] * hr[h] : v[q - q0]);
   }
 }
 

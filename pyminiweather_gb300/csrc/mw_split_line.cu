@@ -27,7 +27,7 @@ namespace mw {
 namespace {
 
 constexpr int kSplitWarps = 20;  // most per CTA (88 registers a thread)
-constexpr LineKind kSplitLines = {1, {kSplitWarps, 0}, {88, 0}, 1, 96, sizeof(RowS), 0.4};
+constexpr LineKind kSplitLines = {1, 1, {0, kSplitWarps, 0}, {0, 88, 0}, 1, 96, sizeof(RowS), 0.4};
 
 struct SplitLineParams : LineGeom {
   dwc hv12, d12, gz12;   // 12 hv, 12 d, 12 dz grav
