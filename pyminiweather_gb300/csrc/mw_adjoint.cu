@@ -624,7 +624,7 @@ int launch_vjp_row_table(int nx, int nz, const double* hyc, const double* hytc, 
                          const double* hypi, void* workspace, cudaStream_t stream);
 int launch_vjp_split(int nx, int nz, double dx, double dz, double dt_full, const double* hyc, const void* table,
                      const double* forcing, const double* g_out, const double* g_base_a, const double* g_base_b,
-                     int add_g_out, double* g_dst, double dt_stage, int direction, cudaStream_t stream);
+                     int add_g_out, double* g_dst, double dt_stage, int direction, bool follows, cudaStream_t stream);
 size_t vjp_split_table_bytes(int nz);
 
 }  // namespace mw
@@ -668,7 +668,7 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
     if (!table_ready && (st = launch_vjp_row_table(nx, nz, hyc, hytc, hyi, hyti, hypi, workspace, (cudaStream_t)stream)))
       return st;
     return launch_vjp_split(nx, nz, dx, dz, dt_full, hyc, workspace, forcing, g_out, g_base_a, g_base_b, add_g_out,
-                            g_dst, dt_stage, direction, (cudaStream_t)stream);
+                            g_dst, dt_stage, direction, follows || !table_ready, (cudaStream_t)stream);
   }
   const Geom g = make_geom(nx, nz);
   VjpArgs a;
