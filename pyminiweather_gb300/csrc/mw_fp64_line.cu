@@ -153,8 +153,12 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
   {
     const int ca = whole ? 0 : (DIR == MW_DIR_X ? p0 - 6 : max(p0 - 6, 0));
     const int cb = whole ? n : (DIR == MW_DIR_X ? p1 + 6 : min(p1 + 6, n));
-    each_cell<DIR>(P, l0, nl, ca, cb, [&](int q, int ll, int c, long long o) {
-      put<DIR>(line_at(P, buf[0], q, ll), q, c, n, whole, MW_LG(a.in, o), hr);
+    each_cell4<DIR>(P, l0, nl, ca, cb, [&](int ll, int c, long long o) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = MW_LG(a.in, q * P.plane + o);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) put<DIR>(line_at(P, buf[0], q, ll), q, c, n, whole, v[q], hr);
     });
   }
   double sw[NS];
@@ -246,8 +250,9 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     if (s == 2) overlap_next();  // at the latest (kLineFewCtas)
     double* g = s == 0 ? a.s1 : (s == 1 ? a.s2 : a.out);
     if (g)
-      each_cell<DIR>(P, l0, nl, p0, p1, [&](int q, int ll, int c, long long o) {
-        MW_LG(g, o) = line_at(P, dst, q, ll)[c];
+      each_cell4<DIR>(P, l0, nl, p0, p1, [&](int ll, int c, long long o) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) MW_LG(g, q * P.plane + o) = line_at(P, dst, q, ll)[c];
       });
   }
   if (DIR == MW_DIR_Z && blockIdx.x == 0 && threadIdx.x < 8) halo_corners(P, hr);

@@ -71,27 +71,6 @@ __device__ __forceinline__ void halo_out(const LineGeom& P, double* g, int line,
   }
 }
 
-// Cells [ca, cb) of the CTA's lines, between a global array and shared memory
-// (x: periodic).  x: a warp per line and variable; z: consecutive threads take
-// the CTA's columns of a row.
-template <int DIR, typename Fn>
-__device__ __forceinline__ void each_cell(const LineGeom& P, int l0, int nl, int ca, int cb, Fn fn) {
-  if (DIR == MW_DIR_X) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int ql = w; ql < 4 * nl; ql += nw) {
-      const int q = ql / nl, l = ql - q * nl;
-      const long long o = q * P.plane + (long long)(l0 + l + kHs) * P.pitch + kHs;
-      for (int c = ca + lane; c < cb; c += 32) fn(q, l, c, o + (c < 0 ? c + P.n : (c >= P.n ? c - P.n : c)));
-    }
-  } else {
-    for (int q = 0; q < 4; ++q)
-      for (int i = threadIdx.x; i < ((cb - ca) << P.log_lines); i += blockDim.x) {
-        const int l = i & ((1 << P.log_lines) - 1), c = ca + (i >> P.log_lines);
-        if (l < nl) fn(q, l, c, q * P.plane + (long long)(c + kHs) * P.pitch + l0 + l + kHs);
-      }
-  }
-}
-
 // Cells [ca, cb) of the CTA's lines, each by one thread: fn(line, cell, offset in a plane of a global array).
 template <int DIR, typename Fn>
 __device__ __forceinline__ void each_cell4(const LineShape& P, int l0, int nl, int ca, int cb, Fn fn) {
