@@ -250,10 +250,7 @@ __global__ void __launch_bounds__(128) k_vjp_gather(VjpArgs a) {
       gather_general<DIR>(a, k, i, acc);
     }
     if (DIR == MW_DIR_Z) acc[DENS] -= a.dt_stage * kGrav * gval(a, WMOM, k, i);
-    for (int q = 0; q < 4; ++q) {
-      const long long o = q * a.plane + idx;
-      store_value(a, o, acc[q]);
-    }
+    for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + idx, acc[q]);
   }
 }
 
@@ -451,7 +448,7 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
 //
 // Bound: FP64 (512 x 256, a stage without bases: 2375 instructions on the
 // fullest SM at 16 cycles each, 38000 of its 53500 active cycles; the rest is
-// the first and last loads and stores, which all warps meet together).  30.8 us
+// the first and last loads and stores, which all warps meet together).  29.7 us
 // a stage at 512 x 256, with the bases counted in, against 14.8 + 21 us for
 // the interface adjoints and the gather as two kernels with the 8 values per
 // interface in memory between them.  Sixteen warps a CTA: 33 us.  Rows read
@@ -478,6 +475,26 @@ __device__ __forceinline__ void gather_wall(const VjpArgs& a, const double* ws, 
       }
     }
   }
+}
+
+// g_dst of a cell (offset o in a plane).  With g_out and both bases, as in the last stage of a direction, the twelve
+// loads are in flight together: one by one behind the stores the few warps of a tile waited for each (31.1 us a stage
+// on average, 29.7 so; the x kernel, with twice the warps, is slower so: 27.3 against 29.1).
+__device__ __forceinline__ void store_cell(const VjpArgs& a, long long o, const double acc[4]) {
+  if (a.add_gout && a.base_a && a.base_b) {
+    double g[4], p[4], r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      g[q] = MW_AT(a.gout, q * a.plane + o, 4 * a.plane);
+      p[q] = MW_AT(a.base_a, q * a.plane + o, 4 * a.plane);
+      r[q] = MW_AT(a.base_b, q * a.plane + o, 4 * a.plane);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) MW_AT(a.gdst, q * a.plane + o, 4 * a.plane) = acc[q] + g[q] + p[q] + r[q];
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + o, acc[q]);
 }
 
 __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV* rows, int tile_rows) {
@@ -560,9 +577,7 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
           acc[q] = gather4(a, A[q][0], A[q][1], A[q][2], A[q][3], D[q][0], D[q][1], D[q][2], D[q][3]);
         if (k == 0 || k == a.nz - 1) gather_wall(a, ws, fa, k, acc);
         acc[DENS] = fma(-a.dt_stage * kGrav, gval(a, WMOM, k, col - kHs), acc[DENS]);
-        if (in)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + o, acc[q]);
+        if (in) store_cell(a, o, acc);
       }
     }
     __syncthreads();
@@ -574,7 +589,7 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
 // interfaces and rows counted alike (about 40 FP64 operations each) and one
 // more per tile for its loads, on the SM with the most tiles; of equals the
 // tallest, which recompute the fewest interfaces.  512 x 256: 29 rows, 144 tiles,
-// 30.8 us.  From a third to twice the charge per tile: the same times within 1 %
+// 29.7 us.  From a third to twice the charge per tile: the same times within 1 %
 // from 100 x 50 to 640 x 448.
 inline int fz_rows(int nx, int nz, int sms) {
   const long long nxt = (nx + 31) / 32;

@@ -8,9 +8,9 @@ namespace mw {
 
 // Most cells of a grid that takes the line kernels: above this the CTAs of a
 // launch come in several waves and the stage kernels, which need no whole lines
-// in a CTA, do as well (us per step, line kernels / six stage launches replayed
-// from a graph: 100x50 24 / 121, 300x150 41 / 122, 512x256 113 / 145, 800x400
-// 237 / 279, 990x495 354 / 387, 992x992 659 / 661, 1200x600 482 / 469).
+// in a CTA, do as well (us per step, eight a call, line kernels / six stage
+// launches: 100x50 18 / 118, 300x150 41 / 122, 512x256 110 / 145, 800x400 237 / 279,
+// 990x495 346 / 376, 1000x640 440 / 452; 1200x600 473 / 457, 992x992 665 / 653).
 constexpr long long kLineCellsMax = 600000;
 
 // The double-FP32 form's (100x50 14 / 61, 300x150 18 / 73, 512x256 38 / 70, 700x500
