@@ -215,11 +215,10 @@ extern "C" int mw_ensemble_plan(int n_members, const mw_ens_member* members, int
         c.gz12[0] = gz12.h, c.gz12[1] = gz12.l;
         c.c12[0] = c12.h, c.c12[1] = c12.l;
         c.c12s = dts / (12.0 * d) * split::kTwoPow896;  // exact: a power-of-two scale
-        const F32Consts f = f32_consts(d, m.dt);  // as launch_dir_f32 forms them
-        c.hv_f = f.HV;
-        c.ihv_f = f.IHV;
-        c.c_f = f32_c(d, m.dt, dts);
+        c.hv_f = f32_hv(d, m.dt);  // as launch_dir_f32 forms them
+        c.c_f = f32_c(d, dts);
         c.dt_f = (float)dts;
+        c.pad = 0.0f;
         c.HV = ieee_hv(d, m.dt);  // as launch_stage_ieee forms them
         c.IHV = 1.0 / c.HV;
         c.c = dts / (12.0 * d) * c.HV;

@@ -11,14 +11,14 @@ namespace mw {
 // Stage constants of one member for one direction-stage, formed on the host
 // when the plan is built, exactly as the single-grid launches form them.
 // Split form: (h, l) float pairs of 12 hv, 12 d, 12 dz g and dt_stage / (12 d),
-// and dt_stage / (12 d) * 2^896 in FP64.  FP32 form: HV, HV dt_stage / (2 d),
-// dt_stage and 1 / HV rounded to float (mw_f32_dir.cuh).  IEEE-FP64 form: HV = -12 hv, 1 / HV,
+// and dt_stage / (12 d) * 2^896 in FP64.  FP32 form: HV = -2 hv, dt_stage / (2 d)
+// and dt_stage rounded to float.  IEEE-FP64 form: HV = -12 hv, 1 / HV,
 // HV dt_stage / (12 d) and dt_stage.  Entry (member * 2 + (direction == z)) * 3 + stage
 // (stage 0, 1, 2: dt/3, dt/2, dt).
 struct EnsMemberConsts {
   float hv12[2], d12[2], gz12[2], c12[2];
   double c12s;
-  float hv_f, c_f, dt_f, ihv_f;
+  float hv_f, c_f, dt_f, pad;
   double HV, IHV, c, dt;
 };
 static_assert(sizeof(EnsMemberConsts) == 88, "EnsMemberConsts layout");

@@ -22,9 +22,8 @@
 // memory by asynchronous copies, one run ahead.
 // Arithmetic: the two stencils by second differences (e = s(k-1) - 2 s(k) +
 // s(k+1), q = s - e / 6: twice the interpolation is q(k-1) + q(k), the third
-// difference e(k) - e(k-1)), fluxes carried over HV = -2 hv as in the
-// IEEE-FP64 form (mw_fp64_flux.cuh), the variables in pairs (DENS, UMOM) and
-// (WMOM, RHOT) through packed FP32 instructions.
+// difference e(k) - e(k-1)), the variables in pairs (DENS, UMOM) and (WMOM,
+// RHOT) through packed FP32 instructions (mw_f32_flux.cuh).
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -143,7 +142,7 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
   const int t = threadIdx.x, nz = a.nz;
   for (int i = t; i <= last - a0 + 5; i += NC) {  // interface a0 - 6 + i, clamped where nothing uses it
     const int k = min(max(a0 - 6 + i, 0), nz);
-    tab[i] = row_z(a.k, MW_AT(a.hyi, k, nz + 1), MW_AT(a.hyti, k, nz + 1), MW_AT(a.hypi, k, nz + 1));
+    tab[i] = row_z(MW_AT(a.hyi, k, nz + 1), MW_AT(a.hyti, k, nz + 1), MW_AT(a.hypi, k, nz + 1));
   }
   if (t < 4) {
     const int h = t < 2 ? t : nz + t, src = t < 2 ? kHs : nz + kHs - 1;
@@ -444,7 +443,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
   const long long g0 = total * w / nw, g1 = total * (w + 1) / nw;
   int k = (int)(g0 / nrun), rn = (int)(g0 - (long long)k * nrun);
   Row row = {0.f, 0.f, 0.f, 0.f};
-  if (g0 < g1) row = row_x(a.k, MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
+  if (g0 < g1) row = row_x(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
   overlap_wait();
   if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   if (g0 >= g1) return;
@@ -467,7 +466,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
     if (c0 == 0) x_halo_in(a, kc);
     x_run<V, SRC>(a, kc, c0, min(len, a.nx - c0), row, buf[cur]);
     if (k != kc && g + 1 < g1)
-      row = row_x(a.k, MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
+      row = row_x(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
     cur ^= 1;
   }
 }
@@ -499,9 +498,6 @@ __device__ __forceinline__ Args member_args(const EnsStageT<float>& es, int e) {
     a.k.gdt[s] = a.k.dt[s] * -float(kGrav);
   }
   a.k.HV = MW_AT(c, 0, 3).hv_f;
-  a.k.IHV = MW_AT(c, 0, 3).ihv_f;
-  a.k.R2 = 2.0f * a.k.HV;
-  a.k.P2 = 2.0f * a.k.IHV;
   return a;
 }
 
@@ -516,7 +512,7 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_ens_x_f32(EnsStageT<float> 
     const int k = item.y, nrun = (a.nx + x_run_max(kEnsV) - 1) / x_run_max(kEnsV), len = (a.nx + nrun - 1) / nrun;
     __syncwarp();
     x_load<kEnsV>(a, k, 0, min(len, a.nx), buf[0]);
-    const Row row = row_x(a.k, MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
+    const Row row = row_x(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
     x_halo_in(a, k);
     int cur = 0;
     for (int c0 = 0; c0 < a.nx; c0 += len) {

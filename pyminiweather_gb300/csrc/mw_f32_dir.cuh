@@ -19,22 +19,10 @@ struct F32DirArgs {
   float* halo_tmp;     // and of the second stage
 };
 
-// HV = -2 hv of the FP32 form (hv = -hv_beta d / (16 dt_full)) and its
-// reciprocal, held in [2^-60, 2^110], where the fluxes over HV keep their range.
-struct F32Consts {
-  float HV, IHV;
-};
-inline double f32_hv(double d, double dt_full) {
-  return std::fmin(std::fmax(2.0 * kHvBeta * d / (16 * dt_full), 0x1p-60), 0x1p110);
-}
-inline F32Consts f32_consts(double d, double dt_full) {
-  const double hv = f32_hv(d, dt_full);
-  return {(float)hv, (float)(1.0 / hv)};
-}
-// The update's factor HV dt_stage / (2 d).
-inline float f32_c(double d, double dt_full, double dt_stage) {
-  return (float)(f32_hv(d, dt_full) * (dt_stage / (2.0 * d)));
-}
+// HV = -2 hv of the FP32 form (hv = -hv_beta d / (16 dt_full)) and the update's
+// factor dt_stage / (2 d): the kernels carry values and fluxes times 2.
+inline float f32_hv(double d, double dt_full) { return (float)(2.0 * kHvBeta * d / (16 * dt_full)); }
+inline float f32_c(double d, double dt_stage) { return (float)(dt_stage / (2.0 * d)); }
 
 // Whether a row is short enough for the z pass's 32-bit offsets within a tile
 // (25 rows below 2^32 bytes); longer ones are stepped stage by stage.

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kF32Warps * 32, 1) k_line_f32(const __grid_con
   if (DIR == MW_DIR_X) {
     if (threadIdx.x < nl) {
       const int k = l0 + threadIdx.x + kHs;
-      rows[threadIdx.x] = row_x(P.k, MW_AT(a.hyc, k, P.nlines + 2 * kHs), MW_AT(a.hytc, k, P.nlines + 2 * kHs));
+      rows[threadIdx.x] = row_x(MW_AT(a.hyc, k, P.nlines + 2 * kHs), MW_AT(a.hytc, k, P.nlines + 2 * kHs));
     }
   } else {
     if (threadIdx.x < 4) {
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kF32Warps * 32, 1) k_line_f32(const __grid_con
       hr[threadIdx.x] = MW_AT(a.hyc, h, n + 2 * kHs) / MW_AT(a.hyc, src, n + 2 * kHs);
     }
     for (int i = first(0) + threadIdx.x; i <= past(0); i += blockDim.x)
-      rz[i - first(0)] = row_z(P.k, MW_AT(a.hyi, i, n + 1), MW_AT(a.hyti, i, n + 1), MW_AT(a.hypi, i, n + 1));
+      rz[i - first(0)] = row_z(MW_AT(a.hyi, i, n + 1), MW_AT(a.hyti, i, n + 1), MW_AT(a.hypi, i, n + 1));
     __syncthreads();  // hr
   }
   overlap_wait();
