@@ -88,7 +88,8 @@ struct Stream {
 };
 
 // What row `idx` of a stage's input yields: the row as it enters the stream,
-// its e, q and flux, and row idx - 2 of the stage's result.  WALL: the row may
+// its e, q and flux, and row idx - 2 of the stage's result (src: dt_stage times
+// the forcing of its w).  WALL: the row may
 // be a wall's (the rows that follow nz - 1 are built from the stream); without
 // it 2 <= idx < nz holds.
 struct Pushed {
@@ -96,7 +97,7 @@ struct Pushed {
 };
 template <bool WALL, bool ANY>
 __device__ __forceinline__ Pushed push(const Stream& st, Vars v, int idx, int nz, const double* hr, const Row& row,
-                                       const Consts& k, int stage, const Vars& init, bool& far) {
+                                       const Consts& k, int stage, const Vars& init, float src, bool& far) {
   if (WALL) {
     if (idx == nz) v = wall_halo(st.s1, hr, 2);
     if (idx == nz + 1) v = wall_halo(st.s0, hr, 3);
@@ -106,8 +107,8 @@ __device__ __forceinline__ Pushed push(const Stream& st, Vars v, int idx, int nz
   cell_eq(st.s0, st.s1, v, r.e, r.q);
   const Vars A = {f2add(st.q.a, r.q.a), f2add(st.q.b, r.q.b)}, D = {f2sub(r.e.a, st.e.a), f2sub(r.e.b, st.e.b)};
   r.F = flux<MW_DIR_Z, ANY>(A, D, row, k, WALL && (idx == 1 || idx == nz + 1), far);
-  r.o = update(init, st.F, r.F, k.c[stage]);
-  r.o.b.x = fmaf(k.gdt[stage], st.s0.a.x, r.o.b.x);  // gravity on the forcing's rho' (interpolate.py:248-250)
+  // gravity on the forcing's rho' (interpolate.py:248-250) and the source
+  r.o = update(init, st.F, r.F, k.c[stage], fmaf(k.gdt[stage], st.s0.a.x, src));
   return r;
 }
 template <bool WALL>
@@ -221,13 +222,15 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
     // row idx into stage s; its result's row idx - 2
     auto stage = [&](int s, const Vars& v, int idx, const Vars& init) {
       bool far = false;
-      Pushed p = push<W, W>(st[s], v, idx, nz, sm.hr, rw[5 - 2 * s], a.k, s, init, far);
-      if (!W && __any_sync(0xffffffffu, far)) p = push<W, true>(st[s], v, idx, nz, sm.hr, rw[5 - 2 * s], a.k, s, init, far);
-      commit<W>(st[s], p, idx, sm.hr);
+      float src = 0.0f;
       if (SRC) {
         const int k = idx - 2;
-        if (k >= a0 && k < nz) p.o.b.x = fmaf(a.k.dt[s], split::d2f(srcs[(k & (kRing - 1)) * NC + t]), p.o.b.x);
+        if (k >= a0 && k < nz) src = a.k.dt[s] * split::d2f(srcs[(k & (kRing - 1)) * NC + t]);
       }
+      Pushed p = push<W, W>(st[s], v, idx, nz, sm.hr, rw[5 - 2 * s], a.k, s, init, src, far);
+      if (!W && __any_sync(0xffffffffu, far))
+        p = push<W, true>(st[s], v, idx, nz, sm.hr, rw[5 - 2 * s], a.k, s, init, src, far);
+      commit<W>(st[s], p, idx, sm.hr);
       return p.o;
     };
     const Vars v1 = stage(0, ring(r), r, st[0].s0);
@@ -321,9 +324,13 @@ __device__ __forceinline__ void x_load(const Args& a, int k, int c0, int len, XB
   copies_commit();
 }
 
-// One stage of a run: v from S and v, shuffles across the warp.
-template <int V, bool ANY>
-__device__ __forceinline__ void x_stage(Vars (&v)[V], const Vars (&S)[V], const Row& row, const Consts& k, float c) {
+// One stage of a run: v from S and v, shuffles across the warp.  SRC: dt times src is added to rho w.
+template <int V, bool ANY, bool SRC>
+__device__ __forceinline__ void x_stage(Vars (&v)[V], const Vars (&S)[V], const Row& row, const Consts& k, float c,
+                                        float dt, const float (&src)[V]) {
+  auto upd = [&](int j, const Vars& Fp, const Vars& F) {
+    return SRC ? update(S[j], Fp, F, c, dt * src[j]) : update(S[j], Fp, F, c);
+  };
   const Vars m2 = shfl_up(v[V - 2]), m1 = shfl_up(v[V - 1]), p = shfl_down(v[0]);
   Vars e0, q0, Fp, F0;
   cell_eq(m2, m1, v[0], e0, q0);
@@ -339,13 +346,13 @@ __device__ __forceinline__ void x_stage(Vars (&v)[V], const Vars (&S)[V], const 
     if (j == 0)
       F0 = F;
     else
-      v[j - 1] = update(S[j - 1], Fp, F, c);
+      v[j - 1] = upd(j - 1, Fp, F);
     Fp = F;
     e0 = e;
     q0 = q;
     before = cur;
   }
-  v[V - 1] = update(S[V - 1], Fp, shfl_down(F0), c);
+  v[V - 1] = upd(V - 1, Fp, shfl_down(F0));
 }
 
 // The run of `len` cells from c0 of row k, staged in b (which it reuses for its
@@ -409,12 +416,9 @@ __device__ __forceinline__ void x_run(const Args& a, int k, int c0, int len, con
 #pragma unroll
     for (int j = 0; j < V; ++j) m = fmaxf(m, fabsf(v[j].b.y));
     if (__any_sync(0xffffffffu, m > near))
-      x_stage<V, true>(v, S, row, a.k, a.k.c[s]);
+      x_stage<V, true, SRC>(v, S, row, a.k, a.k.c[s], a.k.dt[s], src);
     else
-      x_stage<V, false>(v, S, row, a.k, a.k.c[s]);
-    if (SRC)
-#pragma unroll
-      for (int j = 0; j < V; ++j) v[j].b.x = fmaf(a.k.dt[s], src[j], v[j].b.x);
+      x_stage<V, false, SRC>(v, S, row, a.k, a.k.c[s], a.k.dt[s], src);
     if (s == 1 && (a.s2 || a.halo_tmp)) stage_out(a.s2, a.halo_tmp != nullptr);
   }
   stage_out(a.out, false);

@@ -107,6 +107,14 @@ __device__ __forceinline__ Vars update(const Vars& init, const Vars& Fp, const V
   return {f2fma(f2sub(Fp.a, F.a), f2splat(c), init.a), f2fma(f2sub(Fp.b, F.b), f2splat(c), init.b)};
 }
 
+// The same with an increment g of rho w from the source terms: what fluxes and sources add is summed at its
+// own scale and the state rounded once (2501x1251: 83.4 -> 85.2 us a step; 8192x4096 the same).
+__device__ __forceinline__ Vars update(const Vars& init, const Vars& Fp, const Vars& F, float c, float g) {
+  Vars o = update(init, Fp, F, c);
+  o.b.x = init.b.x + fmaf(Fp.b.x - F.b.x, c, g);
+  return o;
+}
+
 // Wall halo of the column value v (ics/bcs.py:92-148): halo row h of -2, -1,
 // nz, nz + 1; hr[h] = hyc(halo row) / hyc(wall row).
 __device__ __forceinline__ Vars wall_halo(const Vars& v, const double* hr, int h) {

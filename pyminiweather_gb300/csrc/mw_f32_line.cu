@@ -148,9 +148,14 @@ __global__ void __launch_bounds__(kF32Warps * 32, 1) k_line_f32(const __grid_con
                       make_float2(__shfl_down_sync(0xffffffffu, F.b.x, 1), __shfl_down_sync(0xffffffffu, F.b.y, 1))};
       if (lane < 31 && i >= max(c0, first(s)) && i < min(c1, past(s))) {
         if (s == 0) iv = t[2];
-        Vars v = update(iv, F, G, P.k.c[s]);
-        if (DIR == MW_DIR_Z) v.b.x = fmaf(P.k.gdt[s], t[2].a.x, v.b.x);
-        if (a.srcw) v.b.x = fmaf(P.k.dt[s], sw, v.b.x);
+        Vars v;
+        if (DIR == MW_DIR_X && !a.srcw) {
+          v = update(iv, F, G, P.k.c[s]);
+        } else {
+          float g = P.k.dt[s] * sw;
+          if (DIR == MW_DIR_Z) g = fmaf(P.k.gdt[s], t[2].a.x, g);
+          v = update(iv, F, G, P.k.c[s], g);
+        }
         put<DIR>(dst, i, n, whole, v, hr);
         const bool edge = i >= p0 && i < p1 && (DIR == MW_DIR_X ? (i < kHs || i >= n - kHs) : (i == 0 || i == n - 1));
         if (edge) {
