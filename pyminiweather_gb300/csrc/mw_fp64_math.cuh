@@ -98,11 +98,11 @@ __device__ __forceinline__ void divide(const double (&a)[N], double y, unsigned 
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const double q0 = a[k] * R;
-    q[k] = fma(R, fma(-y, q0, a[k]), q0);
+    const bool zero = (__double_as_longlong(a[k]) << 1) == 0;
+    q[k] = zero ? q0 : fma(R, fma(-y, q0, a[k]), q0);  // (the correction would take the sign of a zero)
     // exponents of q and of a within [2^-900, 2^900], or a = 0 and q = 0 (integer tests)
     const unsigned eq = (unsigned)(__double_as_longlong(q[k]) >> 52) & 0x7ffu;
     const unsigned ea = (unsigned)(__double_as_longlong(a[k]) >> 52) & 0x7ffu;
-    const bool zero = (__double_as_longlong(a[k]) << 1) == 0;
     far = far || (!zero && (eq - 123u > 1800u || ea - 123u > 1800u));
   }
   if (__any_sync(mask, far)) {
