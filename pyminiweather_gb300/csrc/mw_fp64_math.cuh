@@ -89,20 +89,21 @@ __device__ __forceinline__ double rcp(double y, unsigned mask) {
 // N quotients a[k] / y in 3 FP64 operations each, for the lanes in `mask`:
 // q = a R, then q + R (a - y q), whose error before the last rounding is 2^-90
 // (so it is the correctly rounded quotient but for a few in 2^37).  Quotients
-// that leave the normal range, and divisors with no estimate, take the FP64
-// division.
+// that leave the normal range, those of -0 (the correction of a zero comes out
+// as +0) and divisors with no estimate take the FP64 division.
 template <int N>
 __device__ __forceinline__ void divide(const double (&a)[N], double y, unsigned mask, double (&q)[N]) {
   bool far;
   const double R = rcp_estimate(y, far);
+  const long long y_sign = __double_as_longlong(y) & (long long)0x8000000000000000ull;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const double q0 = a[k] * R;
-    const bool zero = (__double_as_longlong(a[k]) << 1) == 0;
-    q[k] = zero ? q0 : fma(R, fma(-y, q0, a[k]), q0);  // (the correction would take the sign of a zero)
-    // exponents of q and of a within [2^-900, 2^900], or a = 0 and q = 0 (integer tests)
+    q[k] = fma(R, fma(-y, q0, a[k]), q0);
+    // exponents of q and of a within [2^-900, 2^900], or a = 0 and a / y = +0 (integer tests)
     const unsigned eq = (unsigned)(__double_as_longlong(q[k]) >> 52) & 0x7ffu;
     const unsigned ea = (unsigned)(__double_as_longlong(a[k]) >> 52) & 0x7ffu;
+    const bool zero = __double_as_longlong(a[k]) == y_sign;
     far = far || (!zero && (eq - 123u > 1800u || ea - 123u > 1800u));
   }
   if (__any_sync(mask, far)) {
