@@ -298,36 +298,55 @@ int run_stats(int nx, int nz, double dx, double dz, const double* hyc, const dou
 
 // compute_solution_variables, post/stats.py:38-69.  Bound by the FP64 pipe: 12
 // operations per cell (ieee::divide) where the three divisions of a cell and one
-// of the row took ~60 (4096x2048: 511 us, now 257 us; HBM alone 79 us).  A
-// block takes up to kSvCells cells of a row.
-constexpr int kSvThreads = 256, kSvCells = 8 * kSvThreads;
+// of the row took ~60 (4096x2048: 511 us, now 203 us; HBM alone 79 us).  A
+// block takes up to kSvCells cells: a piece of a row, or (ROWS) as many whole
+// rows as fit, so that short rows leave no lanes idle (16x20000: 16 us, a block
+// per row 146; 100x5000: 21, 49).
+constexpr int kSvThreads = 256, kSvCells = 8 * kSvThreads, kSvRows = kSvThreads;
 
-__global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, int per_row, long long nblk,
+template <bool ROWS>
+__global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, int rows, int per_row, long long nblk,
                                                               const double* hyc, const double* hytc,
                                                               const double* state, double* out) {
+  __shared__ double s_hr[kSvRows], s_hrt[kSvRows], s_th[kSvRows];  // of the block's rows (ROWS)
   const int NX = nx + 2 * kHs;
   const long long plane = (long long)NX * (nz + 2 * kHs);
   const long long n = (long long)nx * nz;
   for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    const int k = (int)(blk / per_row), i0 = (int)(blk - (long long)k * per_row) * kSvCells;
-    const double hr = MW_AT(hyc, k + kHs, nz + 2 * kHs);
-    const double hrt[1] = {MW_AT(hytc, k + kHs, nz + 2 * kHs)};
-    double th[1];
-    ieee::divide(hrt, hr, 0xffffffffu, th);
-    for (int i = i0 + threadIdx.x; i - (int)(threadIdx.x & 31) < min(i0 + kSvCells, nx); i += kSvThreads) {
-      const bool act = i < nx;
+    const int kb = (int)(blk / per_row), k0 = kb * rows, i0 = (int)(blk - (long long)kb * per_row) * kSvCells;
+    const int nr = min(rows, nz - k0), len = min(nx - i0, kSvCells);
+    double hr, hrt[1], th[1];
+    if (!ROWS || threadIdx.x < ((nr + 31) & ~31)) {
+      const int r = ROWS ? min((int)threadIdx.x, nr - 1) : 0;
+      hr = MW_AT(hyc, k0 + r + kHs, nz + 2 * kHs);
+      hrt[0] = MW_AT(hytc, k0 + r + kHs, nz + 2 * kHs);
+      ieee::divide(hrt, hr, 0xffffffffu, th);
+    }
+    if (ROWS) {
+      __syncthreads();  // the block before has been read
+      if (threadIdx.x < nr) {
+        s_hr[threadIdx.x] = hr;
+        s_hrt[threadIdx.x] = hrt[0];
+        s_th[threadIdx.x] = th[0];
+      }
+      __syncthreads();
+    }
+    const int cells = nr * len;
+    for (int j = threadIdx.x; j - (int)(threadIdx.x & 31) < cells; j += kSvThreads) {
+      const bool act = j < cells;
       const unsigned mask = __ballot_sync(0xffffffffu, act);
       if (act) {
+        const int r = ROWS ? j / len : 0, k = k0 + r, i = i0 + j - r * len;
         const long long o = (long long)(k + kHs) * NX + i + kHs, idx = (long long)k * nx + i;
         const double d = MW_AT(state, o, 4 * plane);
         const double a[3] = {MW_AT(state, plane + o, 4 * plane), MW_AT(state, 2 * plane + o, 4 * plane),
-                             MW_AT(state, 3 * plane + o, 4 * plane) + hrt[0]};
+                             MW_AT(state, 3 * plane + o, 4 * plane) + (ROWS ? s_hrt[r] : hrt[0])};
         double q[3];
-        ieee::divide(a, hr + d, mask, q);
+        ieee::divide(a, (ROWS ? s_hr[r] : hr) + d, mask, q);
         MW_AT(out, idx, 4 * n) = d;
         MW_AT(out, n + idx, 4 * n) = q[0];
         MW_AT(out, 2 * n + idx, 4 * n) = q[1];
-        MW_AT(out, 3 * n + idx, 4 * n) = q[2] - th[0];
+        MW_AT(out, 3 * n + idx, 4 * n) = q[2] - (ROWS ? s_th[r] : th[0]);
       }
     }
   }
@@ -597,10 +616,13 @@ extern "C" int mw_solution_variables_f64(int nx, int nz, const double* hyc, cons
   if (st) return st;
   MW_REQUIRE(hyc && hytc && state && out, MW_ERR_INVALID_ARG, "NULL pointer argument");
   MW_REQUIRE(aligned(hyc) && aligned(hytc) && aligned(state) && aligned(out), MW_ERR_ALIGN, "misaligned pointer");
-  const int per_row = (nx + kSvCells - 1) / kSvCells;
-  const long long nblk = (long long)per_row * nz;
-  k_solution_vars<<<(unsigned)std::min(nblk, 1LL << 20), kSvThreads, 0, (cudaStream_t)stream>>>(nx, nz, per_row, nblk,
-                                                                                              hyc, hytc, state, out);
+  // blocks of whole rows, or pieces of one; fewer rows where the blocks would not fill the SMs
+  const long long fit = std::min<long long>({kSvCells / nx, kSvRows, nz / (2LL * 152)});
+  const int rows = (int)std::max(1LL, fit), per_row = (nx + kSvCells - 1) / kSvCells;
+  const long long nblk = (long long)per_row * ((nz + rows - 1) / rows);
+  auto kern = rows > 1 ? k_solution_vars<true> : k_solution_vars<false>;
+  kern<<<(unsigned)std::min(nblk, 1LL << 20), kSvThreads, 0, (cudaStream_t)stream>>>(nx, nz, rows, per_row, nblk, hyc,
+                                                                                     hytc, state, out);
   return check_launch("solution variables launch");
 }
 
