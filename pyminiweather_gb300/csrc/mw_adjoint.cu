@@ -50,7 +50,8 @@ struct VjpArgs {
   double* gdst;
   double* ws;       // 8 x n_interfaces: Abar[4], Dbar[4]
   long long nif;    // interfaces per variable plane of ws
-  double kc, ke;    // the gather's factors of the transposed interpolation (of 12 x it, over 12) and third difference
+  double kc, ke;    // IEEE form: the gather's factors of the transposed interpolation (of 12 x it, over 12) and third
+                    // difference, which its interface adjoints do not carry
 };
 
 __device__ __forceinline__ int wrap_x(int j, int nx) { return j < 0 ? j + nx : (j >= nx ? j - nx : j); }
@@ -165,7 +166,7 @@ template <int DIR>
 __device__ __forceinline__ void gather_general(const VjpArgs& a, int k, int i, double acc[4]) {
   const long long n = a.nif;
   auto tap = [&](int q, int j, long long o) {
-    return a.kc * (kC[j] * MW_WS(a, q * n + o)) + a.ke * (kE[j] * MW_WS(a, (4 + q) * n + o));
+    return kC[j] * MW_WS(a, q * n + o) + kE[j] * MW_WS(a, (4 + q) * n + o);
   };
   if (DIR == MW_DIR_X) {
     for (int j = 0; j < 4; ++j)
@@ -242,9 +243,9 @@ __global__ void __launch_bounds__(128) k_vjp_gather(VjpArgs a) {
         const double D2 = MW_WS(a, (4 + q) * n + o0 + 2 * st), D3 = MW_WS(a, (4 + q) * n + o0 + 3 * st);
         // cell i is tap j of interface f = i + 2 - j, so kC = (-1, 7, 7, -1) / 12 and
         // kE = (-1, 3, -3, 1) act on the interfaces i + 2, i + 1, i, i - 1 = (A3, A2, A1, A0)
-        const double ca = fma(7.0, A1 + A2, -(A0 + A3));
+        const double ca = fma(7.0, A1 + A2, -(A0 + A3)) * (1.0 / 12.0);
         const double ce = fma(3.0, D2 - D1, D0 - D3);
-        acc[q] = fma(a.kc * (1.0 / 12.0), ca, a.ke * ce);
+        acc[q] = ca + ce;
       }
     } else {
       gather_general<DIR>(a, k, i, acc);
@@ -441,7 +442,6 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
 // A CTA takes 32 columns of up to kFZRows rows.  Its warps first compute the
 // tile's rows + 3 interface adjoints, each warp a stretch of consecutive
 // interfaces down its 32 columns (the four taps and g move along in
-// registers, one new row of each per interface), into shared memory; then,
 // registers, one new row of each per interface), into shared memory; then,
 // after the one barrier, each gathers a stretch of rows the same way (one new
 // interface per row).
@@ -707,9 +707,9 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
   a.gdst = g_dst;
   a.ws = (double*)workspace;
   a.nif = n_interfaces(nx, nz, direction);
-  const bool ieee = f64_mode == MW_F64_IEEE;  // its interface adjoints carry no factors
-  a.kc = ieee ? dt_stage / a.d : 1.0;
-  a.ke = ieee ? -a.hv * a.kc : 1.0;
+  const bool ieee = f64_mode == MW_F64_IEEE;
+  a.kc = dt_stage / a.d;
+  a.ke = -a.hv * a.kc;
   cudaStream_t s = (cudaStream_t)stream;
   RowV* rows = (RowV*)((double*)workspace + ieee_rows_off(nx, nz));
   // Every launch of the call but its first may come in while the one before it ends (each waits before it touches
