@@ -361,20 +361,6 @@ struct SmemFX {
   double db[kFXWarps][4][32];     // Db
 };
 
-// g_dst's halo cells: zero (its rows strided over the CTAs of the launch).
-__device__ __forceinline__ void zero_frame(const VjpArgs& a) {
-  const int rows = a.nz + 2 * kHs;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const bool all = r < kHs || r >= a.nz + kHs;  // a halo row, or the halo columns of an interior one
-    const int n = all ? a.pitch : 2 * kHs;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      const long long o = (long long)r * a.pitch + (all || t < kHs ? t : a.nx + t);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) MW_AT(a.gdst, q * a.plane + o, 4 * a.plane) = 0.0;
-    }
-  }
-}
-
 // The transposed taps of interface adjoints A0 .. A3, D0 .. D3 (interfaces i - 1 .. i + 2) on cell i.
 __device__ __forceinline__ double gather4(const VjpArgs& a, double A0, double A1, double A2, double A3, double D0,
                                           double D1, double D2, double D3) {
@@ -435,7 +421,7 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
     }
     __syncwarp();
   }
-  zero_frame(a);
+  zero_frame(a.gdst, a.nx, a.nz, a.plane);
 }
 
 // ---- IEEE-FP64 stage adjoint, z: one kernel ---------------------------------
@@ -582,7 +568,7 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
     }
     __syncthreads();
   }
-  zero_frame(a);
+  zero_frame(a.gdst, a.nx, a.nz, a.plane);
 }
 
 // Rows of a tile of k_vjp_ieee_z: those with the fewest rounds of a warp's work,

@@ -308,20 +308,6 @@ __device__ __forceinline__ void vjp_segments(const VjpSplitArgs& a, int nseg, lo
   }
 }
 
-// g_dst's halo cells: zero (its rows strided over the CTAs of the launch).
-__device__ __forceinline__ void zero_frame(const VjpSplitArgs& a) {
-  const int rows = a.nz + 2 * kHs;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const bool all = r < kHs || r >= a.nz + kHs;  // a halo row, or the halo columns of an interior one
-    const int n = all ? a.pitch : 2 * kHs;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      const long long o = (long long)r * a.pitch + (all || t < kHs ? t : a.nx + t);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) MW_AT(a.gdst, q * a.plane + o, 4 * a.plane) = 0.0;
-    }
-  }
-}
-
 // Launched for the x direction (rows are contiguous); the z direction runs
 // k_vjp_split_zt below, which applies the same per-line computation to
 // shared-memory tiles.
@@ -333,7 +319,7 @@ __global__ void __launch_bounds__(kVThreads) k_vjp_split(VjpSplitArgs a, int nse
   const int w = threadIdx.x >> 5;
   const long long n = g1 - g0;
   vjp_segments<DIR>(a, nseg, g0 + n * w / kVWarps, g0 + n * (w + 1) / kVWarps, sm);
-  zero_frame(a);
+  zero_frame(a.gdst, a.nx, a.nz, a.plane);
 }
 
 // z, tiled: the z lines are columns, so a warp walking one column directly
@@ -473,7 +459,7 @@ __global__ void __launch_bounds__(kZTThreads) k_vjp_split_zt(VjpSplitArgs a, int
     }
     __syncthreads();  // the tiles are rewritten by the next item
   }
-  zero_frame(a);
+  zero_frame(a.gdst, a.nx, a.nz, a.plane);
 }
 
 int vjp_resident_ctas(int* out) {

@@ -1,0 +1,67 @@
+"""Grids of a few columns, a few rows or many more of one than of the other: the
+kernels' other shapes of work, and that a call's time follows its cells.
+
+Times are the least of ten, compared within one process with those of a square
+grid of as many cells; the bounds leave a factor of about two over what was
+measured, and are as much below what the shapes took before."""
+import pytest
+import torch
+
+from pyminiweather_gb300 import _native
+from pyminiweather_gb300.data import initialize_fields
+from pyminiweather_gb300.ics import init
+from tests.helpers import make_params
+from tests.test_gpu_short_rows import us
+
+pytestmark = pytest.mark.gpu
+
+
+def developed(nx, nz):
+    p = make_params(nx, nz, "collision")
+    f = initialize_fields(p)
+    init(f, p)
+    gen = torch.Generator(device=f.device).manual_seed(nx * 7 + nz)
+    noise = torch.randn(f.shape, generator=gen, device=f.device, dtype=torch.float64)
+    f.state += noise * torch.tensor([1e-3, 5.0, 2.0, 0.5], device=f.device, dtype=torch.float64)[:, None, None]
+    return p, f
+
+
+class Vjp:
+    """The adjoint of one stage at a developed state."""
+
+    def __init__(self, nx, nz):
+        self.p, self.f = developed(nx, nz)
+        self.g = torch.zeros_like(self.f.state)
+        gen = torch.Generator(device=self.g.device).manual_seed(nx * 1000 + nz)
+        self.g[:, 2:-2, 2:-2] = torch.randn(4, nz, nx, generator=gen, dtype=torch.float64, device=self.g.device)
+        n = int(_native.load().mw_dirstage_vjp_workspace_bytes(nx, nz))
+        self.ws = torch.empty(n // 8 + 1, dtype=torch.float64, device=self.g.device)
+        self.out = torch.empty_like(self.g)
+
+    def __call__(self, mode, direction):
+        p, f = self.p, self.f
+        _native.call("mw_dirstage_vjp_f64", f.nx, f.nz, p["dx"], p["dz"], p["dt"],
+                     *[_native.ptr(a) for a in f.backgrounds()], _native.ptr(f.state), _native.ptr(self.g), None, None,
+                     0, _native.ptr(self.out), p["dt"] / 2, direction, _native.F64_MODES[mode], _native.ptr(self.ws),
+                     self.ws.numel() * 8, _native.stream_handle())
+        return self.out
+
+
+def frame_max(a):
+    a = a.clone()
+    a[:, 2:-2, 2:-2] = 0.0
+    return float(a.abs().max())
+
+
+@pytest.mark.parametrize("mode", ("split", "fp64"))
+@pytest.mark.parametrize("nx,nz", [(2, 1), (2, 300), (3, 2), (300, 2), (4097, 1), (70001, 3), (130, 70)])
+def test_adjoint_clears_the_halo(nx, nz, mode):
+    v = Vjp(nx, nz)
+    for direction in (0, 1):
+        v.out.fill_(7.0)
+        assert frame_max(v(mode, direction)) == 0.0, direction
+
+
+def test_adjoint_of_long_rows_takes_the_time_of_its_cells():
+    long, square = Vjp(3000000, 2), Vjp(3000, 2000)  # 398 us against 377; a CTA to a halo row 1640
+    assert us(lambda: long("split", 0)) <= 2.0 * us(lambda: square("split", 0))
