@@ -425,12 +425,12 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
 }
 
 // ---- IEEE-FP64 stage adjoint, z: one kernel ---------------------------------
-// A CTA takes 32 columns of up to kFZRows rows.  Its warps first compute the
-// tile's rows + 3 interface adjoints, each warp a stretch of consecutive
-// interfaces down its 32 columns (the four taps and g move along in
-// registers, one new row of each per interface), into shared memory; then,
-// after the one barrier, each gathers a stretch of rows the same way (one new
-// interface per row).
+// A CTA takes 2^LC columns (32; fewer on narrow grids, more on flat ones) of up
+// to fz_max_rows(LC) rows.  Its threads, 2^LC to a stretch, first compute the
+// tile's rows + 3 interface adjoints, each a stretch of consecutive interfaces
+// down its column (the four taps and g move along in registers, one new row of
+// each per interface), into shared memory; then, after the one barrier, each
+// gathers a stretch of rows the same way (one new interface per row).
 //
 // Bound: FP64 (512 x 256, a stage without bases: 2375 instructions on the
 // fullest SM at 16 cycles each, 38000 of its 53500 active cycles; the rest is
@@ -439,13 +439,16 @@ __global__ void __launch_bounds__(kFXThreads) k_vjp_ieee_x(VjpArgs a, const RowV
 // the interface adjoints and the gather as two kernels with the 8 values per
 // interface in memory between them.  Sixteen warps a CTA: 33 us.  Rows read
 // one interface ahead: no gain.
-constexpr int kFZRows = 29;  // 32 interfaces: 64 KB of shared memory
 constexpr int kFZThreads = 256;
 constexpr int kFZWarps = kFZThreads / 32;
 
-inline int fz_smem(int rows) { return (int)sizeof(double) * 8 * 32 * (rows + 3); }
+// 64 KB of shared memory: 32 interfaces of 32 columns
+__host__ __device__ constexpr int fz_max_rows(int lc) { return (1024 >> lc) - 3; }
+static_assert(fz_max_rows(7) >= 5, "the widest tile");
+inline int fz_smem(int rows, int lc) { return ((int)sizeof(double) * 8 * (rows + 3)) << lc; }
 
 // The wall rule's halo taps on row k (0 or nz - 1, or both): halo row t passes weight wq of its adjoint to row `src`.
+template <int C>
 __device__ __forceinline__ void gather_wall(const VjpArgs& a, const double* ws, int f0, int k, double acc[4]) {
   for (int t = -2; t <= a.nz + 1; t = t == -1 ? a.nz : t + 1) {
     const int src = t < 0 ? 0 : a.nz - 1;
@@ -454,10 +457,10 @@ __device__ __forceinline__ void gather_wall(const VjpArgs& a, const double* ws, 
     for (int j = 0; j < 4; ++j) {
       const int f = t + 2 - j;
       if (f < 0 || f > a.nz) continue;
-      const double* c = ws + (f - f0) * 256;
+      const double* c = ws + (f - f0) * 8 * C;
       for (int q = 0; q < 4; ++q) {
         if (q == WMOM) continue;
-        acc[q] += (q == UMOM ? wu : 1.0) * (a.kc * (kC[j] * c[q * 32]) + a.ke * (kE[j] * c[(4 + q) * 32]));
+        acc[q] += (q == UMOM ? wu : 1.0) * (a.kc * (kC[j] * c[q * C]) + a.ke * (kE[j] * c[(4 + q) * C]));
       }
     }
   }
@@ -483,22 +486,27 @@ __device__ __forceinline__ void store_cell(const VjpArgs& a, long long o, const 
   for (int q = 0; q < 4; ++q) store_value(a, q * a.plane + o, acc[q]);
 }
 
+template <int LC>
 __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV* rows, int tile_rows) {
   extern __shared__ double fz_ws[];  // [interface][Ab 0..3, Db 0..3][column]
+  constexpr int C = 1 << LC, S = kFZWarps * 32 / C;  // columns and stretches of a tile
   overlap_wait();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nxt = (a.nx + 31) / 32, nzt = (a.nz + tile_rows - 1) / tile_rows;
+  const int lane = threadIdx.x & (C - 1), w = threadIdx.x >> LC;  // column and stretch of the thread
+  const int nxt = (a.nx + C - 1) / C, nzt = (a.nz + tile_rows - 1) / tile_rows;
   for (long long tile = blockIdx.x; tile < (long long)nxt * nzt; tile += gridDim.x) {
     const int k0 = (int)(tile / nxt) * tile_rows, k1 = min(a.nz, k0 + tile_rows);
-    const int c = (int)(tile % nxt) * 32 + lane;
+    const int c = (int)(tile % nxt) * C + lane;
     const bool in = c < a.nx;
     const int col = min(c, a.nx - 1) + kHs;  // columns past the grid repeat the last one and are not stored
     const int fa = max(0, k0 - 1), fb = min(a.nz, k1 + 1);  // interfaces fa .. fb
     double* ws = fz_ws + lane;
     {
-      const int n = fb - fa + 1, f0 = fa + n * w / kFZWarps, f1 = fa + n * (w + 1) / kFZWarps;
+      const int n = fb - fa + 1, f0 = fa + n * w / S, f1 = fa + n * (w + 1) / S;
+      // the lanes of a warp go together: a stretch that is one interface shorter, or empty, ends on one that is not its
+      // own (and not stored)
+      const int end = LC >= 5 ? f1 : f0 + (n + S - 1) / S;
       double s[4][4], gl[4];
-      if (f0 < f1) {
+      if (f0 < end) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
 #pragma unroll
@@ -506,7 +514,8 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
           gl[q] = f0 > 0 ? gval(a, q, f0 - 1, col - kHs) : 0.0;
         }
       }
-      for (int f = f0; f < f1; ++f) {
+      for (int i = f0; i < end; ++i) {
+        const int f = LC >= 5 ? i : min(i, fb);
         double dg[4], Ab[4], Db[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -520,26 +529,28 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
         }
         const RowV rv = MW_AT(rows, a.nz + 2 * kHs + f, 2 * a.nz + 5);
         jt_ieee<MW_DIR_Z>(s, dg, rv, f == 0 || f == a.nz, 0xffffffffu, Ab, Db);
-        double* o = ws + (f - fa) * 256;
+        if (LC >= 5 || i < f1) {
+          double* o = ws + (f - fa) * 8 * C;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          o[q * 32] = Ab[q];
-          o[(4 + q) * 32] = Db[q];
+          for (int q = 0; q < 4; ++q) {
+            o[q * C] = Ab[q];
+            o[(4 + q) * C] = Db[q];
+          }
         }
       }
     }
     __syncthreads();
     {
-      const int n = k1 - k0, r0 = k0 + n * w / kFZWarps, r1 = k0 + n * (w + 1) / kFZWarps;
+      const int n = k1 - k0, r0 = k0 + n * w / S, r1 = k0 + n * (w + 1) / S;
       double A[4][4], D[4][4];
       // interface f of the tile; one outside [0, nz] has no adjoint
       auto load = [&](int f, int j) {
         const bool has = f >= 0 && f <= a.nz;
-        const double* p = ws + (f - fa) * 256;
+        const double* p = ws + (f - fa) * 8 * C;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          A[q][j] = has ? p[q * 32] : 0.0;
-          D[q][j] = has ? p[(4 + q) * 32] : 0.0;
+          A[q][j] = has ? p[q * C] : 0.0;
+          D[q][j] = has ? p[(4 + q) * C] : 0.0;
         }
       };
       if (r0 < r1) {
@@ -561,7 +572,7 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           acc[q] = gather4(a, A[q][0], A[q][1], A[q][2], A[q][3], D[q][0], D[q][1], D[q][2], D[q][3]);
-        if (k == 0 || k == a.nz - 1) gather_wall(a, ws, fa, k, acc);
+        if (k == 0 || k == a.nz - 1) gather_wall<C>(a, ws, fa, k, acc);
         acc[DENS] = fma(-a.dt_stage * kGrav, gval(a, WMOM, k, col - kHs), acc[DENS]);
         if (in) store_cell(a, o, acc);
       }
@@ -571,22 +582,35 @@ __global__ void __launch_bounds__(kFZThreads) k_vjp_ieee_z(VjpArgs a, const RowV
   zero_frame(a.gdst, a.nx, a.nz, a.plane);
 }
 
-// Rows of a tile of k_vjp_ieee_z: those with the fewest rounds of a warp's work,
-// interfaces and rows counted alike (about 40 FP64 operations each) and one
-// more per tile for its loads, on the SM with the most tiles; of equals the
-// tallest, which recompute the fewest interfaces.  512 x 256: 29 rows, 144 tiles,
-// 29.7 us.  From a third to twice the charge per tile: the same times within 1 %
-// from 100 x 50 to 640 x 448.
-inline int fz_rows(int nx, int nz, int sms) {
-  const long long nxt = (nx + 31) / 32;
-  int best = std::min(nz, kFZRows);
+// Columns (log2) and rows of a tile of k_vjp_ieee_z: those with the fewest rounds
+// of a warp's work, interfaces and rows counted alike (about 40 FP64 operations
+// each) and one more per tile for its loads, on the SM with the most tiles; of
+// equals the tallest, which recompute the fewest interfaces.  512 x 256: 29 rows,
+// 144 tiles, 29.7 us.  From a third to twice the charge per tile: the same times
+// within 1 % from 100 x 50 to 640 x 448.  Grids of fewer than 256 columns, where
+// tiles of 32 may leave a good part of the lanes idle, may take narrower tiles
+// (a stage, us in tiles of 32 and as chosen: 8x20000 145, 64; 2x100000 594, 78;
+// 66x9000 189, 153), grids of fewer rows than warps wider ones (3000000x2 2950, 2170).
+struct FzTile {
+  int lc, rows;
+};
+inline FzTile fz_tile(int nx, int nz, int sms) {
+  FzTile best = {5, std::min(nz, fz_max_rows(5))};
   double cost = 0;
-  for (int r = 1; r <= std::min(nz, kFZRows); ++r) {
-    const long long nzt = (nz + r - 1) / r, per_sm = (nxt * nzt + sms - 1) / sms;
-    const double c = per_sm * ((r + 3 + 7) / 8 + (r + 7) / 8 + 1.0);
-    if (r == 1 || c <= cost) {
-      cost = c;
-      best = r;
+  const int widths[] = {5, 4, 3, 2, 1, 6, 7};
+  for (const int lc : widths) {
+    if (lc < 5 ? nx >= 256 : lc > 5 && nz >= kFZWarps) continue;
+    const long long nxt = (nx + (1 << lc) - 1) >> lc;
+    const int S = kFZWarps * 32 >> lc, step = lc >= 5 ? 1 : S, most = std::min(nz, fz_max_rows(lc));
+    // rows such that rows + 3 interfaces are whole rounds of the stretches
+    for (int r = lc >= 5 ? 1 : std::min(S - 3, most); r <= most; r += step) {
+      const long long nzt = (nz + r - 1) / r, per_sm = (nxt * nzt + sms - 1) / sms;
+      const double c = per_sm * ((std::min(r + 3, nz + 1) + S - 1) / S + (r + S - 1) / S + 1.0);
+      // the tallest of a width; another width only for a clear gain
+      if (cost == 0 || (lc == best.lc ? c <= cost : c < 0.9 * cost)) {
+        cost = c;
+        best = {lc, r};
+      }
     }
   }
   return best;
@@ -722,13 +746,20 @@ static int vjp_stage(int nx, int nz, double dx, double dz, double dt_full, const
     int sms = 0, dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const FzTile t = fz_tile(nx, nz, sms);
+    const auto kern = t.lc == 5   ? k_vjp_ieee_z<5>
+                      : t.lc == 7 ? k_vjp_ieee_z<7>
+                      : t.lc == 6 ? k_vjp_ieee_z<6>
+                      : t.lc == 4 ? k_vjp_ieee_z<4>
+                      : t.lc == 3 ? k_vjp_ieee_z<3>
+                      : t.lc == 2 ? k_vjp_ieee_z<2>
+                                  : k_vjp_ieee_z<1>;
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_vjp_ieee_z, cudaFuncAttributeMaxDynamicSharedMemorySize, fz_smem(kFZRows));
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fz_smem(fz_max_rows(t.lc), t.lc));
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "vjp setup: %s", cudaGetErrorString(e));
-    const int tile_rows = fz_rows(nx, nz, sms);
-    const long long tiles = (long long)((nx + 31) / 32) * ((nz + tile_rows - 1) / tile_rows);
-    return launch_overlapping(k_vjp_ieee_z, dim3((unsigned)std::min(tiles, 1LL << 30)), kFZThreads, fz_smem(tile_rows), s,
-                              follows, "vjp", a, rows, tile_rows);
+    const long long tiles = (long long)((nx + (1 << t.lc) - 1) >> t.lc) * ((nz + t.rows - 1) / t.rows);
+    return launch_overlapping(kern, dim3((unsigned)std::min(tiles, 1LL << 30)), kFZThreads, fz_smem(t.rows, t.lc), s,
+                              follows, "vjp", a, rows, t.rows);
   }
   st = launch_overlapping(direction == MW_DIR_X ? k_vjp_iface<MW_DIR_X> : k_vjp_iface<MW_DIR_Z>,
                           dim3(grid_for(a.nif, 128)), 128, 0, s, follows, "vjp interface", a);

@@ -65,3 +65,23 @@ def test_adjoint_clears_the_halo(nx, nz, mode):
 def test_adjoint_of_long_rows_takes_the_time_of_its_cells():
     long, square = Vjp(3000000, 2), Vjp(3000, 2000)  # 398 us against 377; a CTA to a halo row 1640
     assert us(lambda: long("split", 0)) <= 2.0 * us(lambda: square("split", 0))
+
+
+# widths and rows of a tile: 2 to 32 columns of narrow grids, 64 and 128 of flat ones; whole, cut and single-row tiles,
+# stretches with an interface less and without any
+@pytest.mark.parametrize("nx,nz", [(2, 1), (2, 3), (2, 509), (2, 510), (2, 4000), (3, 1100), (5, 70), (7, 253), (8, 125),
+                                   (9, 126), (15, 1000), (16, 61), (17, 62), (40, 700), (66, 900), (100, 500), (255, 200),
+                                   (4000, 1), (5000, 2), (3001, 5), (70000, 6), (3000, 7), (3000, 8)])
+def test_adjoint_z_tiles(nx, nz):
+    """Against the adjoint of the reference's formulas, to the bound derived in test_gpu_adjoint_tiles.py."""
+    v = Vjp(nx, nz)
+    ref, got = v("native", 1).clone(), v("fp64", 1)
+    for q in range(4):
+        err = float((got[q] - ref[q]).abs().max() / ref[q].abs().max().clamp_min(1e-300))
+        assert err <= 1e-13, (q, err)
+    assert frame_max(got) == 0.0
+
+
+def test_adjoint_of_few_columns_takes_the_time_of_its_cells():
+    narrow, square = Vjp(2, 100000), Vjp(500, 400)  # 78 us against 60; in tiles of 32 columns 594
+    assert us(lambda: narrow("fp64", 1)) <= 3.0 * us(lambda: square("fp64", 1))
