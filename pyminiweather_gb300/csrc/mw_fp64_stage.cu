@@ -124,11 +124,13 @@ __device__ __forceinline__ void write_z_halo_column(const Args& a, int col, bool
 // next block are loaded one block ahead.
 constexpr int kWSlots = 64;         // slots per block
 constexpr int kXWarps = kXT / 32;
-constexpr int kXRowsMax = kXWarps;  // rows of one CTA's runs
+constexpr int kXShortBlocks = 8;    // most blocks of a run of the kernel that leaves out empty halves
+constexpr int kXRunsMax = 4;        // most runs per warp of that kernel
 struct SmemXW {
   double sS[kXWarps][4][kWSlots + 2];  // [warp][variable][cell i0-1 .. i0+64], i0 the cell of slot 0
 };
 __host__ __device__ inline int run_blocks(int cells) { return (cells + 2 + kWSlots - 1) / kWSlots; }
+inline int run_halves(int cells) { return (cells + 2 + kWSlots / 2 - 1) / (kWSlots / 2); }
 
 // Walks runs [g0, g1) of the row-major list of runs of `len` cells (nrun per
 // row); row_at(k) gives the constants of row k.  Every lane of the warp calls
@@ -262,16 +264,20 @@ __device__ __forceinline__ void x_warp_walk(const Args& a, int nrun, int len, lo
 #ifndef MW_IEEE_X_MIN_BLOCKS
 #define MW_IEEE_X_MIN_BLOCKS 2
 #endif
-// Single grid: one run per warp, eight consecutive runs of rows [r0, r1) per
-// CTA; the row constants (an FP64 pow per row) are tabled once per CTA while
-// the warps' first loads are in flight.
-__global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Args a, int nrun, int len, long long g0,
-                                                                               long long g1) {
+// Single grid: consecutive runs of rows [r0, r1), one per warp (SHORT: up to
+// kXRunsMax); the row constants (an FP64 power per row) are tabled once per CTA
+// while the warps' first loads are in flight.  SHORT (x_warp_walk): rows of up to
+// kXShortBlocks blocks whose runs end in the first half of one (a stage, 66x9000:
+// 123 us with the empty halves, 103).
+template <bool SHORT>
+__global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Args a, int nrun, int len, int per_warp,
+                                                                               long long g0, long long g1) {
   __shared__ SmemXW sm;
-  __shared__ RowP rows[kXRowsMax];
+  __shared__ RowP rows[kXWarps * (SHORT ? kXRunsMax : 1)];
   __shared__ PowTables pow_tables;
-  const long long b0 = g0 + (long long)blockIdx.x * kXWarps, b1 = min(b0 + kXWarps, g1);
-  const int row0 = (int)(b0 / nrun), nrows = (int)((b1 - 1) / nrun) - row0 + 1;  // nrows <= kXRowsMax
+  if (!SHORT) per_warp = 1;
+  const long long b0 = g0 + (long long)blockIdx.x * kXWarps * per_warp, b1 = min(b0 + kXWarps * per_warp, g1);
+  const int row0 = (int)(b0 / nrun), nrows = (int)((b1 - 1) / nrun) - row0 + 1;  // at most one per run
   const int w = threadIdx.x >> 5;
   auto table = [&]() {
     load_pow_tables(pow_tables);
@@ -287,10 +293,10 @@ __global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Ar
   const bool early = a.flags & kFlagOverlap;
   if (early) table();
   overlap_wait();
-  x_warp_walk<false>(a, nrun, len, min(b0 + w, b1), min(b0 + w + 1, b1), [&](int k) -> const RowP& { return rows[k - row0]; },
-              a.flags & MW_FLAG_WRITE_HALO, sm.sS[w], [&]() {
-                if (!early) table();
-              });
+  x_warp_walk<SHORT>(a, nrun, len, min(b0 + w * per_warp, b1), min(b0 + (w + 1) * per_warp, b1),
+                     [&](int k) -> const RowP& { return rows[k - row0]; }, a.flags & MW_FLAG_WRITE_HALO, sm.sS[w], [&]() {
+                       if (!early) table();
+                     });
 }
 
 // ---- z ---------------------------------------------------------------------
@@ -470,7 +476,7 @@ int resident_ctas(int which, int* out) {
   const bool cached = dev >= 0 && dev < 64;
   if (cached && (*out = cache[which][dev].load(std::memory_order_relaxed)) > 0) return MW_OK;
   int per_sm = 0, sms = 0;
-  cudaError_t e = which == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_x_ieee_w, kXT, 0)
+  cudaError_t e = which == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_x_ieee_w<false>, kXT, 0)
                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_z_ieee, kZT, 0);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return fail(MW_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
@@ -562,6 +568,8 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     // start a run), and an SM's partitions each take two warps of every CTA it
     // gets, so the row is cut where ceil(CTAs / SMs) x (blocks + 1/3) is least
     // -- at most kXRunBlocksMax blocks, which leaves a large grid several waves.
+    // A last block's empty half counts only where it is not left out, or where
+    // the launch is too small for its operations to matter.
     int resident = 0, st = resident_ctas(0, &resident);
     if (st) return st;
     const long long sms = std::max(1, resident / MW_IEEE_X_MIN_BLOCKS);
@@ -569,9 +577,11 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     double best = 0.0;
     const int least = (int)(((long long)nx + kXRunBlocksMax * kWSlots - 1) / (kXRunBlocksMax * kWSlots));
     const int most = (int)(((long long)nx + kWSlots - 3) / (kWSlots - 2));
-    for (int n = least; n <= most; n += std::max(1, n / 32)) {
-      const int blocks = run_blocks((nx + n - 1) / n);
+    const bool shortable = run_blocks(nx) <= kXShortBlocks;
+    for (int n = least; n <= most; n = n == most ? n + 1 : std::min(most, n + std::max(1, n / 32))) {
+      const int cells = (nx + n - 1) / n;
       const long long ctas = ((long long)n * rows + kXWarps - 1) / kXWarps;
+      const double blocks = shortable && ctas > 2 * sms ? run_halves(cells) / 2.0 : run_blocks(cells);
       const double cost = (double)((ctas + sms - 1) / sms) * (blocks + 1.0 / 3);
       if (best == 0.0 || cost < best) {
         best = cost;
@@ -581,10 +591,16 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
     const int len = (nx + nrun - 1) / nrun;
     nrun = (nx + len - 1) / len;
     const long long g0 = (long long)r0 * nrun, g1 = (long long)r1 * nrun;
-    const long long grid = (g1 - g0 + kXWarps - 1) / kXWarps;
+    const bool odd = shortable && run_halves(len) % 2 == 1;
+    // Rows of half a block or less: the table of their constants takes about as long as their cells, and no longer for
+    // 32 rows than for 8 (2x2000000, a stage: 8.7 ms, 5.8).
+    const int per_warp = odd && run_halves(len) == 1
+                             ? (int)std::min<long long>(kXRunsMax, std::max<long long>(1, (g1 - g0) / (kXWarps * resident)))
+                             : 1;
+    const long long grid = (g1 - g0 + kXWarps * per_warp - 1) / (kXWarps * per_warp);
     MW_REQUIRE(grid <= 0x7fffffffLL, MW_ERR_SHAPE, "grid too large for the x direction-stage launch");
-    return launch_overlapping(k_stage_x_ieee_w, dim3((unsigned)grid), kXT, 0, stream, flags & kFlagOverlap,
-                              "x IEEE-FP64 direction-stage", a, nrun, len, g0, g1);
+    return launch_overlapping(odd ? k_stage_x_ieee_w<true> : k_stage_x_ieee_w<false>, dim3((unsigned)grid), kXT, 0,
+                              stream, flags & kFlagOverlap, "x IEEE-FP64 direction-stage", a, nrun, len, per_warp, g0, g1);
   } else {
     const int ntiles = (rows + a.z_tile - 1) / a.z_tile;
     for (int t0 = 0; t0 < ntiles; t0 += 65535) {

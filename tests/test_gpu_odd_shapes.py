@@ -85,3 +85,34 @@ def test_adjoint_z_tiles(nx, nz):
 def test_adjoint_of_few_columns_takes_the_time_of_its_cells():
     narrow, square = Vjp(2, 100000), Vjp(500, 400)  # 78 us against 60; in tiles of 32 columns 594
     assert us(lambda: narrow("fp64", 1)) <= 3.0 * us(lambda: square("fp64", 1))
+
+
+def stage(p, f, mode, direction=0):
+    out = torch.zeros_like(f.state)
+    _native.call("mw_dirstage_f64", f.nx, f.nz, p["dx"], p["dz"], p["dt"], *[_native.ptr(a) for a in f.backgrounds()],
+                 None, _native.ptr(f.state), _native.ptr(f.state), _native.ptr(out), p["dt"] / 2, direction,
+                 _native.F64_MODES[mode], 0, _native.stream_handle())
+    return out
+
+
+# runs that end in the first and in the second half of a block, of one to nine blocks; one to four runs a warp, whose
+# rows end within and with a CTA; rows that are cut into as many runs as there can be
+@pytest.mark.parametrize("nx,nz", [(2, 1), (2, 9), (2, 40001), (5, 20003), (29, 9731), (30, 9730), (31, 9729), (62, 40),
+                                   (66, 9000), (94, 5000), (95, 5001), (200, 3000), (257, 2000), (478, 1300), (510, 700),
+                                   (511, 700), (542, 700), (4000, 16), (20000, 2)])
+def test_x_stage(nx, nz):
+    """The IEEE x stage against the reference's formulas.  A stage adds to a state increments whose terms are sums of
+    at most a few dozen rounded operations on values up to (7 + 7 + 1 + 1) / 12 of the state's or the pressure's range
+    (test_gpu_fp64_runs.py, which states the bar of 1e-12 for one stage)."""
+    p, f = developed(nx, nz)
+    ref, got = stage(p, f, "native"), stage(p, f, "fp64")
+    for q in range(4):
+        a, b = got[q, 2:-2, 2:-2], ref[q, 2:-2, 2:-2]
+        assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max()), q
+
+
+def test_x_stage_of_short_rows_takes_the_time_of_its_slots():
+    # rows of 30 + 2 slots of 32 that a warp's instruction takes, against 62 + 2: 675 us against 1404, in blocks of 64
+    # slots always 1246
+    short, full = developed(30, 200000), developed(62, 200000)
+    assert us(lambda: stage(*short, "fp64")) <= 0.7 * us(lambda: stage(*full, "fp64"))
