@@ -301,11 +301,12 @@ int run_stats(int nx, int nz, double dx, double dz, const double* hyc, const dou
 // of the row took ~60 (4096x2048: 511 us, now 203 us; HBM alone 79 us).  A
 // block takes up to kSvCells cells: a piece of a row, or (ROWS) as many whole
 // rows as fit, so that short rows leave no lanes idle (16x20000: 16 us, a block
-// per row 146; 100x5000: 21, 49).
+// per row 146; 100x5000: 21, 49), and fewer where that gives the SMs less than
+// two blocks each (4000x16, with the call: 27 us in pieces of 2048, 23).
 constexpr int kSvThreads = 256, kSvCells = 8 * kSvThreads, kSvRows = kSvThreads;
 
 template <bool ROWS>
-__global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, int rows, int per_row, long long nblk,
+__global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, int rows, int piece, int per_row, long long nblk,
                                                               const double* hyc, const double* hytc,
                                                               const double* state, double* out) {
   __shared__ double s_hr[kSvRows], s_hrt[kSvRows], s_th[kSvRows];  // of the block's rows (ROWS)
@@ -313,8 +314,8 @@ __global__ void __launch_bounds__(kSvThreads) k_solution_vars(int nx, int nz, in
   const long long plane = (long long)NX * (nz + 2 * kHs);
   const long long n = (long long)nx * nz;
   for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    const int kb = (int)(blk / per_row), k0 = kb * rows, i0 = (int)(blk - (long long)kb * per_row) * kSvCells;
-    const int nr = min(rows, nz - k0), len = min(nx - i0, kSvCells);
+    const int kb = (int)(blk / per_row), k0 = kb * rows, i0 = (int)(blk - (long long)kb * per_row) * piece;
+    const int nr = min(rows, nz - k0), len = min(nx - i0, piece);
     double hr, hrt[1], th[1];
     if (!ROWS || threadIdx.x < ((nr + 31) & ~31)) {
       const int r = ROWS ? min((int)threadIdx.x, nr - 1) : 0;
@@ -616,12 +617,15 @@ extern "C" int mw_solution_variables_f64(int nx, int nz, const double* hyc, cons
   if (st) return st;
   MW_REQUIRE(hyc && hytc && state && out, MW_ERR_INVALID_ARG, "NULL pointer argument");
   MW_REQUIRE(aligned(hyc) && aligned(hytc) && aligned(state) && aligned(out), MW_ERR_ALIGN, "misaligned pointer");
-  // blocks of whole rows, or pieces of one; fewer rows where the blocks would not fill the SMs
+  // blocks of whole rows, or pieces of one; fewer rows or shorter pieces where the blocks would not fill the SMs
   const long long fit = std::min<long long>({kSvCells / nx, kSvRows, nz / (2LL * 152)});
-  const int rows = (int)std::max(1LL, fit), per_row = (nx + kSvCells - 1) / kSvCells;
+  const long long share = ((long long)nx * nz / (2LL * 152) + kSvThreads - 1) / kSvThreads * kSvThreads;
+  const int rows = (int)std::max(1LL, fit);
+  const int piece = rows > 1 ? nx : (int)std::min<long long>(kSvCells, std::max<long long>(kSvThreads, share));
+  const int per_row = (nx + piece - 1) / piece;
   const long long nblk = (long long)per_row * ((nz + rows - 1) / rows);
   auto kern = rows > 1 ? k_solution_vars<true> : k_solution_vars<false>;
-  kern<<<(unsigned)std::min(nblk, 1LL << 20), kSvThreads, 0, (cudaStream_t)stream>>>(nx, nz, rows, per_row, nblk, hyc,
+  kern<<<(unsigned)std::min(nblk, 1LL << 20), kSvThreads, 0, (cudaStream_t)stream>>>(nx, nz, rows, piece, per_row, nblk, hyc,
                                                                                      hytc, state, out);
   return check_launch("solution variables launch");
 }

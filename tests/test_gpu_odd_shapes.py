@@ -4,12 +4,15 @@ kernels' other shapes of work, and that a call's time follows its cells.
 Times are the least of ten, compared within one process with those of a square
 grid of as many cells; the bounds leave a factor of about two over what was
 measured, and are as much below what the shapes took before."""
+import numpy as np
 import pytest
 import torch
 
 from pyminiweather_gb300 import _native
 from pyminiweather_gb300.data import initialize_fields
 from pyminiweather_gb300.ics import init
+from pyminiweather_gb300.post import compute_solution_variables
+from tests import test_gpu_diagnostics as diagnostics
 from tests.helpers import make_params
 from tests.test_gpu_short_rows import us
 
@@ -116,3 +119,15 @@ def test_x_stage_of_short_rows_takes_the_time_of_its_slots():
     # slots always 1246
     short, full = developed(30, 200000), developed(62, 200000)
     assert us(lambda: stage(*short, "fp64")) <= 0.7 * us(lambda: stage(*full, "fp64"))
+
+
+# pieces of a row of 256 cells and more, up to 2048, whole and cut
+@pytest.mark.parametrize("nx,nz", [(255, 2), (257, 2), (512, 300), (513, 303), (4000, 16), (20000, 2), (40961, 9),
+                                   (300000, 1), (700001, 1)])
+def test_solution_variables_of_long_rows(nx, nz):
+    p, f = diagnostics.developed(nx, nz)
+    v = diagnostics.exact(p, f)[2]
+    got = compute_solution_variables(p, f).cpu().numpy()
+    for q in range(4):  # bounds of test_gpu_diagnostics.py
+        scale = np.abs(v[q]).max() if q < 3 else 300.0
+        assert np.abs(got[q] - v[q]).max() <= 4 * 2.0 ** -53 * scale, q
