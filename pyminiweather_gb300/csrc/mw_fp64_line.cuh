@@ -17,6 +17,11 @@ constexpr long long kLineCellsMax = 600000;
 // 85 / 110, 880x620 120 / 134, 900x620 125 / 138; 600x1000 146 / 139, 1100x700
 // 170 / 166, 1250x799 213 / 201).
 constexpr long long kSplitLineCellsMax = 580000;
+// Nor with lines of more cells than this, whose pieces (sixteen at most) take so
+// many warps that an SM holds one or two CTAs (us a step, four a call, line
+// kernels / six stage launches: 75x4000 90 / 107, 4000x120 127 / 125; 5000x100
+// 154 / 138, 100x5000 166 / 144, 6000x75 141 / 123, 75x6000 148 / 128).
+constexpr int kSplitLineMax = 4096;
 // The FP32 form's against its direction kernels (40x12 8.9 / 19.7, 100x50 8.1 / 16.2,
 // 300x150 8.6 / 16.9, 401x199 10.9 / 17.6, 512x256 12.5 / 20.9; 700x500 28.1 / 25.1,
 // 1000x1000 61 / 40).

@@ -226,7 +226,7 @@ int launch_split_line_t(const SplitLineParams& P, int ctas, int threads, size_t 
 
 int line_split_plan(int nx, int nz, LinePlan* plan) {
   *plan = LinePlan();
-  if ((long long)nx * nz > kSplitLineCellsMax) return MW_OK;
+  if ((long long)nx * nz > kSplitLineCellsMax || std::max(nx, nz) > kSplitLineMax) return MW_OK;
   int sms = 0;
   const int st = line_sms(&sms);
   if (st) return st;
