@@ -135,6 +135,7 @@ int ens_step(void* plan, const mw_ens_plan_info* info, const double* hyc, const 
   es.mconsts = (const char*)plan + ens_consts_off(*info);
   es.n_xrows = info->n_xrows;
   es.n_members = info->n_members;
+  const bool split = fmts[0] != 0;
   if (nsteps > 0 && (st = row_table((char*)plan + info->xrows_off))) return st;
   for (int n = 0; n < nsteps; ++n) {
     const int dirs[2] = {*reverse ? MW_DIR_X : MW_DIR_Z, *reverse ? MW_DIR_Z : MW_DIR_X};
@@ -145,7 +146,7 @@ int ens_step(void* plan, const mw_ens_plan_info* info, const double* hyc, const 
       const int grid = dirs[d] == MW_DIR_X ? grid_x : grid_z;
       es.z_parts = dirs[d] == MW_DIR_X ? 1
                                        : ens_z_parts(info->n_z_items, info->z_tile, grid,
-                                                     std::is_same<T, float>::value ? 1 : 4);
+                                                     std::is_same<T, float>::value ? 1 : (split ? 2 : 4));
       if constexpr (std::is_same<T, float>::value) {  // one launch per direction, state -> scratch -> state
         const bool halo = flags & MW_FLAG_WRITE_HALO;
         es.init = d ? A : S;

@@ -76,7 +76,9 @@ __host__ __device__ inline int mconsts_index(const EnsStageT<T>& es, int e) {
 // on a few CTAs still marching whole tiles (48 FP64 members of 64-512 columns:
 // 317 us a z stage, 1.9 times an x stage), so the tiles are halved until they
 // do, but not below 16 rows (each part evaluates one interface more than it has
-// rows; in the FP32 form it marches 12 rows more, and one grid's worth is enough).
+// rows; in the FP32 form it marches 12 rows more, and one grid's worth is enough;
+// in the double-FP32 form two: four members of 1500x1500 1389 us a step with up to
+// four grids' worth, 1352 with two, 200 of 1000x40 1385 and 1361).
 inline int ens_z_parts(int n_items, int z_tile, int grid, int want) {
   int parts = 1;
   while ((long long)n_items * parts < (long long)want * grid && z_tile >= 32 * parts) parts *= 2;
