@@ -140,8 +140,8 @@ int mw_step_f64(int nx, int nz, double dx, double dz, double dt_full, double dt,
  * resulting state is copied into h_out (which may equal h_in).  Enqueued on
  * `stream`; h_out is complete once the stream is.  In the IEEE-FP64 and split
  * forms the copies overlap the computation by nbands row bands (at most 64, at
- * most nz / 16 and at most one per 2^19 cells); the results are those of copy-in, mw_step_f64, copy-out
- * bit for bit.
+ * most nz / 16 and at most one per 2^19 cells); the results are those of
+ * copy-in, mw_step_f64, copy-out bit for bit.
  * h_in / h_out should be page-locked for the copies to run asynchronously.
  * Calls on one device share internal copy and compute streams (the x stages
  * of a band run on one beside the caller's) and are serialised. */
@@ -150,6 +150,9 @@ int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_full, doubl
                      const double* hy_pressure_int, const double* src_w, const double* h_in, double* h_out,
                      double* state, double* state_tmp, double* scratch, int* reverse, int f64_mode, unsigned flags,
                      int nbands, void* stream);
+/* The row bands mw_step_f64_host takes of the nbands it is given (1: copy in,
+ * step, copy out); 0 for a grid or mode that it refuses. */
+int mw_host_step_bands(int nx, int nz, int f64_mode, int nbands);
 
 int mw_step_f32(int nx, int nz, double dx, double dz, double dt_full, double dt, const double* hy_dens_cell,
                 const double* hy_dens_theta_cell, const double* hy_dens_int, const double* hy_dens_theta_int,

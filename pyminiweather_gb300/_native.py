@@ -39,6 +39,7 @@ _SIGNATURES = {
     "mw_step_f64": [_i, _i, _d, _d, _d, _d, _P, _P, _P, _P, _P, _P, _P, _P, _P, _i, ctypes.POINTER(_i), _i, _u, _P],
     "mw_step_f64_host": [_i, _i, _d, _d, _d, _d, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, ctypes.POINTER(_i), _i,
                          _u, _i, _P],
+    "mw_host_step_bands": [_i, _i, _i, _i],
     "mw_step_f32": [_i, _i, _d, _d, _d, _d, _P, _P, _P, _P, _P, _P, _P, _P, _P, _i, ctypes.POINTER(_i), _u, _P],
     "mw_step_f64_noalloc": [_i, _i, _d, _d, _d, _d, _P, _P, _P, _P, _P, _P, _P, _P, _i, ctypes.POINTER(_i), _i, _u,
                             _P],

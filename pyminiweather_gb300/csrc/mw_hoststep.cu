@@ -71,6 +71,13 @@ int resources(CopyRes** r) {
   return MW_OK;
 }
 
+// The bands of a step that may have up to nbands.  Grids of the line kernels have one: bands are stepped by stages.
+int host_bands(int nx, int nz, int f64_mode, int nbands) {
+  if (f64_mode != MW_F64_SPLIT && f64_mode != MW_F64_IEEE) return 1;
+  return (int)std::max(1LL, std::min<long long>({nbands, kMaxBands, nz / 16, (long long)nx * nz / kBandCells}));
+}
+static_assert(2 * kBandCells > kLineCellsMax && 2 * kBandCells > kSplitLineCellsMax, "banded grids take no line kernels");
+
 // First interior row of band b.  With ten or more bands the first three and
 // the last three are half as tall as the others, so that the copies out start
 // sooner and the last copy out ends sooner after the last copy in.
@@ -117,6 +124,10 @@ extern "C" int mw_step_f64(int nx, int nz, double dx, double dz, double dt_full,
                            const double* src_w, double* state, double* state_tmp, double* scratch, int nsteps,
                            int* reverse, int f64_mode, unsigned flags, void* stream);
 
+extern "C" int mw_host_step_bands(int nx, int nz, int f64_mode, int nbands) {
+  return check_grid(nx, nz) == MW_OK && valid_f64_mode(f64_mode) ? host_bands(nx, nz, f64_mode, nbands) : 0;
+}
+
 extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_full, double dt, const double* hyc,
                                 const double* hytc, const double* hyi, const double* hyti, const double* hypi,
                                 const double* src_w, const double* h_in, double* h_out, double* state,
@@ -131,13 +142,8 @@ extern "C" int mw_step_f64_host(int nx, int nz, double dx, double dz, double dt_
   const Geom g = make_geom(nx, nz);
   const size_t bytes = sizeof(double) * 4 * (size_t)g.plane;
   cudaStream_t s = (cudaStream_t)stream;
-  // grids of the line kernels (a direction per launch) are stepped whole, as mw_step_f64 steps them
-  LinePlan plan;
-  if (f64_mode == MW_F64_IEEE && (st = line_ieee_plan(nx, nz, &plan))) return st;
-  const int nb = plan.fits ? 1
-                           : std::max(1, (int)std::min<long long>({nbands, kMaxBands, nz / 16,
-                                                                    (long long)nx * nz / kBandCells}));
-  if ((f64_mode != MW_F64_SPLIT && f64_mode != MW_F64_IEEE) || nb == 1) {  // no bands: copy in, step, copy out
+  const int nb = host_bands(nx, nz, f64_mode, nbands);
+  if (nb == 1) {  // copy in, step, copy out
     cudaError_t e = cudaMemcpyAsync(state, h_in, bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(MW_ERR_CUDA, "copy in: %s", cudaGetErrorString(e));
     if ((st = mw_step_f64(nx, nz, dx, dz, dt_full, dt, hyc, hytc, hyi, hyti, hypi, src_w, state, state_tmp, scratch, 1,
