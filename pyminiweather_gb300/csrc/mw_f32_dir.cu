@@ -42,11 +42,10 @@ constexpr int kAhead = 9;      // rows loaded ahead
 constexpr int kLag = 6;        // row r of the state comes in when row r - 6 of the result goes out
 constexpr int kZTileMax = 512; // rows per z CTA
 constexpr int kXWarps = 4;     // warps per x CTA
-// Launches of at most this many CTAs let the next one in at their head: both
-// then find an SM per CTA (100x50: 15.9 against 16.9 us a step).  A larger one's
-// CTAs would share SMs with the next one's, which stay there (2501x1251: 98 us a
-// step with every launch doing so, 79 with none).
-constexpr unsigned kFewCtas = 76;
+// A launch lets the next one in only when it ends: earlier, its CTAs would share
+// SMs with the next one's, which stay there (2501x1251: 98 us a step with every
+// launch doing so at its head, 79 with none; 20001x1, of under a CTA per SM, 16.2
+// either way).
 
 struct Args {
   int nx, nz, pitch;
@@ -151,7 +150,6 @@ __device__ __forceinline__ void z_march(const Args& a, int cb, int z0, int z1, S
   }
   __syncthreads();
   overlap_wait();
-  if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   const int c = cb * NC + t;
   // the wall halo rows (arrays that ask for them): of the initial state here, and of the x-halo columns of
   // both arrays from the halo columns' own first and last rows
@@ -449,7 +447,6 @@ __global__ void __launch_bounds__(32 * kXWarps, 4) k_dir_x_f32(const __grid_cons
   Row row = {0.f, 0.f, 0.f, 0.f};
   if (g0 < g1) row = row_x(MW_AT(a.hyc, k + kHs, a.nz + 2 * kHs), MW_AT(a.hytc, k + kHs, a.nz + 2 * kHs));
   overlap_wait();
-  if (gridDim.x * gridDim.y <= kFewCtas) overlap_next();
   if (g0 >= g1) return;
   x_load<V, SRC>(a, k, rn * len, min(len, a.nx - rn * len), buf[0]);
   int cur = 0;
@@ -625,7 +622,9 @@ int launch_dir_f32(int nx, int nz, double dx, double dz, double dt_full, double 
   const int sms = dev->sms.load(std::memory_order_relaxed);
   if (direction == MW_DIR_X) {
     // Cells per lane: 8 where the rows' runs then give every SM partition a
-    // warp or more, else 4 (twice the warps, 9 instead of 5 % of them halo).
+    // warp or more, else 4 (twice the warps, 9 instead of 5 % of them halo): a
+    // few rows too long for the line kernels (us a step, eight a call, 4 / 8:
+    // 20001x1 16.2 / 18.0, 20000x2 17.0 / 18.4, 16100x3 17.5 / 19.2, 16100x9 20.4 / 21.3).
     auto runs = [&](int v) { return (nx + x_run_max(v) - 1) / x_run_max(v); };
     const int v = (long long)runs(8) * nz >= 4LL * sms ? 8 : 4;
     const int nrun0 = runs(v), lenc = (nx + nrun0 - 1) / nrun0, nrun = (nx + lenc - 1) / lenc;
