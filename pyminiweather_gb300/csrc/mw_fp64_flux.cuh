@@ -65,7 +65,7 @@ __device__ __forceinline__ RowP row_consts_p(double r, double rt, double P, doub
     pw *= o.d.IRT12;
   }
   const double lo = fabs(o.b[kMaxDeg]), hi = fabs(o.b[1]);
-  const bool normal = lo >= 0x1p-1000 && hi <= 0x1p1000 && pw >= 0x1p-1000;
+  const bool normal = fmin(lo, hi) >= 0x1p-1000 && fmax(lo, hi) <= 0x1p1000 && pw >= 0x1p-1000 && pw <= 0x1p1000;
   const unsigned long long bI = (unsigned long long)__double_as_longlong(o.d.IRT12);
   o.eI = normal ? (int)(bI >> 52 & 0x7ffu) : 4096;
   o.mI = (unsigned)(bI >> 36 & 0xffffu) + 0x10001u;
