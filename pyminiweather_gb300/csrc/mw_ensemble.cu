@@ -220,9 +220,10 @@ extern "C" int mw_ensemble_plan(int n_members, const mw_ens_member* members, int
         c.c_f = f32_c(d, dts);
         c.dt_f = (float)dts;
         c.pad = 0.0f;
-        c.HV = ieee_hv(d, m.dt);  // as launch_stage_ieee forms them
-        c.IHV = 1.0 / c.HV;
-        c.c = dts / (12.0 * d) * c.HV;
+        const IeeeScale sc = ieee_scale(d, m.dt, dts);  // as launch_stage_ieee forms them
+        c.HV = sc.HV;
+        c.IHV = sc.IHV;
+        c.c = sc.c;
         c.dt = dts;
         MW_REQUIRE(std::isfinite(c.c12s), MW_ERR_INVALID_ARG,
                    "member %d: dt / (12 d) = %g is above the split form's range", e, dts / (12.0 * d));

@@ -19,10 +19,10 @@ struct RowD {
   double P;      // 12 / HV x background pressure C0 (rho theta)^gamma
   double PC1;    // P C(gamma, 1) IRT12: the pressure perturbation per unit of 12 (rho theta)' to first order
 };
-// (scale: that of the interpolated values, if not 12).
-__device__ __forceinline__ RowD row_consts(double r, double rt, double P, double HV, double IHV, double scale = 12.0) {
-  const double irt = 1.0 / (scale * rt), p = scale * P * IHV;
-  return {scale * r * HV, scale * rt, irt, p, p * c_pow_g.c[1] * irt};
+// HS, IS: HV and 1 / HV times the scale of the interpolated values, 12 (scale, if another).
+__device__ __forceinline__ RowD row_consts(double r, double rt, double P, double HS, double IS, double scale = 12.0) {
+  const double irt = 1.0 / (scale * rt), p = P * IS;
+  return {r * HS, scale * rt, irt, p, p * c_pow_g.c[1] * irt};
 }
 
 // P ((1 + d)^gamma - 1) + add, d = AT IRT12, for the lanes in `mask`, which
@@ -53,10 +53,10 @@ struct RowP {
   int eI;                 // biased exponent of IRT12; 4096 where the b[n] would leave the normal range
   unsigned mI;            // an upper bound of 2^16 x IRT12's significand (in [1, 2)): top 16 fraction bits + 1
 };
-__device__ __forceinline__ RowP row_consts_p(double r, double rt, double P, double HV, double IHV,
+__device__ __forceinline__ RowP row_consts_p(double r, double rt, double P, double HS, double IS,
                                              double scale = 12.0) {
   RowP o;
-  o.d = row_consts(r, rt, P, HV, IHV, scale);
+  o.d = row_consts(r, rt, P, HS, IS, scale);
   double pw = o.d.IRT12;
   o.b[0] = 0.0;
 #pragma unroll

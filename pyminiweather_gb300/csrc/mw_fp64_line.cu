@@ -34,7 +34,8 @@ namespace ieee {
 // Most warps per CTA with SL slots per lane (as their registers allow).
 __host__ __device__ constexpr int line_warps(int sl) { return sl == 0 ? 24 : (sl == 1 ? 20 : 16); }
 struct LineParams : LineGeom {
-  double HV, IHV;        // HV = -12 hv of the direction and 1 / HV
+  double HV, IHV;        // HV = -12 hv of the direction and 1 / HV (ieee_scale)
+  double H12, I12;       // 12 of either
   double c[3], dt[3];    // per stage HV dt_stage / (12 d) and dt_stage
 };
 
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     }
     __syncthreads();
     if (w == 0) {
-      const double pr = kC0 * pow_gamma(rt, pow_tables), irt = rcp(12.0 * rt, kAll), p = 12.0 * pr * P.IHV;
-      if (lane < nl) rows[lane] = {12.0 * r * P.HV, 12.0 * rt, irt, p, p * c_pow_g.c[1] * irt};
+      const double pr = kC0 * pow_gamma(rt, pow_tables), irt = rcp(12.0 * rt, kAll), p = pr * P.I12;
+      if (lane < nl) rows[lane] = {r * P.H12, 12.0 * rt, irt, p, p * c_pow_g.c[1] * irt};
     }
   } else {
     if (threadIdx.x < 4) {
@@ -140,10 +141,10 @@ __global__ void __launch_bounds__(line_warps(SL) * 32, 1) k_line_ieee(const __gr
     for (int j = 0; j < NS; ++j) {
       const int i = min(max(c0 - 1 + 32 * j + sub, 0), n);
       const double rt12 = 12.0 * MW_AT(a.hyti, i, n + 1);
-      rz[j].R = MW_AT(a.hyi, i, n + 1) * (12.0 * P.HV);
+      rz[j].R = MW_AT(a.hyi, i, n + 1) * P.H12;
       rz[j].RT12 = rt12;
       rz[j].IRT12 = rcp(rt12, kAll);
-      rz[j].P = MW_AT(a.hypi, i, n + 1) * (12.0 * P.IHV);
+      rz[j].P = MW_AT(a.hypi, i, n + 1) * P.I12;
       rz[j].PC1 = rz[j].P * c_pow_g.c[1] * rz[j].IRT12;
     }
   }
@@ -382,11 +383,14 @@ int launch_line_ieee(const LinePlan& plan, int nx, int nz, double dx, double dz,
   P.a = a;
   const bool isx = direction == MW_DIR_X;
   const double d = isx ? dx : dz;
-  P.HV = ieee_hv(d, dt_full);
-  P.IHV = 1.0 / P.HV;
+  const IeeeScale sc = ieee_scale(d, dt_full, dt);
+  P.HV = sc.HV;
+  P.IHV = sc.IHV;
+  P.H12 = sc.H12;
+  P.I12 = sc.I12;
   for (int s = 0; s < 3; ++s) {
     P.dt[s] = dt / (3 - s);
-    P.c[s] = P.dt[s] / (12.0 * d) * P.HV;
+    P.c[s] = sc.c / (3 - s);
   }
   const LineSpread& sp = isx ? plan.x : plan.z;
   MW_REQUIRE(sp.pieces == 1 || a.in != a.out, MW_ERR_ALIAS, "a direction of cut lines needs another array for its result");

@@ -75,6 +75,8 @@ struct Args {
   unsigned flags;
   double HV;    // -12 hv, hv = -hv_beta d / (16 dt_full) (interpolate.py:101,149)
   double IHV;   // 1 / HV
+  double H12;   // 12 HV
+  double I12;   // 12 / HV
   double c;     // HV dt_stage / (12 d)
   double dt;    // dt_stage (source terms)
   double gdt;   // -dt_stage grav (z)
@@ -284,8 +286,8 @@ __global__ void __launch_bounds__(kXT, MW_IEEE_X_MIN_BLOCKS) k_stage_x_ieee_w(Ar
     __syncthreads();
     for (int r = threadIdx.x; r < nrows; r += kXT) {
       const double rt = MW_AT(a.hytc, row0 + r + kHs, a.nz + 2 * kHs);
-      rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow_gamma(rt, pow_tables), a.HV,
-                             a.IHV);
+      rows[r] = row_consts_p(MW_AT(a.hyc, row0 + r + kHs, a.nz + 2 * kHs), rt, kC0 * pow_gamma(rt, pow_tables), a.H12,
+                             a.I12);
     }
     __syncthreads();
   };
@@ -311,8 +313,8 @@ template <int NC>
 __device__ __forceinline__ void z_tile(const Args& a, int cb, int z0, int z1, bool hbot, bool htop, SmemZ& sm) {
   for (int rr = threadIdx.x; rr <= z1 - z0; rr += NC) {
     const int k = z0 + rr;
-    sm.row[rr] = row_consts_p(MW_AT(a.hyi, k, a.nz + 1), MW_AT(a.hyti, k, a.nz + 1), MW_AT(a.hypi, k, a.nz + 1), a.HV,
-                              a.IHV);
+    sm.row[rr] = row_consts_p(MW_AT(a.hyi, k, a.nz + 1), MW_AT(a.hyti, k, a.nz + 1), MW_AT(a.hypi, k, a.nz + 1), a.H12,
+                              a.I12);
   }
   __syncthreads();
   overlap_wait();
@@ -411,6 +413,8 @@ __device__ __forceinline__ Args member_args(const EnsStage& es, int e) {
                                    (long long)kEnsConstsPerMember * es.n_members);
   a.HV = c.HV;
   a.IHV = c.IHV;
+  a.H12 = 12.0 * c.HV;
+  a.I12 = 12.0 * c.IHV;
   a.c = c.c;
   a.dt = c.dt;
   a.gdt = -c.dt * kGrav;
@@ -426,7 +430,7 @@ static_assert(sizeof(RowD) <= kEnsRowBytes, "row-constant table entry size");
 __global__ void k_ens_row_table_ieee(const double* hyc, const double* hytc, long long n, RowD* table) {
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
     const double rt = MW_AT(hytc, j, n);
-    MW_AT(table, j, n) = row_consts(MW_AT(hyc, j, n), rt, kC0 * pow(rt, kGamma), 1.0, 1.0);
+    MW_AT(table, j, n) = row_consts(MW_AT(hyc, j, n), rt, kC0 * pow(rt, kGamma), 12.0, 12.0);
   }
 }
 
@@ -540,9 +544,12 @@ int launch_stage_ieee(int nx, int nz, double dx, double dz, double dt_full, cons
   a.out = out;
   a.flags = flags;
   const double d = direction == MW_DIR_X ? dx : dz;
-  a.HV = ieee_hv(d, dt_full);
-  a.IHV = 1.0 / a.HV;
-  a.c = dt_stage / (12.0 * d) * a.HV;
+  const IeeeScale sc = ieee_scale(d, dt_full, dt_stage);
+  a.HV = sc.HV;
+  a.IHV = sc.IHV;
+  a.H12 = sc.H12;
+  a.I12 = sc.I12;
+  a.c = sc.c;
   a.dt = dt_stage;
   a.gdt = -dt_stage * kGrav;
   a.r0 = r0;
