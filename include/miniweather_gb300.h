@@ -188,8 +188,8 @@ int mw_step_f64_noalloc(int nx, int nz, double dx, double dz, double dt_full, do
  * Ensembles of uneven grids.  No counterpart in the reference (one grid per
  * process there): many members, each a full simulation with its own nx, nz,
  * dx, dz and dt, advance together, one persistent kernel launch per
- * direction-stage walking a work list over all members.  Each member's state
- * is a (4, nz+4, nx+4) block at state_off (elements) in the shared state,
+ * direction-stage (FP32: per direction) walking a work list over all members.
+ * Each member's state is a (4, nz+4, nx+4) block at state_off (elements) in the shared state,
  * state_tmp and scratch buffers; its backgrounds sit at cell_off (nz+4
  * values) and int_off (nz+1 values) in the shared background buffers.  dt is
  * the member's params["dt"]: the RK step and the hyperviscosity time scale.
@@ -248,11 +248,10 @@ int mw_ensemble_step_f32(void* plan_device, const mw_ens_plan_info* info, const 
  * a base may be g_dst itself (accumulation); g_dst must not overlap g_out or
  * forcing.  f64_mode: MW_F64_NATIVE (FP64 arithmetic, the reference's
  * formulas: an interface kernel then a gather), MW_F64_IEEE (FP64 arithmetic
- * with the fewest operations, after a small background-table kernel: one
- * kernel in x, an interface kernel then the gather in z) or MW_F64_SPLIT
- * (double-FP32 interior arithmetic as the split forward, one kernel after a
- * small background-table kernel).
- * workspace: mw_dirstage_vjp_workspace_bytes.
+ * with the fewest operations) or MW_F64_SPLIT (double-FP32 interior arithmetic
+ * as the split forward), one kernel each after a small background-table kernel.
+ * workspace: mw_dirstage_vjp_workspace_bytes, which serves every mode (most of
+ * it holds the native form's interface adjoints).
  * ------------------------------------------------------------------------- */
 size_t mw_dirstage_vjp_workspace_bytes(int nx, int nz);
 int mw_dirstage_vjp_f64(int nx, int nz, double dx, double dz, double dt_full, const double* hy_dens_cell,

@@ -632,8 +632,9 @@ long long n_interfaces(int nx, int nz, int dir) {
   return dir == MW_DIR_X ? (long long)nz * (nx + 1) : (long long)(nz + 1) * nx;
 }
 
-// Doubles of the workspace before the IEEE row table: the interface adjoints
-// of either direction (8 values per interface).
+// Doubles of the workspace before the IEEE row table: the native form's
+// interface adjoints of either direction (8 values per interface; one size
+// serves every mode, and the IEEE form leaves them alone).
 long long ieee_rows_off(int nx, int nz) {
   return 8 * std::max(n_interfaces(nx, nz, MW_DIR_X), n_interfaces(nx, nz, MW_DIR_Z));
 }

@@ -276,7 +276,9 @@ int launch_line_t(const LineParams& P, int ctas, int threads, size_t smem, bool 
 // two slots of a run repeat its neighbours' (x pass of mw_fp64_stage.cu)
 constexpr LineKind kIeeeLines = {0, 2, {line_warps(0), line_warps(1), line_warps(2)}, {80, 96, 128}, 2, 64, 0, 0.0};
 
-constexpr int kMaxPieces = 16;
+constexpr int kMaxPieces = 16, kMinPiece = 24;
+// The last piece may be shorter than the others by a cell per piece; the halo slots beside it hold six cells.
+static_assert(kMinPiece - (kMaxPieces - 1) > 6, "a last piece must be longer than its neighbours' halo");
 // A warp of half slots against one of whole ones: 0.61 in FP64 instructions, more in time (us a step, one a call:
 // 60x30 27.9 -> 23.5, 100x50 26.7 -> 23.4; where partitions get two warps for one it loses, 200x100 31.0 -> 36.2).
 constexpr double kHalfCost = 0.75;
@@ -309,7 +311,7 @@ LineSpread spread_lines(const LineKind& kind, int n, int nlines, bool isx, int s
   LineSpread best;
   double least = 0.0;
   for (int sl = kind.min_slots; sl <= kind.max_slots; ++sl)
-    for (int pieces = 1; pieces == 1 || (pieces <= kMaxPieces && (n + pieces - 1) / pieces >= 24); ++pieces) {
+    for (int pieces = 1; pieces == 1 || (pieces <= kMaxPieces && (n + pieces - 1) / pieces >= kMinPiece); ++pieces) {
       const int piece = (n + pieces - 1) / pieces;
       if ((n + piece - 1) / piece != pieces) continue;  // an empty last piece
       const int range = pieces == 1 ? n : piece + 8;

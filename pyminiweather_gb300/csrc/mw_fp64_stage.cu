@@ -38,10 +38,12 @@
 // from the neighbouring lane, or from the block before.  z pass: one thread
 // per column marching a tile of rows, e, q and the flux of the row before kept
 // in registers.  Halo cells are never read: the periodic-x and wall-z rules of
-// ics/bcs.py are applied to the indices and values as they are loaded.  The
-// result at a cell depends on its neighbourhood alone, not on how the grid is
-// split over warps (the series' degree is chosen per lane).  Every global
-// access goes through MW_AT (bounds-checked in the debug library).
+// ics/bcs.py are applied to the indices and values as they are loaded.  On
+// single grids the result at a cell depends on its neighbourhood alone, not on
+// how the grid is split over warps (the series' degree is chosen per lane); the
+// ensembles' x pass and the line kernels (mw_fp64_line.cu) take one degree per
+// warp, so the last bits of a cell there may follow the cells its warp holds.
+// Every global access goes through MW_AT (bounds-checked in the debug library).
 #include <algorithm>
 #include <atomic>
 
