@@ -201,7 +201,7 @@ __device__ __forceinline__ double load_state(const float* p) { return split::f2d
 // ke = ((rho u)^2 + (rho w)^2) / rho takes one reciprocal: 7 + n FP64
 // operations per cell, n the series' degree, which bounds the kernel (FP64
 // pipe).  The same quantities as the reference's up to a few roundings per
-// cell (the sums agree to ~1e-16 relative).  At 4096x2048: 213 us; with a
+// cell (the sums agree to ~1e-16 relative).  At 4096x2048: 191 us; with a
 // power per warp and row, the background in every cell's sums and the series
 // in d, 357 us.
 constexpr int kStatRows = 16;  // rows whose constants a block holds at a time

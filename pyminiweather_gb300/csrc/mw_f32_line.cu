@@ -6,8 +6,8 @@
 // launches of a call overlapping; the arithmetic is that of the direction
 // kernels (mw_f32_dir.cu), value for value.  Those fill and drain a pipeline per
 // thread (z) or work through long runs (x), which takes a launch 8 us or more
-// however small the grid; here a cell is one lane's work (100x50 16.2 -> 8.1 us a
-// step, 512x256 20.9 -> 12.5), at the price of four shared-memory reads and both
+// however small the grid; here a cell is one lane's work (100x50 15.6 -> 7.9 us a
+// step, 512x256 19.1 -> 12.5), at the price of four shared-memory reads and both
 // neighbours' second differences per cell, which larger grids pay for (700x500
 // 25.1 -> 28.1).  A cell is a float4 in shared memory, twice (a stage's input and
 // its result).

@@ -279,8 +279,9 @@ constexpr LineKind kIeeeLines = {0, 2, {line_warps(0), line_warps(1), line_warps
 constexpr int kMaxPieces = 16, kMinPiece = 24;
 // The last piece may be shorter than the others by a cell per piece; the halo slots beside it hold six cells.
 static_assert(kMinPiece - (kMaxPieces - 1) > 6, "a last piece must be longer than its neighbours' halo");
-// A warp of half slots against one of whole ones: 0.61 in FP64 instructions, more in time (us a step, one a call:
-// 60x30 27.9 -> 23.5, 100x50 26.7 -> 23.4; where partitions get two warps for one it loses, 200x100 31.0 -> 36.2).
+// A warp of half slots against one of whole ones: 0.61 in FP64 instructions, more in time (us a step, eight a call:
+// 60x30 20.5 -> 16.6, 100x50 20.0 -> 17.6; where partitions get two warps for one it loses, 200x100 31.0 -> 36.2 a step
+// in calls of one).
 constexpr double kHalfCost = 0.75;
 
 // The spread with the least time.  An SM that gets m CTAs of W warps with SL

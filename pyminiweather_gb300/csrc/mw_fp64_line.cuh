@@ -9,22 +9,25 @@ namespace mw {
 // Most cells of a grid that takes the line kernels: above this the CTAs of a
 // launch come in several waves and the stage kernels, which need no whole lines
 // in a CTA, do as well (us per step, eight a call, line kernels / six stage
-// launches: 100x50 18 / 118, 300x150 41 / 122, 512x256 110 / 145, 800x400 237 / 279,
-// 990x495 346 / 376, 1000x640 440 / 452; 1200x600 473 / 457, 992x992 665 / 653).
+// launches: 100x50 17.6 / 115, 300x150 41 / 116, 512x256 110 / 139, 800x400 236 / 272,
+// 990x495 348 / 377; from half a million cells on it is one or the other by how
+// the lines divide over the SMs: 880x620 400 / 384, 900x620 391 / 423, 1000x600
+// 429 / 380, 1200x600 473 / 457).
 constexpr long long kLineCellsMax = 600000;
 
-// The double-FP32 form's (100x50 14 / 61, 300x150 18 / 73, 512x256 38 / 70, 700x500
-// 85 / 110, 880x620 120 / 134, 900x620 125 / 138; 600x1000 146 / 139, 1100x700
-// 170 / 166, 1250x799 213 / 201).
+// The double-FP32 form's (100x50 12.8 / 63, 300x150 18 / 74, 512x256 38 / 70, 700x500
+// 85 / 109, 880x620 121 / 135; 600x1000 146 / 139, 1100x700 170 / 166, 1250x799
+// 213 / 201).
 constexpr long long kSplitLineCellsMax = 580000;
 // Nor with lines of more cells than this, whose pieces (sixteen at most) take so
 // many warps that an SM holds one or two CTAs (us a step, four a call, line
 // kernels / six stage launches: 75x4000 90 / 107, 4000x120 127 / 125; 5000x100
 // 154 / 138, 100x5000 166 / 144, 6000x75 141 / 123, 75x6000 148 / 128).
 constexpr int kSplitLineMax = 4096;
-// The FP32 form's against its direction kernels (40x12 8.9 / 19.7, 100x50 8.1 / 16.2,
-// 300x150 8.6 / 16.9, 401x199 10.9 / 17.6, 512x256 12.5 / 20.9; 700x500 28.1 / 25.1,
-// 1000x1000 61 / 40).
+// The FP32 form's against its direction kernels (40x12 8.7 / 19.1, 100x50 7.9 / 15.6,
+// 300x150 8.7 / 16.6, 401x199 10.7 / 16.1, 512x256 12.5 / 19.1; 700x500 28.1 / 25.1,
+// 1000x1000 61 / 40).  Grids of a few long rows lose earlier (four a call: 1500x200
+// 31 / 26, 4000x75 39 / 26).
 constexpr long long kF32LineCellsMax = 300000;
 
 struct LineArgs {

@@ -13,10 +13,10 @@ constexpr int kLineMax = 8;            // most lines per CTA
 constexpr size_t kLineSmem = 200 << 10;
 // A launch of at most this many CTAs, about one per SM, lets the next one in at
 // its head, whose row constants then cost no time (us a step, eight in a call:
-// IEEE form 100x50 24.2 -> 22.8, 150x75 26.0 -> 23.6, double-FP32 14.3 -> 13.3); a
-// larger one only after its last stage: the next one's CTAs take what is free
-// beside its own, and earlier that is unevenly much (256x128, IEEE: 60 us a step
-// with the trigger at the head, 41 here, 47 without overlap).
+// IEEE form 60x30 17.9 -> 16.6, 100x50 18.2 -> 17.6, 150x75 21.7 -> 20.5, double-FP32
+// 100x50 14.2 -> 12.8); a larger one only after its last stage: the next one's CTAs
+// take what is free beside its own, and earlier that is unevenly much (IEEE,
+// 256x128: 47.6 us a step with the trigger at the head, 37.9 here; 300x150 57, 41).
 constexpr unsigned kLineFewCtas = 152;
 
 struct LineShape {

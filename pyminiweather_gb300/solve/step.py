@@ -123,7 +123,8 @@ def evolve(params: Dict, fields, mesh=None, dt: float = 1e-4, nsteps: int = 1) -
 # others, so the short banded launches fill each other's tails, and both forms
 # do best with 32 bands: the split form is bound by the copies (9.3 ms per
 # step), the IEEE-FP64 form by its compute (17.4 ms against 16.1 ms for the
-# step alone).  The library uses fewer where a band would have under 2^19 cells.
+# step alone, up to 25 ms while other users load the host link).  The library uses
+# fewer where a band would have under 2^19 cells.
 HOST_STEP_BANDS = {"split": 32, "fp64": 32}
 
 
