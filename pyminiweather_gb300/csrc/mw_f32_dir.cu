@@ -129,8 +129,7 @@ struct SmemZ {
 // calls it (one barrier after the row table is formed).  tab: z1 - z0 + 17 rows
 // of shared memory.  SRC: the forcing of w comes through a ring of its own (srcs,
 // kRing rows of NC) beside the state's: read where the three stages add it, it
-// stood in each one's way (2501x1251: 175 us a step against 79 without forcing,
-// 113 here).
+// stood in each one's way (2501x1251: 175 us a step, 127 here, 82 without forcing).
 // TMP: the second stage is stored too.  Without it the march is unrolled by four
 // (8192x2048: 145 against 169 us, the streams' rows keep their registers); with
 // it the extra stores bound the pass and the compact loop does better (190
